@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(kT) k_dense_pick(const uint64_t *__restrict__ 
 template <class PT, bool FP32, bool VL>
 __device__ __forceinline__ bool linked(const SPos<PT> &p, const SPos<PT> &q, const Geom &g,
                                        const VLRec<FP32> &va, const VLRec<FP32> &vb,
-                                       unsigned long long &rechecks) {
+                                       uint32_t &rechecks) {
   float t_lo = g.t_lo, t_hi = g.t_hi;
   double lsq = g.linksq;
   if constexpr (VL) {
@@ -598,53 +598,42 @@ __device__ __forceinline__ double box_dist2(const Geom &g, double x, double y, d
 }
 
 // Per-thread tallies of the befriending kernels, flushed once per warp.
+// (one thread's share of a run stays far below 2^32)
 struct BfStats {
-  unsigned long long tests = 0, rechecks = 0, cand = 0, skips = 0, unions = 0, steps = 0;
-  unsigned long long scan = 0, window = 0;
+  uint32_t tests = 0, rechecks = 0, cand = 0, skips = 0, unions = 0, steps = 0;
+  uint32_t scan = 0, window = 0;
 
-  __device__ void flush(Counters *ctr) {
+  __device__ void add(unsigned long long *to, uint32_t v) {
+    unsigned long long w = v;
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-      tests += __shfl_down_sync(0xffffffffu, tests, d);
-      rechecks += __shfl_down_sync(0xffffffffu, rechecks, d);
-      cand += __shfl_down_sync(0xffffffffu, cand, d);
-      skips += __shfl_down_sync(0xffffffffu, skips, d);
-      unions += __shfl_down_sync(0xffffffffu, unions, d);
-      steps += __shfl_down_sync(0xffffffffu, steps, d);
-      scan += __shfl_down_sync(0xffffffffu, scan, d);
-      window += __shfl_down_sync(0xffffffffu, window, d);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      if (tests) atomicAdd(&ctr->pair_tests, tests);
-      if (rechecks) atomicAdd(&ctr->rechecks, rechecks);
-      if (cand) atomicAdd(&ctr->cand_pairs, cand);
-      if (skips) atomicAdd(&ctr->root_skips, skips);
-      if (unions) atomicAdd(&ctr->unions, unions);
-      if (steps) atomicAdd(&ctr->find_steps, steps);
-      if (scan) atomicAdd(&ctr->scan_iters, scan);
-      if (window) atomicAdd(&ctr->window_iters, window);
-    }
+    for (int d = 16; d > 0; d >>= 1) w += __shfl_down_sync(0xffffffffu, w, d);
+    if ((threadIdx.x & 31) == 0 && w) atomicAdd(to, w);
+  }
+  __device__ void flush(Counters *ctr) {
+    add(&ctr->pair_tests, tests);
+    add(&ctr->rechecks, rechecks);
+    add(&ctr->cand_pairs, cand);
+    add(&ctr->root_skips, skips);
+    add(&ctr->unions, unions);
+    add(&ctr->find_steps, steps);
+    add(&ctr->scan_iters, scan);
+    add(&ctr->window_iters, window);
   }
 };
 
-// Whether any particle of fine cell a (particles [sa, ea), fine coordinates
-// ax, ay, az) is linked to any particle of fine cell b (fine coordinates bx,
-// by, bz).  The loop runs over the cell with fewer particles, and each of
-// its particles farther than the linking length from the other cell's box
-// is skipped; the pair predicate is symmetric (the difference of a pair
+// Whether any particle of fine cell a (particles [sa, ea), packed fine
+// coordinates ga) is linked to any particle of fine cell b ([sb, eb), gb):
+// 1 or 0, or 2 when `limit` steps did not tell.
+// The loop runs over the cell with fewer particles, and each of its
+// particles farther than the linking length from the other cell's box is
+// skipped; the pair predicate is symmetric (the difference of a pair
 // only changes sign, and a variable length comes from the lower of the two
-// grid cells), so the orientation does not change the answer.  Every 16
-// particles, `apart()` is asked whether a and b are still in different
-// components (another thread may have joined them meanwhile); if not, the
-// search stops and reports no link, which is then harmless.
-template <class PT, bool FP32, bool VL, class Apart>
-__device__ __forceinline__ bool cells_linked(const Geom &g, int ax, int ay, int az, uint32_t sa,
-                                             uint32_t ea, uint32_t b, int bx, int by, int bz,
-                                             const uint32_t *__restrict__ run_start,
-                                             const SPos<PT> *__restrict__ spos,
-                                             const VLRec<FP32> *__restrict__ svl, BfStats &st,
-                                             Apart apart) {
-  uint32_t sb = __ldg(run_start + b), eb = __ldg(run_start + b + 1);
+// grid cells), so the orientation does not change the answer.
+template <class PT, bool FP32, bool VL>
+__device__ __forceinline__ int cells_linked(const Geom &g, uint64_t ga, uint64_t gb, uint32_t sa,
+                                            uint32_t ea, uint32_t sb, uint32_t eb, int limit,
+                                            const SPos<PT> *__restrict__ spos,
+                                            const VLRec<FP32> *__restrict__ svl, BfStats &st) {
   if (eb - sb < ea - sa) {
     uint32_t t = sa;
     sa = sb;
@@ -652,56 +641,24 @@ __device__ __forceinline__ bool cells_linked(const Geom &g, int ax, int ay, int 
     t = ea;
     ea = eb;
     eb = t;
-    bx = ax;
-    by = ay;
-    bz = az;
+    gb = ga;
   }
+  const int bx = (int)(gb & kM21), by = (int)((gb >> 21) & kM21), bz = (int)(gb >> 42);
   for (uint32_t i = sa; i < ea; i++) {
-    if (((i - sa) & 15) == 15 && !apart()) return false;
     const SPos<PT> p = spos[i];
+    if (limit-- <= 0) return 2;
     if (box_dist2(g, (double)p.x, (double)p.y, (double)p.z, bx, by, bz) > g.prune_sq) continue;
     VLRec<FP32> va{};
     if constexpr (VL) va = svl[i];
     for (uint32_t j = sb; j < eb; j++) {
+      if (limit-- <= 0) return 2;
       st.tests++;
       VLRec<FP32> vb{};
       if constexpr (VL) vb = svl[j];
-      if (linked<PT, FP32, VL>(p, spos[j], g, va, vb, st.rechecks)) return true;
+      if (linked<PT, FP32, VL>(p, spos[j], g, va, vb, st.rechecks)) return 1;
     }
   }
-  return false;
-}
-
-// Link fine cells a and b if any pair of their particles is linked.  The
-// cells are internally connected, so one linked pair joins them entirely.
-// `ra` caches a root of a's component: it may be stale (a root that was hooked
-// since), but it stays in a's component, so "b reaches ra" still proves that
-// a and b are already joined.
-template <class PT, bool FP32, bool VL>
-__device__ __forceinline__ void try_link(const Geom &g, uint32_t a, int ax, int ay, int az,
-                                         uint32_t &ra, uint32_t b,
-                                         int bx, int by, int bz, uint32_t sa, uint32_t ea,
-                                         const uint32_t *__restrict__ run_start,
-                                         const SPos<PT> *__restrict__ spos,
-                                         const VLRec<FP32> *__restrict__ svl, uint32_t *parent,
-                                         Counters *ctr, BfStats &st) {
-  st.cand++;
-  const uint32_t pb = __ldcg(parent + b);
-  st.steps++;
-  if (pb == ra) { st.skips++; return; }
-  const uint32_t rb = (pb == b) ? b : uf_find_n(parent, pb, st.steps);
-  if (rb == ra) { st.skips++; return; }
-  ra = uf_find_n(parent, ra, st.steps);
-  if (rb == ra) { st.skips++; return; }
-  auto apart = [&]() {
-    return uf_find_n(parent, a, st.steps) != uf_find_n(parent, b, st.steps);
-  };
-  if (cells_linked<PT, FP32, VL>(g, ax, ay, az, sa, ea, b, bx, by, bz, run_start, spos, svl, st,
-                                 apart)) {
-    uf_union(parent, ra, rb, ctr, g.union_cap);
-    st.unions++;
-    ra = uf_find_n(parent, ra, st.steps);
-  }
+  return 0;
 }
 
 // Union-find in shared memory over the fine cells of one top cell (local
@@ -742,6 +699,193 @@ __device__ __forceinline__ uint32_t bit_span(int lo, int hi) {
   return (hi - lo == 31 ? 0xffffffffu : ((1u << (hi - lo + 1)) - 1u)) << lo;
 }
 
+// The global union-find, and the one of a top cell's fine cells in shared
+// memory (indices counted from the top cell's first fine cell, `first`).
+struct GlobalUF {
+  uint32_t *parent;
+  __device__ __forceinline__ uint32_t find(uint32_t x, BfStats &st) const {
+    return uf_find_n(parent, x, st.steps);
+  }
+  __device__ __forceinline__ void join(uint32_t a, uint32_t b, Counters *ctr, uint32_t cap) const {
+    uf_union(parent, a, b, ctr, cap);
+  }
+};
+struct LocalUF {
+  uint32_t *lpar, *ncomp;
+  uint32_t first;
+  __device__ __forceinline__ uint32_t find(uint32_t x, BfStats &) const {
+    return lfind(lpar, x - first);
+  }
+  __device__ __forceinline__ void join(uint32_t a, uint32_t b, Counters *ctr, uint32_t cap) const {
+    if (lunion(lpar, a, b, ctr, cap)) atomicSub(ncomp, 1u);
+  }
+};
+
+// Cell pairs a warp has found to be in reach and in different components,
+// waiting to be tested: fewer than 32 are left over when 32 more may be added.
+constexpr uint32_t kPairSlots = 64;
+// Steps that one lane spends on a cell pair by itself; the whole warp takes
+// those that need more, 32 particle pairs a step.  Most pairs that link do so
+// within a few steps (of the 256^3 box's 2 million listed pairs a few hundred
+// need the warp), and giving the warp every pair of more than 32 particle
+// pairs made the dense kernel 1.6 times as long.
+constexpr int kSoloSteps = 48;
+
+// What the pair tests read, the same for all warps of a kernel.
+template <class PT, bool FP32>
+struct PairArgs {
+  const BoxDev *boxes;
+  const uint16_t *run_box;
+  const uint32_t *run_start;
+  const uint64_t *run_g;
+  const SPos<PT> *spos;
+  const VLRec<FP32> *svl;
+  Counters *ctr;
+};
+
+// cells_linked() by a whole warp (same arguments on every lane): the lanes
+// take 32 particles of the smaller cell at a time, drop those farther than
+// the linking length from the other cell's box, and hold each one left
+// against 32 particles of the other cell a step.  A search that one lane
+// would run for thousands of dependent steps takes 1/32 of them.
+template <class PT, bool FP32, bool VL, class UF>
+__device__ __forceinline__ bool warp_cells_linked(const PairArgs<PT, FP32> &A, const UF &uf,
+                                                  const Geom &g, uint64_t ga, uint64_t gb,
+                                                  uint32_t a, uint32_t b, uint32_t sa,
+                                                  uint32_t ea, uint32_t sb, uint32_t eb,
+                                                  BfStats &st) {
+  const uint32_t lane = threadIdx.x & 31;
+  if (eb - sb < ea - sa) {
+    uint32_t t = sa;
+    sa = sb;
+    sb = t;
+    t = ea;
+    ea = eb;
+    eb = t;
+    gb = ga;
+  }
+  const int bx = (int)(gb & kM21), by = (int)((gb >> 21) & kM21), bz = (int)(gb >> 42);
+  for (uint32_t i0 = sa; i0 < ea; i0 += 32) {
+    SPos<PT> p{};
+    VLRec<FP32> va{};
+    bool near = false;
+    if (i0 + lane < ea) {
+      p = A.spos[i0 + lane];
+      near = !(box_dist2(g, (double)p.x, (double)p.y, (double)p.z, bx, by, bz) > g.prune_sq);
+      if constexpr (VL) va = A.svl[i0 + lane];
+    }
+    uint32_t left = __ballot_sync(0xffffffffu, near);
+    for (uint32_t step = 1; left; step++) {
+      const int l = __ffs(left) - 1;
+      left &= left - 1u;
+      SPos<PT> q{};
+      q.x = __shfl_sync(0xffffffffu, p.x, l);
+      q.y = __shfl_sync(0xffffffffu, p.y, l);
+      q.z = __shfl_sync(0xffffffffu, p.z, l);
+      VLRec<FP32> vq{};
+      if constexpr (VL) {
+        vq.rkey = __shfl_sync(0xffffffffu, va.rkey, l);
+        vq.lsq = __shfl_sync(0xffffffffu, va.lsq, l);
+      }
+      for (uint32_t j0 = sb; j0 < eb; j0 += 32) {
+        const uint32_t j = j0 + lane;
+        bool hit = false;
+        if (j < eb) {
+          VLRec<FP32> vb{};
+          if constexpr (VL) vb = A.svl[j];
+          st.tests++;
+          hit = linked<PT, FP32, VL>(q, A.spos[j], g, vq, vb, st.rechecks);
+        }
+        if (__any_sync(0xffffffffu, hit)) return true;
+      }
+      // joined by another warp meanwhile: the answer no longer matters
+      if ((step & 7) == 0 && __any_sync(0xffffffffu, uf.find(a, st) == uf.find(b, st)))
+        return false;
+    }
+  }
+  return false;
+}
+
+// Tests the cell pairs in pairs[0, n), n <= 32, one per lane, and joins the
+// linked ones: first whether the two cells are in one component by now, then
+// a bounded number of tests by each lane, then the pairs that these did not
+// settle one after another by the whole warp.
+template <class PT, bool FP32, bool VL, class UF>
+__device__ __forceinline__ void drain_pairs(const PairArgs<PT, FP32> &A, const UF &uf,
+                                            const uint2 *pairs, uint32_t n, BfStats &st) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t a = 0, b = 0, sa = 0, ea = 0, sb = 0, eb = 0;
+  uint64_t ga = 0, gb = 0;
+  bool want = lane < n, big = false;
+  if (want) {
+    const uint2 pr = pairs[lane];
+    a = pr.x;
+    b = pr.y;
+    sa = A.run_start[a];
+    ea = A.run_start[a + 1];
+    sb = A.run_start[b];
+    eb = A.run_start[b + 1];
+    ga = A.run_g[a];
+    gb = A.run_g[b];
+    const uint32_t ra = uf.find(a, st), rb = uf.find(b, st);
+    want = ra != rb;
+    if (!want) st.skips++;
+    if (want) {
+      const Geom &g = A.boxes[A.run_box[a]].g;
+      const int is = cells_linked<PT, FP32, VL>(g, ga, gb, sa, ea, sb, eb, kSoloSteps, A.spos,
+                                                A.svl, st);
+      if (is == 1) {
+        uf.join(ra, rb, A.ctr, g.union_cap);
+        st.unions++;
+      }
+      big = is == 2;
+    }
+  }
+  uint32_t todo = __ballot_sync(0xffffffffu, big);
+  while (todo) {
+    const int l = __ffs(todo) - 1;
+    todo &= todo - 1u;
+    const uint32_t la = __shfl_sync(0xffffffffu, a, l), lb = __shfl_sync(0xffffffffu, b, l);
+    const uint32_t lsa = __shfl_sync(0xffffffffu, sa, l), lea = __shfl_sync(0xffffffffu, ea, l);
+    const uint32_t lsb = __shfl_sync(0xffffffffu, sb, l), leb = __shfl_sync(0xffffffffu, eb, l);
+    const uint64_t lga = __shfl_sync(0xffffffffu, ga, l), lgb = __shfl_sync(0xffffffffu, gb, l);
+    const uint32_t ra = uf.find(la, st), rb = uf.find(lb, st);
+    // (each lane looks for itself: the pair is skipped when any lane finds it joined)
+    if (__any_sync(0xffffffffu, ra == rb)) {
+      if ((int)lane == l) st.skips++;
+      continue;
+    }
+    const Geom &g = A.boxes[A.run_box[la]].g;
+    if (warp_cells_linked<PT, FP32, VL>(A, uf, g, lga, lgb, la, lb, lsa, lea, lsb, leb, st)) {
+      if ((int)lane == l) {
+        uf.join(ra, rb, A.ctr, g.union_cap);
+        st.unions++;
+      }
+      __syncwarp();
+    }
+  }
+}
+
+// Adds the lanes' pairs (where `add` is set) to the warp's list and tests 32
+// of them whenever it holds that many (with `last`, what it holds).  Called by
+// all lanes, with fewer than 32 pairs in the list.
+template <class PT, bool FP32, bool VL, class UF>
+__device__ __forceinline__ void push_pairs(const PairArgs<PT, FP32> &A, const UF &uf, uint2 *pairs,
+                                           uint32_t &npair, bool add, uint32_t a, uint32_t b,
+                                           bool last, BfStats &st) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t m = __ballot_sync(0xffffffffu, add);
+  if (add) pairs[npair + __popc(m & ((1u << lane) - 1u))] = make_uint2(a, b);
+  npair += __popc(m);
+  if (npair >= 32 || (last && npair)) {
+    __syncwarp();
+    const uint32_t n = min(npair, 32u);
+    npair -= n;
+    drain_pairs<PT, FP32, VL>(A, uf, pairs + npair, n, st);
+    __syncwarp();
+  }
+}
+
 // Dense top cells: the fine-cell pairs inside a top cell are joined with a
 // union-find in shared memory, near pairs before far ones; then every fine
 // cell is joined to its local root in the global union-find (a
@@ -750,33 +894,36 @@ __device__ __forceinline__ uint32_t bit_span(int lo, int hi) {
 // cell's faces are left to the global passes.  The occupied fine cells of
 // the top cell are first marked in bit rows (bit x of rows[z k + y]), so a
 // cell visits only the occupied cells of its forward window, a row at a
-// time, and finds their local indices from the rows' prefix counts.  `tid`/`nt` number the
-// threads that share the top cell and `sync` is their barrier; `lpar` holds
-// k3all parents followed by the k^2 rows and their k^2 prefix counts.
-template <class PT, bool FP32, bool VL, class Sync>
-__device__ __forceinline__ void dense_top(uint32_t slot, uint32_t *lpar, uint32_t tid,
-                                          uint32_t nt, Sync sync, const BoxDev *boxes,
-                                          const uint16_t *run_box, uint64_t k3all,
-                                          const uint32_t *run_start, const uint64_t *run_g,
-                                          const uint2 *dense_range, uint32_t *grows,
-                                          uint32_t kk, const SPos<PT> *spos,
-                                          const VLRec<FP32> *svl, uint32_t *parent,
-                                          Counters *ctr, BfStats &st) {
+// time, and finds their local indices from the rows' prefix counts.  A CTA shares the
+// top cell when `cta` is set, else one warp has it; `lpar` holds
+// k3all parents followed by the k^2 rows and their k^2 prefix counts; `pairs`
+// is the warp's list of pairs to test.
+template <class PT, bool FP32, bool VL>
+__device__ __forceinline__ void dense_top(const PairArgs<PT, FP32> &A, uint32_t slot,
+                                          uint32_t *lpar, bool cta, uint2 *pairs, uint64_t k3all,
+                                          const uint2 *dense_range, uint2 *grows, uint32_t kk,
+                                          uint32_t rows_stride, uint32_t *parent, BfStats &st) {
+  const uint32_t tid = cta ? threadIdx.x : threadIdx.x & 31, nt = cta ? blockDim.x : 32;
+  auto sync = [&]() {
+    if (cta) __syncthreads();
+    else __syncwarp();
+  };
   const uint2 fr = dense_range[slot];
   const uint32_t f = fr.x, n = fr.y - fr.x;
-  const Geom &g = boxes[run_box[f]].g;
+  const Geom &g = A.boxes[A.run_box[f]].g;
   const int k = g.k, W = g.W;
   const uint32_t nrow = (uint32_t)(k * k);
   uint32_t *rows = lpar + k3all;   // occupancy bits of each (z, y) row
   uint32_t *pref = rows + nrow;    // occupied fine cells before each row
   // components left: once one is left, every remaining candidate is joined
   volatile uint32_t *ncomp = lpar + k3all + 2 * kk;
+  const LocalUF uf{lpar, lpar + k3all + 2 * kk, f};
   if (tid == 0) *ncomp = n;
   for (uint32_t i = tid; i < n; i += nt) lpar[i] = i;
   for (uint32_t j = tid; j < nrow; j += nt) rows[j] = 0u;
   sync();
   for (uint32_t i = tid; i < n; i += nt) {
-    const uint64_t pg = run_g[f + i];
+    const uint64_t pg = A.run_g[f + i];
     const int gx = (int)(pg & kM21), gy = (int)((pg >> 21) & kM21), gz = (int)(pg >> 42);
     atomicOr(rows + (gz - div_k(gz, g) * k) * k + (gy - div_k(gy, g) * k),
              1u << (gx - div_k(gx, g) * k));
@@ -802,52 +949,60 @@ __device__ __forceinline__ void dense_top(uint32_t slot, uint32_t *lpar, uint32_
     }
   }
   sync();
+  uint32_t npair = 0;
   for (int pass = 0; pass < 2; pass++) {
-    for (uint32_t i = tid; i < n; i += nt) {
-      if (*ncomp == 1) break;
-      const uint32_t a = f + i;
-      const uint64_t pg = run_g[a];
-      const int gx = (int)(pg & kM21), gy = (int)((pg >> 21) & kM21), gz = (int)(pg >> 42);
-      const int sx = gx - div_k(gx, g) * k, sy = gy - div_k(gy, g) * k, sz = gz - div_k(gz, g) * k;
-      const uint32_t sa = run_start[a], ea = run_start[a + 1];
+    // pass 0: cells at Chebyshev distance 1; pass 1: those at 2 and more
+    const int Wp = pass == 0 ? 1 : W;
+    for (uint32_t i0 = tid & ~31u;; i0 += nt) {
+      // past the warp's cells (or once one component is left; one answer for
+      // the whole warp) the pairs still listed are tested
+      const bool last = i0 >= n || __shfl_sync(0xffffffffu, *ncomp, 0) == 1;
+      const uint32_t i = i0 + (tid & 31);
+      const bool act = i < n && !last;
+      int sx = 0, sy = 0, sz = 0;
+      uint32_t ri = 0;
+      if (act) {
+        const uint64_t pg = A.run_g[f + i];
+        const int gx = (int)(pg & kM21), gy = (int)((pg >> 21) & kM21), gz = (int)(pg >> 42);
+        sx = gx - div_k(gx, g) * k;
+        sy = gy - div_k(gy, g) * k;
+        sz = gz - div_k(gz, g) * k;
+        ri = lfind(lpar, i);  // may go stale: re-found before a pair is listed
+      }
       // columns within reach, and the near ones (|dx| <= 1)
       const uint32_t reach = bit_span(max(sx - W, 0), min(sx + W, k - 1));
       const uint32_t near = bit_span(max(sx - 1, 0), min(sx + 1, k - 1));
       const uint32_t after = sx == 31 ? 0u : (0xffffffffu << (sx + 1));
-      uint32_t ri = lfind(lpar, i);  // may go stale: re-found before a pair test
-      for (int dz = 0; dz <= W && sz + dz < k; dz++)
-        for (int dy = (dz == 0 ? 0 : -W); dy <= W; dy++) {
-          const int ty = sy + dy;
-          if (ty < 0 || ty >= k) continue;
-          if (*ncomp == 1) break;
-          const int rc = max(abs(dy), dz);  // the row's distance in y and z
-          uint32_t m;
-          if (pass == 0) m = rc <= 1 ? near : 0u;       // Chebyshev distance <= 1
-          else m = rc <= 1 ? (reach & ~near) : reach;   // Chebyshev distance >= 2
-          if (dz == 0 && dy == 0) m &= after;           // forward only in a's own row
-          const int tz = sz + dz;
+      // the forward rows (dz, dy) in order, from (0, 0) to (Wp, Wp)
+      for (int dz = 0, dy = 0; dz <= (last ? 0 : Wp); dy == Wp ? (dz++, dy = -Wp) : dy++) {
+        const int ty = sy + dy, tz = sz + dz;
+        uint32_t occ = 0, bits = 0, before = 0;
+        if (act && ty >= 0 && ty < k && tz < k) {
+          uint32_t m = pass == 0 ? near : max(abs(dy), dz) <= 1 ? reach & ~near : reach;
+          if (dz == 0 && dy == 0) m &= after;  // forward only in a's own row
           const uint32_t row = (uint32_t)(tz * k + ty);
-          const uint32_t occ = rows[row];
-          uint32_t bits = occ & m;
-          while (bits) {
-            const int tx = __ffs(bits) - 1;
+          occ = rows[row];
+          bits = occ & m;
+          before = pref[row];
+        }
+        while (last || __any_sync(0xffffffffu, bits)) {
+          bool apart = false;
+          uint32_t lj = 0;
+          if (bits) {
+            lj = before + __popc(occ & ((bits & -bits) - 1u));
             bits &= bits - 1u;
-            const uint32_t lj = pref[row] + __popc(occ & ((1u << tx) - 1u));
             st.cand++;
             const uint32_t rj = lfind(lpar, lj);
-            if (rj == ri || rj == (ri = lfind(lpar, i))) {
-              st.skips++;
-              continue;
-            }
-            auto apart = [&]() { return lfind(lpar, i) != lfind(lpar, lj); };
-            if (cells_linked<PT, FP32, VL>(g, gx, gy, gz, sa, ea, f + lj, gx + (tx - sx), gy + dy,
-                                           gz + dz, run_start, spos, svl, st, apart)) {
-              if (lunion(lpar, ri, rj, ctr, g.union_cap))
-                atomicSub(const_cast<uint32_t *>(ncomp), 1u);
-              st.unions++;
-            }
+            if (rj != ri) ri = lfind(lpar, i);
+            apart = rj != ri;
+            if (!apart) st.skips++;
           }
+          push_pairs<PT, FP32, VL>(A, uf, pairs, npair, apart, f + i, f + lj, last, st);
+          if (last) break;
         }
+        if (last) break;
+      }
+      if (last) break;
     }
     sync();
   }
@@ -856,15 +1011,19 @@ __device__ __forceinline__ void dense_top(uint32_t slot, uint32_t *lpar, uint32_
   for (uint32_t i = tid; i < n; i += nt) {
     const uint32_t r = f + lfind(lpar, i);
     if (r != f + i && atomicCAS(parent + f + i, f + i, r) != f + i)
-      uf_union(parent, f + i, r, ctr, g.union_cap);
+      uf_union(parent, f + i, r, A.ctr, g.union_cap);
   }
-  // rows and prefixes stay for the warp path, which looks up this top
-  // cell's fine cells from its neighbours
-  uint32_t *gr = grows + (uint64_t)slot * 2 * kk;
-  for (uint32_t j = tid; j < nrow; j += nt) {
-    gr[j] = rows[j];
-    gr[kk + j] = pref[j];
+  // the rows stay for the queued cells' path, which looks up this top cell's
+  // fine cells from its neighbours: a word per plane (bit y: row y holds fine
+  // cells), then per row its occupancy and the index of its first fine cell
+  uint2 *gr = grows + (uint64_t)slot * rows_stride;
+  for (uint32_t z = tid; z < (uint32_t)k; z += nt) {
+    uint32_t plane = 0;
+    for (int y = 0; y < k; y++) plane |= (rows[z * k + y] != 0u ? 1u : 0u) << y;
+    reinterpret_cast<uint32_t *>(gr)[z] = plane;
   }
+  for (uint32_t j = tid; j < nrow; j += nt)
+    gr[(k + 1) / 2 + j] = make_uint2(rows[j], f + pref[j]);
   sync();
 }
 
@@ -876,45 +1035,44 @@ __device__ __forceinline__ void dense_top(uint32_t slot, uint32_t *lpar, uint32_
 // differ widely.
 template <class PT, bool FP32, bool VL>
 __global__ void __launch_bounds__(128) k_befriend_dense(
-    const BoxDev *__restrict__ boxes, const uint16_t *__restrict__ run_box, uint64_t k3all,
-    const uint32_t *__restrict__ run_start, const uint64_t *__restrict__ run_g,
-    const uint2 *__restrict__ dense_range, const uint32_t *__restrict__ big, DevScal *sc,
-    uint32_t nd_cap, uint32_t *__restrict__ grows, uint32_t kk,
-    const SPos<PT> *__restrict__ spos, const VLRec<FP32> *__restrict__ svl, uint32_t *parent,
-    Counters *ctr, uint32_t lstride) {
+    const PairArgs<PT, FP32> A, uint64_t k3all, const uint2 *__restrict__ dense_range,
+    const uint32_t *__restrict__ big, DevScal *sc, uint32_t nd_cap, uint2 *__restrict__ grows,
+    uint32_t kk, uint32_t rows_stride, uint32_t *parent, uint32_t lstride) {
   if (sc->failed) return;  // a sort of this run gave up: its order is not valid
   extern __shared__ uint32_t smem[];
   __shared__ uint32_t s_slot;
+  __shared__ uint2 s_pairs[4][kPairSlots];
+  uint2 *pairs = s_pairs[threadIdx.x >> 5];
   const uint32_t nd = min(sc->nd, nd_cap), nbig = sc->nbig;
-  BfStats st;
-  auto cta_sync = []() { __syncthreads(); };
-  while (true) {
-    if (threadIdx.x == 0) {
-      const uint32_t b = atomicAdd(&sc->next_big, 1u);
-      s_slot = b < nbig ? big[b] : kNone;
-    }
-    __syncthreads();
-    const uint32_t slot = s_slot;
-    __syncthreads();
-    if (slot == kNone) break;
-    dense_top<PT, FP32, VL>(slot, smem, threadIdx.x, blockDim.x, cta_sync, boxes, run_box,
-                            k3all, run_start, run_g, dense_range, grows, kk, spos, svl, parent,
-                            ctr, st);
-  }
   const uint32_t lane = threadIdx.x & 31;
-  uint32_t *lpar = smem + (size_t)(threadIdx.x >> 5) * lstride;
-  auto warp_sync = []() { __syncwarp(); };
+  uint32_t *own = smem + (size_t)(threadIdx.x >> 5) * lstride;
+  BfStats st;
+  bool cta = true;
   while (true) {
     uint32_t slot = 0;
-    if (lane == 0) slot = atomicAdd(&sc->next_dense, 1u);
-    slot = __shfl_sync(0xffffffffu, slot, 0);
-    if (slot >= nd) break;
-    const uint2 fr = dense_range[slot];
-    if (fr.y - fr.x > kBigTop) continue;
-    dense_top<PT, FP32, VL>(slot, lpar, lane, 32, warp_sync, boxes, run_box, k3all, run_start,
-                            run_g, dense_range, grows, kk, spos, svl, parent, ctr, st);
+    if (cta) {
+      if (threadIdx.x == 0) {
+        const uint32_t b = atomicAdd(&sc->next_big, 1u);
+        s_slot = b < nbig ? big[b] : kNone;
+      }
+      __syncthreads();
+      slot = s_slot;
+      __syncthreads();
+      if (slot == kNone) {
+        cta = false;
+        continue;
+      }
+    } else {
+      if (lane == 0) slot = atomicAdd(&sc->next_dense, 1u);
+      slot = __shfl_sync(0xffffffffu, slot, 0);
+      if (slot >= nd) break;
+      const uint2 fr = dense_range[slot];
+      if (fr.y - fr.x > kBigTop) continue;
+    }
+    dense_top<PT, FP32, VL>(A, slot, cta ? smem : own, cta, pairs, k3all, dense_range, grows, kk,
+                            rows_stride, parent, st);
   }
-  st.flush(ctr);
+  st.flush(A.ctr);
 }
 
 // Whether fine cell a's neighbour top cell in direction o lies within W fine
@@ -936,17 +1094,18 @@ constexpr uint32_t kSimple = 2;  // two slot bits per range below
 constexpr uint32_t kSimpleChunk = 1024;  // fine cells per grab of a CTA
 
 template <class PT, bool FP32, bool VL>
-__global__ void __launch_bounds__(kT, 5) k_befriend_simple(
-    const BoxDev *__restrict__ boxes, const uint16_t *__restrict__ run_box,
-    const uint32_t *__restrict__ run_start, const uint64_t *__restrict__ run_g, DevScal *sc,
-    const uint2 *__restrict__ top_range,
-    const uint32_t *__restrict__ top_slot, const SPos<PT> *__restrict__ spos,
-    const VLRec<FP32> *__restrict__ svl, uint32_t *parent, uint32_t *__restrict__ queue,
-    Counters *ctr) {
+__global__ void __launch_bounds__(kT, 4) k_befriend_simple(
+    const PairArgs<PT, FP32> A, DevScal *sc, const uint2 *__restrict__ top_range,
+    const uint32_t *__restrict__ top_slot, uint32_t *parent, uint32_t *__restrict__ queue) {
   if (sc->failed) return;  // a sort of this run gave up: its order is not valid
   const uint32_t R = sc->R;
-  const int lane = threadIdx.x & 31;
+  const uint32_t lane = threadIdx.x & 31;
   __shared__ uint32_t s_base;
+  __shared__ uint32_t s_first[14][kT];  // first candidate of each top cell, per thread
+  __shared__ uint2 s_pairs[kT / 32][kPairSlots];
+  uint2 *pairs = s_pairs[threadIdx.x >> 5];
+  const GlobalUF uf{parent};
+  uint32_t npair = 0;
   BfStats st;
   // CTAs take chunks of consecutive fine cells from a counter: the work per
   // cell varies a lot across the box (clumps, queued cells), and a static
@@ -956,220 +1115,313 @@ __global__ void __launch_bounds__(kT, 5) k_befriend_simple(
     __syncthreads();
     const uint32_t base = s_base;
     __syncthreads();
-    if (base >= R) break;
-    const uint32_t end = min(base + kSimpleChunk, R);
-    for (uint32_t a = base + threadIdx.x; a < end; a += blockDim.x) {
-    const BoxDev &bx = boxes[run_box[a]];
-    const Geom &g = bx.g;
-    const int k = g.k, W = g.W;
-    const uint64_t pg = run_g[a];
-    const int gx = (int)(pg & kM21), gy = (int)((pg >> 21) & kM21), gz = (int)(pg >> 42);
-    const int tx = div_k(gx, g), ty = div_k(gy, g), tz = div_k(gz, g);
-    const int sx = gx - tx * k, sy = gy - ty * k, sz = gz - tz * k;
-    uint32_t R0[14], NN[14];
+    // past the last chunk, the pairs still listed are tested
+    const bool last = base >= R;
+    const uint32_t end = last ? base + 1 : min(base + kSimpleChunk, R);
+    for (uint32_t a0 = base + (threadIdx.x & ~31u); a0 < end || last; a0 += kT) {
+      const uint32_t a = a0 + lane;
+      int gx = 0, gy = 0, gz = 0, W = 0;
+      bool queued = false;
+      // candidate slots: bit 2 nb + q stands for fine cell s_first[nb] + q.  The
+      // first fine cell of every range is loaded at once and dropped here when
+      // out of reach; the slots left are visited from one call site below
+      uint32_t m = 0;
+      if (a < end && !last) {
+        const BoxDev &bx = A.boxes[A.run_box[a]];
+        const Geom &g = bx.g;
+        const int k = g.k;
+        W = g.W;
+        const uint64_t pg = A.run_g[a];
+        gx = (int)(pg & kM21);
+        gy = (int)((pg >> 21) & kM21);
+        gz = (int)(pg >> 42);
+        const int tx = div_k(gx, g), ty = div_k(gy, g), tz = div_k(gz, g);
+        const int sx = gx - tx * k, sy = gy - ty * k, sz = gz - tz * k;
+        uint32_t many = 0;  // slots of the ranges, then whether one holds more than kSimple
 #pragma unroll
-    for (int nb = 0; nb < 14; nb++) {
-      const int ux = tx + kFwd[nb][0], uy = ty + kFwd[nb][1], uz = tz + kFwd[nb][2];
-      // a top cell more than W fine cells away from a is skipped without a load
-      const bool in = !(ux < 0 || uy < 0 || ux >= g.T[0] || uy >= g.T[1] || uz >= g.T[2]) &&
-                      reaches(sx, kFwd[nb][0], k, W) && reaches(sy, kFwd[nb][1], k, W) &&
-                      reaches(sz, kFwd[nb][2], k, W);
-      const uint64_t tb = in ? bx.top_base + ((uint64_t)uz * g.T[1] + uy) * g.T[0] + ux : 0;
-      const uint2 tr = in ? top_range[tb] : make_uint2(0u, 0u);
-      const uint32_t f = tr.x, e = tr.y;
-      R0[nb] = nb == 0 ? a + 1 : f;
-      NN[nb] = e > R0[nb] ? e - R0[nb] : 0u;
-      // pairs inside a dense top cell are joined by k_befriend_dense
-      if (nb == 0 && in && top_slot[tb] != kNone) NN[nb] = 0u;
-    }
-    bool simple = true;
-#pragma unroll
-    for (int nb = 0; nb < 14; nb++) simple &= NN[nb] <= kSimple;
-    const unsigned active = __activemask();
-    const unsigned qmask = __ballot_sync(active, !simple);
-    if (qmask) {
-      const int leader = __ffs(qmask) - 1;
-      uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(&sc->qcount, (uint32_t)__popc(qmask));
-      base = __shfl_sync(active, base, leader);
-      if (!simple) queue[base + __popc(qmask & ((1u << lane) - 1u))] = a;
-    }
-    if (!simple) continue;
-    // candidate slots: bit 2 nb + q stands for fine cell R0[nb] + q.  The
-    // first fine cell of every range is loaded at once and dropped here when
-    // out of reach; the slots left are visited from one call site below (a
-    // single inlined copy of the link test keeps the kernel's code small)
-    uint32_t m = 0;
-#pragma unroll
-    for (int nb = 0; nb < 14; nb++) {
-      if (NN[nb] == 0) continue;
-      st.scan += NN[nb];
-      const uint64_t qg = run_g[R0[nb]];
-      const int bx2 = (int)(qg & kM21), by2 = (int)((qg >> 21) & kM21), bz2 = (int)(qg >> 42);
-      if (max(abs(bx2 - gx), max(abs(by2 - gy), abs(bz2 - gz))) <= W) m |= 1u << (2 * nb);
-      if (NN[nb] > 1) m |= 2u << (2 * nb);
-    }
-    uint32_t ra = 0xffffffffu, sa = 0, ea = 0;
-    while (m) {
-      const int bit = __ffs(m) - 1;
-      m &= m - 1;
-      const int nb = bit >> 1;
-      uint32_t r = 0;
-#pragma unroll
-      for (int t = 0; t < 14; t++) r = t == nb ? R0[t] : r;
-      r += (uint32_t)(bit & 1);
-      const uint64_t qg = run_g[r];  // L1 hit for the first cell of a range
-      const int bx2 = (int)(qg & kM21), by2 = (int)((qg >> 21) & kM21), bz2 = (int)(qg >> 42);
-      if ((bit & 1) && max(abs(bx2 - gx), max(abs(by2 - gy), abs(bz2 - gz))) > W) continue;
-      if (ra == 0xffffffffu) {
-        ra = __ldcg(parent + a);
-        sa = run_start[a];
-        ea = run_start[a + 1];
-      }
-      try_link<PT, FP32, VL>(g, a, gx, gy, gz, ra, r, bx2, by2, bz2, sa, ea, run_start, spos, svl, parent,
-                             ctr, st);
-    }
-    }
-  }
-  st.flush(ctr);
-}
-
-// Warp path, one warp per queued fine cell a.  Lanes 0..13 fetch the 14
-// top-cell ranges at once; the candidate slots of all 14 (fine cells of small
-// top cells, window slots of dense ones, found through their occupancy rows)
-// are then flattened and taken 32 at a time, so a cell costs a few L2 round
-// trips instead of one per slot.  Warps take cells from an atomic counter as they finish, so a few
-// expensive cells do not hold back a whole static share.  PHASE 0 visits the
-// candidates within one fine cell, PHASE 1 the farther ones, so that a dense
-// neighbourhood is joined (and compressed) before its far pairs are tried and
-// most of those become root skips.
-template <class PT, bool FP32, bool VL, int PHASE>
-__global__ void __launch_bounds__(kT, 4) k_befriend(
-    const BoxDev *__restrict__ boxes, const uint16_t *__restrict__ run_box, uint64_t k3all,
-    const uint32_t *__restrict__ run_start, const uint64_t *__restrict__ run_g,
-    const uint32_t *__restrict__ queue, DevScal *sc, const uint2 *__restrict__ top_range,
-    const uint32_t *__restrict__ top_slot,
-    const uint32_t *__restrict__ grows, uint32_t kk, const SPos<PT> *__restrict__ spos,
-    const VLRec<FP32> *__restrict__ svl, uint32_t *parent, Counters *ctr) {
-  if (sc->failed) return;  // a sort of this run gave up: its order is not valid
-  const uint32_t NQ = sc->qcount;
-  uint32_t *next = PHASE == 0 ? &sc->next0 : &sc->next1;
-  const int lane = threadIdx.x & 31;
-  BfStats st;
-  while (true) {
-    uint32_t qi = 0;
-    if (lane == 0) qi = atomicAdd(next, 1u);
-    qi = __shfl_sync(0xffffffffu, qi, 0);
-    if (qi >= NQ) break;
-    const uint32_t a = queue[qi];
-    const BoxDev &bx = boxes[run_box[a]];
-    const Geom &g = bx.g;
-    const int k = g.k, W = g.W;
-    const uint64_t pg = run_g[a];
-    const int gx = (int)(pg & kM21), gy = (int)((pg >> 21) & kM21), gz = (int)(pg >> 42);
-    const int tx = div_k(gx, g), ty = div_k(gy, g), tz = div_k(gz, g);
-    const uint32_t sa = run_start[a], ea = run_start[a + 1];
-    uint32_t ra = __ldcg(parent + a);
-    const int sx = gx - tx * k, sy = gy - ty * k, sz = gz - tz * k;
-    // lane l < 14 describes neighbour top cell l
-    uint32_t r0 = 0, nsparse = 0, nslots = 0, mapbase = 0;
-    int x0 = 0, y0 = 0, z0 = 0, nx = 1, ny = 1, ox = 0, oy = 0, oz = 0;
-    if (lane < 14) {
-      const int ux = tx + kFwd[lane][0], uy = ty + kFwd[lane][1], uz = tz + kFwd[lane][2];
-      if (!(ux < 0 || uy < 0 || ux >= g.T[0] || uy >= g.T[1] || uz >= g.T[2]) &&
-          reaches(sx, kFwd[lane][0], k, W) && reaches(sy, kFwd[lane][1], k, W) &&
-          reaches(sz, kFwd[lane][2], k, W)) {
-        const uint64_t tb = bx.top_base + ((uint64_t)uz * g.T[1] + uy) * g.T[0] + ux;
-        const uint2 tr = top_range[tb];
-        const uint32_t f = tr.x, e = tr.y;
-        const uint32_t slot = top_slot[tb];
-        r0 = lane == 0 ? a + 1 : f;
-        // pairs inside a dense top cell are joined by k_befriend_dense
-        if (lane == 0 && slot != kNone) r0 = e;
-        if (r0 < e) {
-          if (slot == kNone) {
-            nsparse = e - r0;
-          } else {
-            x0 = max(gx - W, ux * k);
-            const int x1 = min(gx + W, ux * k + k - 1);
-            y0 = max(gy - W, uy * k);
-            const int y1 = min(gy + W, uy * k + k - 1);
-            z0 = max(gz - W, uz * k);
-            const int z1 = min(gz + W, uz * k + k - 1);
-            if (x1 >= x0 && y1 >= y0 && z1 >= z0) {
-              nx = x1 - x0 + 1;
-              ny = y1 - y0 + 1;
-              nslots = (uint32_t)(nx * ny * (z1 - z0 + 1));
-              mapbase = slot;
-              ox = ux * k;
-              oy = uy * k;
-              oz = uz * k;
-            }
+        for (int nb = 0; nb < 14; nb++) {
+          const int ux = tx + kFwd[nb][0], uy = ty + kFwd[nb][1], uz = tz + kFwd[nb][2];
+          // a top cell more than W fine cells away from a is skipped without a load
+          if (!(ux < 0 || uy < 0 || ux >= g.T[0] || uy >= g.T[1] || uz >= g.T[2]) &&
+              reaches(sx, kFwd[nb][0], k, W) && reaches(sy, kFwd[nb][1], k, W) &&
+              reaches(sz, kFwd[nb][2], k, W)) {
+            const uint64_t tb = bx.top_base + ((uint64_t)uz * g.T[1] + uy) * g.T[0] + ux;
+            const uint2 tr = top_range[tb];
+            const uint32_t r0 = nb == 0 ? a + 1 : tr.x;
+            uint32_t nn = tr.y > r0 ? tr.y - r0 : 0u;
+            // pairs inside a dense top cell are joined by k_befriend_dense
+            if (nb == 0 && nn && top_slot[tb] != kNone) nn = 0u;
+            s_first[nb][threadIdx.x] = r0;
+            many |= nn > kSimple;
+            m |= min(nn, kSimple) == 0 ? 0u : (nn == 1 ? 1u : 3u) << (2 * nb);
           }
         }
+        queued = many != 0;
       }
-    }
-    const uint32_t cnt = nsparse + nslots;
-    uint32_t incl = cnt;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
-      if (lane >= d) incl += t;
-    }
-    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    const uint32_t excl = incl - cnt;
-    for (uint32_t j0 = 0; j0 < total; j0 += 32) {
-      const uint32_t j = j0 + lane;
-      // the neighbour top cell l whose items hold j
-      int l = 0;
-#pragma unroll
-      for (int q = 1; q < 14; q++)
-        if (j >= __shfl_sync(0xffffffffu, excl, q)) l = q;
-      const uint32_t l_excl = __shfl_sync(0xffffffffu, excl, l);
-      const uint32_t l_r0 = __shfl_sync(0xffffffffu, r0, l);
-      const uint32_t l_ns = __shfl_sync(0xffffffffu, nsparse, l);
-      const int l_x0 = __shfl_sync(0xffffffffu, x0, l), l_y0 = __shfl_sync(0xffffffffu, y0, l),
-                l_z0 = __shfl_sync(0xffffffffu, z0, l), l_nx = __shfl_sync(0xffffffffu, nx, l),
-                l_ny = __shfl_sync(0xffffffffu, ny, l), l_ox = __shfl_sync(0xffffffffu, ox, l),
-                l_oy = __shfl_sync(0xffffffffu, oy, l), l_oz = __shfl_sync(0xffffffffu, oz, l);
-      const uint32_t l_map = __shfl_sync(0xffffffffu, mapbase, l);
-      if (j >= total) continue;
-      const uint32_t off = j - l_excl;
-      uint32_t r;
-      int bx2, by2, bz2;
-      if (off < l_ns) {
-        st.scan++;
-        r = l_r0 + off;
-        const uint64_t qg = run_g[r];
-        bx2 = (int)(qg & kM21);
-        by2 = (int)((qg >> 21) & kM21);
-        bz2 = (int)(qg >> 42);
-        if (max(abs(bx2 - gx), max(abs(by2 - gy), abs(bz2 - gz))) > W) continue;
-      } else {
-        st.window++;
-        const uint32_t sl = off - l_ns;
-        bx2 = l_x0 + (int)(sl % (uint32_t)l_nx);
-        by2 = l_y0 + (int)((sl / (uint32_t)l_nx) % (uint32_t)l_ny);
-        bz2 = l_z0 + (int)(sl / (uint32_t)(l_nx * l_ny));
-        // a slot of the other phase is dropped before its row is read
-        const int cheb_s = max(abs(bx2 - gx), max(abs(by2 - gy), abs(bz2 - gz)));
-        if ((PHASE == 0 && cheb_s > 1) || (PHASE == 1 && cheb_s <= 1)) continue;
-        // occupancy bit of the slot's fine cell, then its index from the
-        // top cell's row prefix (fine cells are in sub-cell order)
-        const uint32_t *gr = grows + (uint64_t)l_map * 2 * kk;
-        const uint32_t row = (uint32_t)((bz2 - l_oz) * k + (by2 - l_oy));
-        const uint32_t occ = gr[row];
-        const int cx = bx2 - l_ox;
-        if (!((occ >> cx) & 1u)) continue;
-        r = l_r0 + gr[kk + row] + __popc(occ & ((1u << cx) - 1u));
+      const uint32_t qmask = __ballot_sync(0xffffffffu, queued);
+      if (qmask) {
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(&sc->qcount, (uint32_t)__popc(qmask));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (queued) {
+          queue[at + __popc(qmask & ((1u << lane) - 1u))] = a;
+          m = 0;
+        }
       }
-      const int cheb = max(abs(bx2 - gx), max(abs(by2 - gy), abs(bz2 - gz)));
-      if ((PHASE == 0 && cheb > 1) || (PHASE == 1 && cheb <= 1)) continue;
-      try_link<PT, FP32, VL>(g, a, gx, gy, gz, ra, r, bx2, by2, bz2, sa, ea, run_start, spos, svl, parent, ctr,
-                             st);
+      uint32_t ra = kNone;
+      while (last || __any_sync(0xffffffffu, m)) {
+        bool apart = false;
+        uint32_t r = 0;
+        if (m) {
+          const int bit = __ffs(m) - 1;
+          m &= m - 1u;
+          r = s_first[bit >> 1][threadIdx.x] + (uint32_t)(bit & 1);
+          const uint64_t qg = A.run_g[r];
+          st.scan++;
+          if (max(abs((int)(qg & kM21) - gx),
+                  max(abs((int)((qg >> 21) & kM21) - gy), abs((int)(qg >> 42) - gz))) <= W) {
+            st.cand++;
+            if (ra == kNone) ra = __ldcg(parent + a);
+            uint32_t rb = __ldcg(parent + r);
+            st.steps++;
+            if (rb != ra && rb != r) rb = uf_find_n(parent, rb, st.steps);
+            // ra may have been hooked since; it stays in a's component
+            if (rb != ra) ra = uf_find_n(parent, ra, st.steps);
+            apart = rb != ra;
+            if (!apart) st.skips++;
+          }
+        }
+        push_pairs<PT, FP32, VL>(A, uf, pairs, npair, apart, a, r, last, st);
+        if (last) break;
+      }
+      if (last) break;
     }
+    if (last) break;
   }
-  st.flush(ctr);
+  st.flush(A.ctr);
+}
+
+// The queued fine cells: candidates in the 13 forward top cells (and, when a's
+// own top cell is not dense, in the rest of it).  PHASE 0 visits the
+// candidates within one fine cell, PHASE 1 the farther ones, so that a dense
+// neighbourhood is joined (and compressed) before its far pairs are tried and
+// most of those are found joined.
+//
+// The kernel is bound by the latency of its table reads and by instruction
+// issue, so a warp works its cells off in three levels, each with all lanes
+// busy and many reads in flight.  It takes 32 queued cells, one per lane (or
+// 32 / G cells of G lanes each when the queue is short, so that it still fills
+// the chip; one atomic per grab), and steps its lanes through the neighbour
+// top cells together, the next neighbour's range and slot being read
+// meanwhile.  1: of a dense neighbour the plane words (bit y: row y of the
+// plane holds fine cells) give the window's non-empty rows, of a sparse one
+// the fine cells give those in reach: one bit each, listed.  2: the listed
+// rows are taken 32 at a time, one per lane: the row's word gives the
+// candidates, each compared with its cell's root.  3: candidates in another
+// component are tested 32 at a time (drain_pairs).  Most rows are empty, hence
+// the plane words: with a word read per row the far phase issued 1.2 times the
+// instructions and took 1.25 times as long.  Near and far phase on the 256^3
+// box: 0.94 + 0.73 ms with a warp per cell and a lane per window slot, 0.28 +
+// 0.40 ms so (ncu, cold cache); the whole befriending of the 512^3 box at the
+// 1024^3 box's parameters 36.5 -> 21.5 ms.
+constexpr uint32_t kRowSlots = 64;
+constexpr int kPlanes = 8;  // plane words read at a time
+// floor(i / d) = i * kDiv[d] >> 16 for i < 64, d <= 32
+__constant__ uint32_t kDiv[33] = {
+    0,    65536, 32769, 21846, 16385, 13108, 10923, 9363, 8193, 7282, 6554,
+    5958, 5462,  5042,  4682,  4370,  4097,  3856,  3641, 3450, 3277, 3121,
+    2979, 2850,  2731,  2622,  2521,  2428,  2341,  2260, 2185, 2115, 2049};
+
+template <class PT, bool FP32, bool VL, int PHASE>
+__global__ void __launch_bounds__(kT, 3) k_befriend(
+    const PairArgs<PT, FP32> A, const uint32_t *__restrict__ queue, DevScal *sc,
+    const uint2 *__restrict__ top_range, const uint32_t *__restrict__ top_slot,
+    const uint2 *__restrict__ grows, uint32_t rows_stride, uint32_t *parent) {
+  if (sc->failed) return;  // a sort of this run gave up: its order is not valid
+  __shared__ uint2 s_pairs[kT / 32][kPairSlots];
+  // listed rows: index of the row's word and its columns within reach, or the
+  // fine cell itself and no columns; and the lane of the cell they are for
+  __shared__ uint2 s_row[kT / 32][kRowSlots];
+  __shared__ uint8_t s_lane[kT / 32][kRowSlots];
+  uint2 *pairs = s_pairs[threadIdx.x >> 5], *rows = s_row[threadIdx.x >> 5];
+  uint8_t *rlane = s_lane[threadIdx.x >> 5];
+  const GlobalUF uf{parent};
+  const uint32_t NQ = sc->qcount;
+  if (NQ == 0) return;
+  uint32_t *next = PHASE == 0 ? &sc->next0 : &sc->next1;
+  const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u;
+  // lanes per cell: the fewest (1, 2, 4, 8) that give every thread of the grid work
+  int lg = 0;
+  while (lg < 3 && ((uint64_t)NQ << lg) < (uint64_t)gridDim.x * blockDim.x) lg++;
+  const uint32_t G = 1u << lg, sub = lane & (G - 1);
+  // a lane's share of its cell's bits: every G-th
+  const uint64_t share = (lg == 0 ? ~0ull : lg == 1 ? 0x5555555555555555ull
+                          : lg == 2 ? 0x1111111111111111ull : 0x0101010101010101ull) << sub;
+  uint32_t npair = 0, nrow = 0;
+  BfStats st;
+  while (true) {
+    uint32_t q0 = 0;
+    if (lane == 0) q0 = atomicAdd(next, 32u >> lg);
+    q0 = __shfl_sync(0xffffffffu, q0, 0);
+    // past the last cells, the pairs still listed are tested
+    const bool last = q0 >= NQ;
+    const uint32_t qi = q0 + (lane >> lg);
+    const bool act = qi < NQ && !last;
+    const uint32_t a = queue[act ? qi : 0u];
+    const BoxDev &bx = A.boxes[A.run_box[a]];
+    const Geom &g = bx.g;
+    const int k = g.k, W = PHASE == 0 ? 1 : g.W;
+    const uint64_t pg = A.run_g[a];
+    const int gx = (int)(pg & kM21), gy = (int)((pg >> 21) & kM21), gz = (int)(pg >> 42);
+    const int tx = div_k(gx, g), ty = div_k(gy, g), tz = div_k(gz, g);
+    const int sx = gx - tx * k, sy = gy - ty * k, sz = gz - tz * k;
+    const uint32_t ra = __ldcg(parent + a);
+    uint2 tr = make_uint2(0u, 0u), tr_next = tr;  // range and slot of a neighbour top cell
+    uint32_t slot = kNone, slot_next = kNone;
+    auto fetch = [&](int nb, uint2 &range, uint32_t &sl) {
+      const int ox = kFwd[nb][0], oy = kFwd[nb][1], oz = kFwd[nb][2];
+      const int ux = tx + ox, uy = ty + oy, uz = tz + oz;
+      range = make_uint2(0u, 0u);
+      sl = kNone;
+      if (act && !(ux < 0 || uy < 0 || ux >= g.T[0] || uy >= g.T[1] || uz >= g.T[2]) &&
+          reaches(sx, ox, k, W) && reaches(sy, oy, k, W) && reaches(sz, oz, k, W)) {
+        const uint64_t tb = bx.top_base + ((uint64_t)uz * g.T[1] + uy) * g.T[0] + ux;
+        range = top_range[tb];
+        sl = top_slot[tb];
+      }
+    };
+    if (!last) fetch(0, tr, slot);
+#pragma unroll 1
+    for (int nb = last ? 14 : 0; nb < 15; nb++) {  // (nb = 14: what is left in the lists)
+      if (nb < 13) fetch(nb + 1, tr_next, slot_next);
+      // items of this neighbour: fine cells (sparse), or rows of the window (dense)
+      const uint32_t r0 = nb == 0 ? a + 1 : tr.x;
+      const uint2 *gr = nullptr;
+      int cx = 0, cy = 0, cz = 0;         // a in the neighbour's own fine coordinates
+      int y0 = 0, ny = 1, z0 = 0, nz = 0;  // the window's rows there
+      uint32_t cnt = 0, chunk = 32;       // items (rows or cells) and how many at a time
+      if (nb < 14 && r0 < tr.y) {
+        if (slot == kNone) {
+          cnt = tr.y - r0;
+        } else if (nb != 0) {  // pairs inside a dense top cell are k_befriend_dense's
+          gr = grows + (uint64_t)slot * rows_stride;
+          cx = sx - kFwd[nb][0] * k;
+          cy = sy - kFwd[nb][1] * k;
+          cz = sz - kFwd[nb][2] * k;
+          y0 = max(cy - W, 0);
+          ny = min(cy + W, k - 1) - y0 + 1;
+          z0 = max(cz - W, 0);
+          nz = min(cz + W, k - 1) - z0 + 1;
+          cnt = (uint32_t)(ny * nz);
+          // whole planes, as many as kPlanes and 64 bits take
+          chunk = (uint32_t)ny * min((64u * kDiv[ny]) >> 16, (uint32_t)kPlanes);
+        }
+      }
+      const uint32_t reach = gr ? bit_span(max(cx - W, 0), min(cx + W, k - 1)) : 0u;
+      // the near columns, which were PHASE 0's in the rows within one row of a
+      const uint32_t inner = PHASE == 1 && gr && cx >= -1 && cx <= k
+                                 ? bit_span(max(cx - 1, 0), min(cx + 1, k - 1)) : 0u;
+      for (uint32_t i0 = 0; nb == 14 || __any_sync(0xffffffffu, i0 < cnt); i0 += chunk) {
+        uint64_t todo = 0;  // bit i: item i0 + i is to be listed
+        if (gr && i0 < cnt) {
+          const uint32_t *planes = reinterpret_cast<const uint32_t *>(gr);
+          const uint32_t span = bit_span(0, ny - 1);
+#pragma unroll
+          for (int u = 0; u < kPlanes; u++)
+            if (u * ny < (int)min(chunk, cnt - i0)) {
+              const int z = z0 + (int)((i0 * kDiv[ny]) >> 16) + u;
+              todo |= (uint64_t)((planes[z] >> y0) & span) << (u * ny);
+            }
+          todo &= share;
+          st.window += __popcll(todo);
+        } else if (i0 < cnt) {
+          const uint32_t n = min(cnt - i0, 32u);
+#pragma unroll 4
+          for (uint32_t u = sub; u < n; u += G) {
+            const uint64_t qg = A.run_g[r0 + i0 + u];
+            const int cheb =
+                max(abs((int)(qg & kM21) - gx),
+                    max(abs((int)((qg >> 21) & kM21) - gy), abs((int)(qg >> 42) - gz)));
+            if (cheb <= W && (PHASE == 0 || cheb > 1)) todo |= 1ull << u;
+            st.scan++;
+          }
+        }
+        while (true) {
+          bool add = todo != 0;
+          uint2 e = make_uint2(0u, 0u);
+          if (add) {
+            const uint32_t i = i0 + (uint32_t)__ffsll((long long)todo) - 1u;
+            todo &= todo - 1u;
+            if (gr) {
+              const int zz = (int)((i * kDiv[ny]) >> 16), z = z0 + zz, y = y0 + (int)i - zz * ny;
+              e.x = (uint32_t)(gr - grows) + (uint32_t)((k + 1) / 2 + z * k + y);
+              e.y = PHASE == 1 && max(abs(y - cy), abs(z - cz)) <= 1 ? reach & ~inner : reach;
+              add = e.y != 0;
+            } else {
+              e.x = r0 + i;
+            }
+          }
+          const uint32_t m = __ballot_sync(0xffffffffu, add);
+          if (add) {
+            const uint32_t at = nrow + __popc(m & below);
+            rows[at] = e;
+            rlane[at] = (uint8_t)lane;
+          }
+          nrow += __popc(m);
+          const bool more = __any_sync(0xffffffffu, todo != 0);
+          if (nrow >= 32 || nb == 14) {
+            // the last 32 listed rows, one per lane
+            __syncwarp();
+            const uint32_t n = min(nrow, 32u);
+            nrow -= n;
+            uint32_t bits = 0, occ = 0, first = 0;
+            int own = 0;
+            if (lane < n) {
+              const uint2 w = rows[nrow + lane];
+              own = rlane[nrow + lane];
+              if (w.y) {
+                const uint2 word = grows[w.x];
+                occ = word.x;
+                bits = occ & w.y;
+                first = word.y;
+              } else {
+                bits = 1;
+                first = w.x;
+              }
+            }
+            const uint32_t ca = __shfl_sync(0xffffffffu, a, own);
+            uint32_t cr = __shfl_sync(0xffffffffu, ra, own);
+            do {
+              bool apart = false;
+              uint32_t b = 0;
+              if (bits) {
+                b = first + __popc(occ & ((bits & -bits) - 1u));
+                bits &= bits - 1u;
+                st.cand++;
+                st.steps++;
+                // (PHASE 1: the cached parent may be an older one, which is still
+                // in the candidate's component)
+                uint32_t rb = PHASE == 1 ? __ldca(parent + b) : __ldcg(parent + b);
+                if (rb != cr && rb != b) rb = uf_find_n(parent, rb, st.steps);
+                // cr may have been hooked since; it stays in its cell's component
+                if (rb != cr) cr = uf_find_n(parent, cr, st.steps);
+                apart = rb != cr;
+                if (!apart) st.skips++;
+              }
+              push_pairs<PT, FP32, VL>(A, uf, pairs, npair, apart, ca, b, last, st);
+            } while (__any_sync(0xffffffffu, bits != 0));
+            __syncwarp();
+          }
+          if (!more) break;
+        }
+        if (nb == 14) break;
+      }
+      tr = tr_next;
+      slot = slot_next;
+    }
+    if (last) break;
+  }
+  st.flush(A.ctr);
 }
 
 __global__ void __launch_bounds__(kT) k_compress(uint32_t *parent,
@@ -1674,13 +1926,13 @@ int dense_warps_per_cta(uint64_t k3all) {
   return (int)std::max<uint64_t>(1, std::min<uint64_t>(4, (200u << 10) / per));
 }
 
-// Occupancy rows of a top cell (k^2).
+// 8-byte words of a dense top cell's occupancy: k plane words of 4 bytes, k^2 rows.
 uint64_t rows_per_top(uint64_t k3all) {
   const uint64_t k = (uint64_t)std::llround(std::cbrt((double)k3all));
-  return k * k;
+  return (k + 1) / 2 + k * k;
 }
 
-// Dense top cells whose rows and row prefixes fit in 4 bytes per processed
+// Dense top cells whose planes and rows fit in 4 bytes per processed
 // particle plus 1 GiB.
 int64_t rows_cap_for(int64_t np_cap, uint64_t k3all) {
   return (int64_t)(((uint64_t)np_cap * 4 + (1ull << 30)) / (rows_per_top(k3all) * 8));
@@ -1835,7 +2087,8 @@ void Plan::issue(bool want_member, cudaStream_t s, bool timed) {
   // union-find), then the queued cells' warp path, near then far ----
   uint32_t *queue = b_rtmp1.as<uint32_t>();  // the keep scan's, free since the emission
   const int dwpc = dense_warps_per_cta(k3all);
-  const uint32_t kk = (uint32_t)rows_per_top(k3all);
+  const uint32_t kmax = (uint32_t)std::llround(std::cbrt((double)k3all)), kk = kmax * kmax;
+  const uint32_t rows_stride = (uint32_t)rows_per_top(k3all);
   const size_t dsm = (size_t)dwpc * dense_words(k3all) * sizeof(uint32_t);
   const unsigned gd = (unsigned)std::max<int64_t>(
       1, std::min<int64_t>((nd_cap + dwpc - 1) / dwpc, (int64_t)kSMs * 64 / dwpc));
@@ -1846,30 +2099,26 @@ void Plan::issue(bool want_member, cudaStream_t s, bool timed) {
     // dense top cells on a second stream, beside the sparse cells
     CMH_CUDA(cudaEventRecord(ev_fork, s));
     CMH_CUDA(cudaStreamWaitEvent(bf_stream, ev_fork, 0));
+    const PairArgs<PT, FP> pa{boxes, b_run_box.as<uint16_t>(), b_run_start.as<uint32_t>(), run_g,
+                              b_spos.as<SPos<PT>>(), svl, c};
     k_befriend_dense<PT, FP, VL><<<gd, 32 * dwpc, dsm, bf_stream>>>(
-        boxes, b_run_box.as<uint16_t>(), k3all, b_run_start.as<uint32_t>(),
-        run_g, b_dense_range.as<uint2>(), b_dense_big.as<uint32_t>(), sc, (uint32_t)nd_cap,
-        b_rows.as<uint32_t>(), kk, b_spos.as<SPos<PT>>(), svl, b_parent.as<uint32_t>(), c,
-        (uint32_t)dense_words(k3all));
+        pa, k3all, b_dense_range.as<uint2>(), b_dense_big.as<uint32_t>(), sc, (uint32_t)nd_cap,
+        b_rows.as<uint2>(), kk, rows_stride, b_parent.as<uint32_t>(), (uint32_t)dense_words(k3all));
     CMH_LAUNCHED();
     CMH_CUDA(cudaEventRecord(ev_join, bf_stream));
     k_befriend_simple<PT, FP, VL><<<rg(k_befriend_simple<PT, FP, VL>, npc), kT, 0, s>>>(
-        boxes, b_run_box.as<uint16_t>(), b_run_start.as<uint32_t>(), run_g,
-        sc, b_top_range.as<uint2>(), b_top_slot.as<uint32_t>(),
-        b_spos.as<SPos<PT>>(), svl, b_parent.as<uint32_t>(), queue, c);
+        pa, sc, b_top_range.as<uint2>(), b_top_slot.as<uint32_t>(), b_parent.as<uint32_t>(), queue);
     CMH_LAUNCHED();
     CMH_CUDA(cudaStreamWaitEvent(s, ev_join, 0));
-    k_befriend<PT, FP, VL, 0><<<rg(k_befriend<PT, FP, VL, 0>, npc * 32), kT, 0, s>>>(
-        boxes, b_run_box.as<uint16_t>(), k3all, b_run_start.as<uint32_t>(),
-        run_g, queue, sc, b_top_range.as<uint2>(), b_top_slot.as<uint32_t>(),
-        b_rows.as<uint32_t>(), kk, b_spos.as<SPos<PT>>(), svl, b_parent.as<uint32_t>(), c);
+    k_befriend<PT, FP, VL, 0><<<rg(k_befriend<PT, FP, VL, 0>, npc * 8), kT, 0, s>>>(
+        pa, queue, sc, b_top_range.as<uint2>(), b_top_slot.as<uint32_t>(), b_rows.as<uint2>(),
+        rows_stride, b_parent.as<uint32_t>());
     CMH_LAUNCHED();
     k_compress<<<rg(k_compress, npc), kT, 0, s>>>(b_parent.as<uint32_t>(), sc);
     CMH_LAUNCHED();
-    k_befriend<PT, FP, VL, 1><<<rg(k_befriend<PT, FP, VL, 1>, npc * 32), kT, 0, s>>>(
-        boxes, b_run_box.as<uint16_t>(), k3all, b_run_start.as<uint32_t>(),
-        run_g, queue, sc, b_top_range.as<uint2>(), b_top_slot.as<uint32_t>(),
-        b_rows.as<uint32_t>(), kk, b_spos.as<SPos<PT>>(), svl, b_parent.as<uint32_t>(), c);
+    k_befriend<PT, FP, VL, 1><<<rg(k_befriend<PT, FP, VL, 1>, npc * 8), kT, 0, s>>>(
+        pa, queue, sc, b_top_range.as<uint2>(), b_top_slot.as<uint32_t>(), b_rows.as<uint2>(),
+        rows_stride, b_parent.as<uint32_t>());
     CMH_LAUNCHED();
   };
   if (fp32 && varlink) befriend(std::true_type{}, std::true_type{});
@@ -2027,7 +2276,10 @@ void Plan::prepare(const std::vector<BoxSpec> &specs, bool want_member) {
   np_cap = std::max<int64_t>(np_cap, std::max<int64_t>(want_np, 1));
   // dense top cells: their rows take at most 4 bytes per processed particle
   // plus 1 GiB (dense top cells past the cap are scanned instead)
-  nd_cap = std::max<int64_t>(nd_cap, np_cap / 1024 + 1024);
+  // (a first run that finds more of them than slots scans the rest, ~3x the
+  // befriending time: the 1024^3 workload's parameters have one dense top cell
+  // per 650 processed particles, the 256^3 ones one per 1100)
+  nd_cap = std::max<int64_t>(nd_cap, std::max(np_cap / 1024 + 1024, np_cap / 256));
   nd_cap = std::min<int64_t>(nd_cap, std::max<int64_t>(1024, rows_cap_for(np_cap, k3all)));
   double mincut = 1e300;
   for (const BoxDev &bd : boxes_host) mincut = std::min(mincut, bd.g.nphalomin);
@@ -2053,7 +2305,7 @@ void Plan::prepare(const std::vector<BoxSpec> &specs, bool want_member) {
   b_top_slot.ensure(n_top * 4);
   b_rtmp1.ensure(npc * 4);
   b_rtmp2.ensure(npc * 4);
-  b_rows.ensure((size_t)nd_cap * rows_per_top(k3all) * 2 * sizeof(uint32_t));
+  b_rows.ensure((size_t)nd_cap * rows_per_top(k3all) * sizeof(uint2));
   b_dense_range.ensure((size_t)nd_cap * sizeof(uint2));
   b_dense_big.ensure((size_t)nd_cap * sizeof(uint32_t));
   b_parent.ensure(npc * 4);

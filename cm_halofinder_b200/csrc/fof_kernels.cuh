@@ -234,8 +234,7 @@ __device__ __forceinline__ uint32_t uf_find(uint32_t *parent, uint32_t x) {
 }
 
 // find() that also counts its parent loads
-__device__ __forceinline__ uint32_t uf_find_n(uint32_t *parent, uint32_t x,
-                                              unsigned long long &steps) {
+__device__ __forceinline__ uint32_t uf_find_n(uint32_t *parent, uint32_t x, uint32_t &steps) {
   while (true) {
     uint32_t p = __ldcg(parent + x);
     steps++;
