@@ -877,7 +877,7 @@ __device__ __forceinline__ void push_pairs(const PairArgs<PT, FP32> &A, const UF
   const uint32_t m = __ballot_sync(0xffffffffu, add);
   if (add) pairs[npair + __popc(m & ((1u << lane) - 1u))] = make_uint2(a, b);
   npair += __popc(m);
-  if (npair >= 32 || (last && npair)) {
+  while (npair >= 32 || (last && npair)) {
     __syncwarp();
     const uint32_t n = min(npair, 32u);
     npair -= n;
@@ -885,6 +885,10 @@ __device__ __forceinline__ void push_pairs(const PairArgs<PT, FP32> &A, const UF
     __syncwarp();
   }
 }
+
+// 16-byte words before the rows of a dense top cell's occupancy (2 k plane
+// words and a fine cell's index).
+__host__ __device__ constexpr int row_head(int k) { return (2 * k + 1 + 3) / 4; }
 
 // Dense top cells: the fine-cell pairs inside a top cell are joined with a
 // union-find in shared memory, near pairs before far ones; then every fine
@@ -896,12 +900,13 @@ __device__ __forceinline__ void push_pairs(const PairArgs<PT, FP32> &A, const UF
 // cell visits only the occupied cells of its forward window, a row at a
 // time, and finds their local indices from the rows' prefix counts.  A CTA shares the
 // top cell when `cta` is set, else one warp has it; `lpar` holds
-// k3all parents followed by the k^2 rows and their k^2 prefix counts; `pairs`
+// k3all parents followed by the k^2 rows, their k^2 prefix counts, k^2 rows of
+// the cells outside the main component and two single words; `pairs`
 // is the warp's list of pairs to test.
 template <class PT, bool FP32, bool VL>
 __device__ __forceinline__ void dense_top(const PairArgs<PT, FP32> &A, uint32_t slot,
                                           uint32_t *lpar, bool cta, uint2 *pairs, uint64_t k3all,
-                                          const uint2 *dense_range, uint2 *grows, uint32_t kk,
+                                          const uint2 *dense_range, uint4 *grows, uint32_t kk,
                                           uint32_t rows_stride, uint32_t *parent, BfStats &st) {
   const uint32_t tid = cta ? threadIdx.x : threadIdx.x & 31, nt = cta ? blockDim.x : 32;
   auto sync = [&]() {
@@ -915,9 +920,10 @@ __device__ __forceinline__ void dense_top(const PairArgs<PT, FP32> &A, uint32_t 
   const uint32_t nrow = (uint32_t)(k * k);
   uint32_t *rows = lpar + k3all;   // occupancy bits of each (z, y) row
   uint32_t *pref = rows + nrow;    // occupied fine cells before each row
+  uint32_t *rest = pref + nrow;    // the occupied fine cells outside the main component
   // components left: once one is left, every remaining candidate is joined
-  volatile uint32_t *ncomp = lpar + k3all + 2 * kk;
-  const LocalUF uf{lpar, lpar + k3all + 2 * kk, f};
+  volatile uint32_t *ncomp = lpar + k3all + 3 * kk, *vmain = ncomp + 1;
+  const LocalUF uf{lpar, lpar + k3all + 3 * kk, f};
   if (tid == 0) *ncomp = n;
   for (uint32_t i = tid; i < n; i += nt) lpar[i] = i;
   for (uint32_t j = tid; j < nrow; j += nt) rows[j] = 0u;
@@ -949,10 +955,36 @@ __device__ __forceinline__ void dense_top(const PairArgs<PT, FP32> &A, uint32_t 
     }
   }
   sync();
+  // The main component: the commonest root among 32 fine cells spread over the
+  // top cell.  Most of the fine cells of a clump are in it once the near pairs
+  // are joined, and for a cell of the main component only those in `rest` are
+  // candidates still.
+  auto find_main = [&]() {
+    if (tid < 32) {
+      const uint32_t r = lfind(lpar, (uint32_t)(((uint64_t)tid * n) >> 5));
+      const uint32_t same = (uint32_t)__popc(__match_any_sync(0xffffffffu, r));
+      const uint32_t most = __reduce_max_sync(0xffffffffu, same);
+      const uint32_t who = __ballot_sync(0xffffffffu, same == most);
+      const uint32_t m = __shfl_sync(0xffffffffu, r, __ffs(who) - 1);
+      if (tid == 0) *vmain = m;
+    }
+    for (uint32_t j = tid; j < nrow; j += nt) rest[j] = 0u;
+    sync();
+    const uint32_t m = *vmain;
+    for (uint32_t i = tid; i < n; i += nt) {
+      if (lfind(lpar, i) == m) continue;
+      const uint64_t pg = A.run_g[f + i];
+      const int gx = (int)(pg & kM21), gy = (int)((pg >> 21) & kM21), gz = (int)(pg >> 42);
+      atomicOr(rest + (gz - div_k(gz, g) * k) * k + (gy - div_k(gy, g) * k),
+               1u << (gx - div_k(gx, g) * k));
+    }
+    sync();
+  };
   uint32_t npair = 0;
   for (int pass = 0; pass < 2; pass++) {
     // pass 0: cells at Chebyshev distance 1; pass 1: those at 2 and more
     const int Wp = pass == 0 ? 1 : W;
+    if (pass == 1) find_main();
     for (uint32_t i0 = tid & ~31u;; i0 += nt) {
       // past the warp's cells (or once one component is left; one answer for
       // the whole warp) the pairs still listed are tested
@@ -969,6 +1001,7 @@ __device__ __forceinline__ void dense_top(const PairArgs<PT, FP32> &A, uint32_t 
         sz = gz - div_k(gz, g) * k;
         ri = lfind(lpar, i);  // may go stale: re-found before a pair is listed
       }
+      const bool main = pass == 1 && act && ri == lfind(lpar, *vmain);
       // columns within reach, and the near ones (|dx| <= 1)
       const uint32_t reach = bit_span(max(sx - W, 0), min(sx + W, k - 1));
       const uint32_t near = bit_span(max(sx - 1, 0), min(sx + 1, k - 1));
@@ -982,7 +1015,7 @@ __device__ __forceinline__ void dense_top(const PairArgs<PT, FP32> &A, uint32_t 
           if (dz == 0 && dy == 0) m &= after;  // forward only in a's own row
           const uint32_t row = (uint32_t)(tz * k + ty);
           occ = rows[row];
-          bits = occ & m;
+          bits = (main ? rest[row] : occ) & m;
           before = pref[row];
         }
         while (last || __any_sync(0xffffffffu, bits)) {
@@ -1015,15 +1048,24 @@ __device__ __forceinline__ void dense_top(const PairArgs<PT, FP32> &A, uint32_t 
   }
   // the rows stay for the queued cells' path, which looks up this top cell's
   // fine cells from its neighbours: a word per plane (bit y: row y holds fine
-  // cells), then per row its occupancy and the index of its first fine cell
-  uint2 *gr = grows + (uint64_t)slot * rows_stride;
+  // cells) and one of those outside the main component, a fine cell of the
+  // main component, then per row its occupancy, the index of its first fine
+  // cell and its occupancy outside the main component
+  find_main();
+  uint4 *gr = grows + (uint64_t)slot * rows_stride;
+  uint32_t *head = reinterpret_cast<uint32_t *>(gr);
   for (uint32_t z = tid; z < (uint32_t)k; z += nt) {
-    uint32_t plane = 0;
-    for (int y = 0; y < k; y++) plane |= (rows[z * k + y] != 0u ? 1u : 0u) << y;
-    reinterpret_cast<uint32_t *>(gr)[z] = plane;
+    uint32_t plane = 0, prest = 0;
+    for (int y = 0; y < k; y++) {
+      plane |= (rows[z * k + y] != 0u ? 1u : 0u) << y;
+      prest |= (rest[z * k + y] != 0u ? 1u : 0u) << y;
+    }
+    head[z] = plane;
+    head[k + z] = prest;
   }
+  if (tid == 0) head[2 * k] = f + *vmain;
   for (uint32_t j = tid; j < nrow; j += nt)
-    gr[(k + 1) / 2 + j] = make_uint2(rows[j], f + pref[j]);
+    gr[row_head(k) + j] = make_uint4(rows[j], f + pref[j], rest[j], 0u);
   sync();
 }
 
@@ -1036,7 +1078,7 @@ __device__ __forceinline__ void dense_top(const PairArgs<PT, FP32> &A, uint32_t 
 template <class PT, bool FP32, bool VL>
 __global__ void __launch_bounds__(128) k_befriend_dense(
     const PairArgs<PT, FP32> A, uint64_t k3all, const uint2 *__restrict__ dense_range,
-    const uint32_t *__restrict__ big, DevScal *sc, uint32_t nd_cap, uint2 *__restrict__ grows,
+    const uint32_t *__restrict__ big, DevScal *sc, uint32_t nd_cap, uint4 *__restrict__ grows,
     uint32_t kk, uint32_t rows_stride, uint32_t *parent, uint32_t lstride) {
   if (sc->failed) return;  // a sort of this run gave up: its order is not valid
   extern __shared__ uint32_t smem[];
@@ -1075,125 +1117,181 @@ __global__ void __launch_bounds__(128) k_befriend_dense(
   st.flush(A.ctr);
 }
 
-// Whether fine cell a's neighbour top cell in direction o lies within W fine
-// cells of a (s = a's fine coordinate inside its top cell).
-__device__ __forceinline__ bool reaches(int s, int o, int k, int W) {
-  return o == 0 || (o > 0 ? s >= k - W : s <= W - 1);
+// The forward top cells (and a's own, bit 0) that hold cells within W of fine
+// cell a: along an axis the lower (upper) neighbour when a lies within W cells
+// of that face and the neighbour exists.
+__device__ __forceinline__ uint32_t reached_tops(const Geom &g, int W, const int (&t)[3],
+                                                 const int (&s)[3]) {
+  // the neighbours (bits in kFwd's order) at offset -1, 0 and +1 along each axis
+  constexpr uint32_t at[3][3] = {
+      {0x0924, 0x1249, 0x2492},
+      {0x00e0, 0x0703, 0x381c},
+      {0x0000, 0x001f, 0x3fe0}};
+  uint32_t m = 0x3fffu;
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+    m &= at[a][1] | (s[a] < W && t[a] > 0 ? at[a][0] : 0u) |
+         (s[a] >= g.k - W && t[a] + 1 < g.T[a] ? at[a][2] : 0u);
+  return m;
 }
+
+// A warp's candidate (a, b) pairs: fewer than 32 are left over when 32 more may
+// be added.
+constexpr uint32_t kListSlots = 64;
 
 // Candidates of fine cell a are the fine cells b > a (key order, so each
 // unordered pair is visited once) within W fine cells on every axis; they
 // live in a's top cell (after a) and the 13 forward top cells.
 //
-// Fast path, one thread per fine cell: the ranges of the top cells a can
-// reach are loaded at once; when none holds more than kSimple candidate cells
-// (the common case away from clumps), the first of each is loaded at once too
-// and the cell is finished in two L2 round trips.  Other cells are queued for
-// the warp path below.
-constexpr uint32_t kSimple = 2;  // two slot bits per range below
-constexpr uint32_t kSimpleChunk = 1024;  // fine cells per grab of a CTA
+// The sparse path: pairs of a fine cell and a top cell in its reach ("items",
+// about two per cell).  A warp takes 32 fine cells, one per lane, and lists
+// their items; it takes the listed items 32 at a time, one per lane: an item
+// of a dense top cell is queued for k_befriend_cross (a's own top cell, when
+// dense, is k_befriend_dense's), the fine cells of a sparse one that lie in
+// reach are listed as candidates; those are compared with a's root 32 at a
+// time, and the pairs in different components are tested 32 at a time
+// (drain_pairs).  Every level thus works with full warps and keeps 32 or more
+// reads in flight, where a thread per fine cell would step through 14
+// neighbours of which two are in reach.  Bound by read latency (long-scoreboard
+// stalls; 40 registers and 6 CTAs per SM, with the pair tests in a call, were no
+// faster).  At half the 256^3 box (ncu, cold): a thread per fine cell here with
+// whole cells queued for the two phases below, their sparse neighbours read in
+// each, took 0.32 + 0.18 + 0.21 ms; this split 0.33 + 0.07 + 0.06 ms.
 
 template <class PT, bool FP32, bool VL>
-__global__ void __launch_bounds__(kT, 4) k_befriend_simple(
+__global__ void __launch_bounds__(kT, 4) k_befriend_sparse(
     const PairArgs<PT, FP32> A, DevScal *sc, const uint2 *__restrict__ top_range,
-    const uint32_t *__restrict__ top_slot, uint32_t *parent, uint32_t *__restrict__ queue) {
+    const uint32_t *__restrict__ top_slot, uint32_t *parent, uint32_t *__restrict__ q_cell,
+    uint32_t *__restrict__ q_top, uint32_t q_cap) {
   if (sc->failed) return;  // a sort of this run gave up: its order is not valid
   const uint32_t R = sc->R;
-  const uint32_t lane = threadIdx.x & 31;
-  __shared__ uint32_t s_base;
-  __shared__ uint32_t s_first[14][kT];  // first candidate of each top cell, per thread
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5, below = (1u << lane) - 1u;
+  __shared__ uint2 s_item[kT / 32][kListSlots];  // {fine cell, neighbour}
+  __shared__ uint2 s_cand[kT / 32][kListSlots];  // {fine cell, candidate}
   __shared__ uint2 s_pairs[kT / 32][kPairSlots];
-  uint2 *pairs = s_pairs[threadIdx.x >> 5];
+  uint2 *items = s_item[wid], *cands = s_cand[wid], *pairs = s_pairs[wid];
   const GlobalUF uf{parent};
-  uint32_t npair = 0;
+  uint32_t nitem = 0, ncand = 0, npair = 0;
   BfStats st;
-  // CTAs take chunks of consecutive fine cells from a counter: the work per
-  // cell varies a lot across the box (clumps, queued cells), and a static
-  // share would leave the CTAs of the busy regions running alone at the end
+  // Warps take 32 to 128 consecutive fine cells at a time from a counter: the
+  // work per cell varies a lot across the box (clumps, empty neighbourhoods).
+  // Whole CTAs taking 1024 cells, with two barriers a chunk, were 15 % slower.
+  const uint32_t warps = gridDim.x * (kT / 32);
+  const uint32_t step = R >= warps * 256 ? 128u : 32u;
   while (true) {
-    if (threadIdx.x == 0) s_base = atomicAdd(&sc->next_simple, kSimpleChunk);
-    __syncthreads();
-    const uint32_t base = s_base;
-    __syncthreads();
-    // past the last chunk, the pairs still listed are tested
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(&sc->next_simple, step);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    // past the last chunk, what is left in the lists
     const bool last = base >= R;
-    const uint32_t end = last ? base + 1 : min(base + kSimpleChunk, R);
-    for (uint32_t a0 = base + (threadIdx.x & ~31u); a0 < end || last; a0 += kT) {
-      const uint32_t a = a0 + lane;
-      int gx = 0, gy = 0, gz = 0, W = 0;
-      bool queued = false;
-      // candidate slots: bit 2 nb + q stands for fine cell s_first[nb] + q.  The
-      // first fine cell of every range is loaded at once and dropped here when
-      // out of reach; the slots left are visited from one call site below
-      uint32_t m = 0;
-      if (a < end && !last) {
-        const BoxDev &bx = A.boxes[A.run_box[a]];
-        const Geom &g = bx.g;
-        const int k = g.k;
-        W = g.W;
-        const uint64_t pg = A.run_g[a];
-        gx = (int)(pg & kM21);
-        gy = (int)((pg >> 21) & kM21);
-        gz = (int)(pg >> 42);
-        const int tx = div_k(gx, g), ty = div_k(gy, g), tz = div_k(gz, g);
-        const int sx = gx - tx * k, sy = gy - ty * k, sz = gz - tz * k;
-        uint32_t many = 0;  // slots of the ranges, then whether one holds more than kSimple
-#pragma unroll
-        for (int nb = 0; nb < 14; nb++) {
-          const int ux = tx + kFwd[nb][0], uy = ty + kFwd[nb][1], uz = tz + kFwd[nb][2];
-          // a top cell more than W fine cells away from a is skipped without a load
-          if (!(ux < 0 || uy < 0 || ux >= g.T[0] || uy >= g.T[1] || uz >= g.T[2]) &&
-              reaches(sx, kFwd[nb][0], k, W) && reaches(sy, kFwd[nb][1], k, W) &&
-              reaches(sz, kFwd[nb][2], k, W)) {
-            const uint64_t tb = bx.top_base + ((uint64_t)uz * g.T[1] + uy) * g.T[0] + ux;
-            const uint2 tr = top_range[tb];
-            const uint32_t r0 = nb == 0 ? a + 1 : tr.x;
-            uint32_t nn = tr.y > r0 ? tr.y - r0 : 0u;
-            // pairs inside a dense top cell are joined by k_befriend_dense
-            if (nb == 0 && nn && top_slot[tb] != kNone) nn = 0u;
-            s_first[nb][threadIdx.x] = r0;
-            many |= nn > kSimple;
-            m |= min(nn, kSimple) == 0 ? 0u : (nn == 1 ? 1u : 3u) << (2 * nb);
+    const uint32_t end = last ? base + 1 : min(base + step, R);
+    for (uint32_t a0 = base; a0 < end || last; a0 += 32) {
+      uint32_t tops = 0;
+      if (!last && a0 + lane < end) {
+        const Geom &g = A.boxes[A.run_box[a0 + lane]].g;
+        const uint64_t pg = A.run_g[a0 + lane];
+        const int c[3] = {(int)(pg & kM21), (int)((pg >> 21) & kM21), (int)(pg >> 42)};
+        const int t[3] = {div_k(c[0], g), div_k(c[1], g), div_k(c[2], g)};
+        const int f[3] = {c[0] - t[0] * g.k, c[1] - t[1] * g.k, c[2] - t[2] * g.k};
+        tops = reached_tops(g, g.W, t, f);
+      }
+      do {
+        {
+          const uint32_t m = __ballot_sync(0xffffffffu, tops != 0);
+          if (tops) {
+            items[nitem + __popc(m & below)] = make_uint2(a0 + lane, (uint32_t)__ffs(tops) - 1u);
+            tops &= tops - 1u;
+          }
+          nitem += __popc(m);
+        }
+        if (nitem < 32 && !last) continue;
+        // the last 32 items, one per lane
+        __syncwarp();
+        const uint32_t n = min(nitem, 32u);
+        nitem -= n;
+        uint32_t a = 0, r0 = 0, cnt = 0, slot = kNone, nb = 0;
+        int gx = 0, gy = 0, gz = 0, W = 0;
+        if (lane < n) {
+          const uint2 it = items[nitem + lane];
+          a = it.x;
+          nb = it.y;
+          const BoxDev &bx = A.boxes[A.run_box[a]];
+          const Geom &g = bx.g;
+          const uint64_t pg = A.run_g[a];
+          gx = (int)(pg & kM21);
+          gy = (int)((pg >> 21) & kM21);
+          gz = (int)(pg >> 42);
+          W = g.W;
+          const uint64_t tb = bx.top_base +
+                              ((uint64_t)(div_k(gz, g) + kFwd[nb][2]) * g.T[1] +
+                               (uint64_t)(div_k(gy, g) + kFwd[nb][1])) * g.T[0] +
+                              (uint64_t)(div_k(gx, g) + kFwd[nb][0]);
+          const uint2 tr = top_range[tb];
+          slot = top_slot[tb];
+          r0 = nb == 0 ? a + 1 : tr.x;
+          cnt = tr.y > r0 ? tr.y - r0 : 0u;
+          if (nb == 0 && slot != kNone) cnt = 0;  // k_befriend_dense's
+        }
+        const bool dense = cnt != 0 && slot != kNone;
+        const uint32_t qm = __ballot_sync(0xffffffffu, dense);
+        if (qm) {
+          uint32_t at = 0;
+          if (lane == 0) at = atomicAdd(&sc->qcount, (uint32_t)__popc(qm));
+          at = __shfl_sync(0xffffffffu, at, 0) + __popc(qm & below);
+          if (dense && at < q_cap) {  // (past the queue's end the cells are read one by one)
+            q_cell[at] = a;
+            q_top[at] = nb << 28 | slot;
+            cnt = 0;
           }
         }
-        queued = many != 0;
-      }
-      const uint32_t qmask = __ballot_sync(0xffffffffu, queued);
-      if (qmask) {
-        uint32_t at = 0;
-        if (lane == 0) at = atomicAdd(&sc->qcount, (uint32_t)__popc(qmask));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (queued) {
-          queue[at + __popc(qmask & ((1u << lane) - 1u))] = a;
-          m = 0;
-        }
-      }
-      uint32_t ra = kNone;
-      while (last || __any_sync(0xffffffffu, m)) {
-        bool apart = false;
-        uint32_t r = 0;
-        if (m) {
-          const int bit = __ffs(m) - 1;
-          m &= m - 1u;
-          r = s_first[bit >> 1][threadIdx.x] + (uint32_t)(bit & 1);
-          const uint64_t qg = A.run_g[r];
-          st.scan++;
-          if (max(abs((int)(qg & kM21) - gx),
-                  max(abs((int)((qg >> 21) & kM21) - gy), abs((int)(qg >> 42) - gz))) <= W) {
-            st.cand++;
-            if (ra == kNone) ra = __ldcg(parent + a);
-            uint32_t rb = __ldcg(parent + r);
-            st.steps++;
-            if (rb != ra && rb != r) rb = uf_find_n(parent, rb, st.steps);
-            // ra may have been hooked since; it stays in a's component
-            if (rb != ra) ra = uf_find_n(parent, ra, st.steps);
-            apart = rb != ra;
-            if (!apart) st.skips++;
+        for (uint32_t i0 = 0; __any_sync(0xffffffffu, i0 < cnt) || (last && i0 == 0); i0 += 32) {
+          uint32_t todo = 0;  // bit i: fine cell r0 + i0 + i is within reach
+          if (i0 < cnt) {
+            const uint32_t m = min(cnt - i0, 32u);
+#pragma unroll 4
+            for (uint32_t u = 0; u < m; u++) {
+              const uint64_t qg = A.run_g[r0 + i0 + u];
+              const int cheb =
+                  max(abs((int)(qg & kM21) - gx),
+                      max(abs((int)((qg >> 21) & kM21) - gy), abs((int)(qg >> 42) - gz)));
+              if (cheb <= W) todo |= 1u << u;
+            }
+            st.scan += m;
           }
+          const bool end_items = !__any_sync(0xffffffffu, i0 + 32 < cnt);
+          do {
+            const uint32_t m = __ballot_sync(0xffffffffu, todo != 0);
+            if (todo) {
+              cands[ncand + __popc(m & below)] =
+                  make_uint2(a, r0 + i0 + (uint32_t)__ffs(todo) - 1u);
+              todo &= todo - 1u;
+            }
+            ncand += __popc(m);
+            const bool flush = last && end_items && !__any_sync(0xffffffffu, todo != 0);
+            if (ncand < 32 && !flush) continue;
+            do {
+              // the last 32 candidates against their cells' roots
+              __syncwarp();
+              const uint32_t nc = min(ncand, 32u);
+              ncand -= nc;
+              bool apart = false;
+              uint2 c = make_uint2(0u, 0u);
+              if (lane < nc) {
+                c = cands[ncand + lane];
+                st.cand++;
+                st.steps += 2;
+                uint32_t ra = __ldcg(parent + c.x), rb = __ldcg(parent + c.y);
+                if (rb != ra && rb != c.y) rb = uf_find_n(parent, rb, st.steps);
+                if (rb != ra && ra != c.x) ra = uf_find_n(parent, ra, st.steps);
+                apart = rb != ra;
+                if (!apart) st.skips++;
+              }
+              push_pairs<PT, FP32, VL>(A, uf, pairs, npair, apart, c.x, c.y, flush && ncand == 0,
+                                       st);
+            } while (flush && ncand);
+          } while (__any_sync(0xffffffffu, todo != 0));
         }
-        push_pairs<PT, FP32, VL>(A, uf, pairs, npair, apart, a, r, last, st);
-        if (last) break;
-      }
+      } while (__any_sync(0xffffffffu, tops != 0));
       if (last) break;
     }
     if (last) break;
@@ -1201,223 +1299,176 @@ __global__ void __launch_bounds__(kT, 4) k_befriend_simple(
   st.flush(A.ctr);
 }
 
-// The queued fine cells: candidates in the 13 forward top cells (and, when a's
-// own top cell is not dense, in the rest of it).  PHASE 0 visits the
-// candidates within one fine cell, PHASE 1 the farther ones, so that a dense
-// neighbourhood is joined (and compressed) before its far pairs are tried and
-// most of those are found joined.
+// The queued items: fine cells and the dense forward top cells in their reach.
+// PHASE 0 visits the candidates within one fine cell, PHASE 1 the farther
+// ones, so that a dense neighbourhood is joined (and compressed) before its far
+// pairs are tried and most of those are found joined.
 //
 // The kernel is bound by the latency of its table reads and by instruction
-// issue, so a warp works its cells off in three levels, each with all lanes
-// busy and many reads in flight.  It takes 32 queued cells, one per lane (or
-// 32 / G cells of G lanes each when the queue is short, so that it still fills
-// the chip; one atomic per grab), and steps its lanes through the neighbour
-// top cells together, the next neighbour's range and slot being read
-// meanwhile.  1: of a dense neighbour the plane words (bit y: row y of the
-// plane holds fine cells) give the window's non-empty rows, of a sparse one
-// the fine cells give those in reach: one bit each, listed.  2: the listed
+// issue, so a warp works its items off in three levels, each with all lanes
+// busy and many reads in flight.  It takes 32 items, one per lane (or 32 / G
+// items of G lanes each when the queue is short, so that it still fills the
+// chip; one atomic per grab).  1: the neighbour's plane words (bit y: row y of
+// the plane holds fine cells) give the window's non-empty rows -- of those
+// outside the neighbour's main component when that is joined to the cell
+// already, as it mostly is inside clumps -- one bit each, listed.  2: the listed
 // rows are taken 32 at a time, one per lane: the row's word gives the
 // candidates, each compared with its cell's root.  3: candidates in another
 // component are tested 32 at a time (drain_pairs).  Most rows are empty, hence
-// the plane words: with a word read per row the far phase issued 1.2 times the
-// instructions and took 1.25 times as long.  Near and far phase on the 256^3
-// box: 0.94 + 0.73 ms with a warp per cell and a lane per window slot, 0.28 +
-// 0.40 ms so (ncu, cold cache); the whole befriending of the 512^3 box at the
-// 1024^3 box's parameters 36.5 -> 21.5 ms.
-constexpr uint32_t kRowSlots = 64;
-constexpr int kPlanes = 8;  // plane words read at a time
-// floor(i / d) = i * kDiv[d] >> 16 for i < 64, d <= 32
+// the plane words, and most candidates inside clumps are joined already, hence
+// the main components: without them a far phase over whole cells issued 1.4
+// times the instructions.  Befriending of the 256^3 box: 2.80 ms with a warp per
+// cell and a lane per window slot, 1.76 ms with 32 cells a warp, 1.20 ms with
+// items of dense neighbours only; of the 512^3 box at the 1024^3 box's
+// parameters 36.5, 21.5 and 13.6 ms.
+constexpr int kPlanes = 5;  // plane words read at a time
+// floor(i / d) = i * kDiv[d] >> 16 for i < 1200, d <= 32
 __constant__ uint32_t kDiv[33] = {
     0,    65536, 32769, 21846, 16385, 13108, 10923, 9363, 8193, 7282, 6554,
     5958, 5462,  5042,  4682,  4370,  4097,  3856,  3641, 3450, 3277, 3121,
     2979, 2850,  2731,  2622,  2521,  2428,  2341,  2260, 2185, 2115, 2049};
 
 template <class PT, bool FP32, bool VL, int PHASE>
-__global__ void __launch_bounds__(kT, 3) k_befriend(
-    const PairArgs<PT, FP32> A, const uint32_t *__restrict__ queue, DevScal *sc,
-    const uint2 *__restrict__ top_range, const uint32_t *__restrict__ top_slot,
-    const uint2 *__restrict__ grows, uint32_t rows_stride, uint32_t *parent) {
+__global__ void __launch_bounds__(kT, 3) k_befriend_cross(
+    const PairArgs<PT, FP32> A, const uint32_t *__restrict__ q_cell,
+    const uint32_t *__restrict__ q_top, uint32_t q_cap, DevScal *sc,
+    const uint4 *__restrict__ grows, uint32_t rows_stride, uint32_t *parent) {
   if (sc->failed) return;  // a sort of this run gave up: its order is not valid
   __shared__ uint2 s_pairs[kT / 32][kPairSlots];
-  // listed rows: index of the row's word and its columns within reach, or the
-  // fine cell itself and no columns; and the lane of the cell they are for
-  __shared__ uint2 s_row[kT / 32][kRowSlots];
-  __shared__ uint8_t s_lane[kT / 32][kRowSlots];
-  uint2 *pairs = s_pairs[threadIdx.x >> 5], *rows = s_row[threadIdx.x >> 5];
-  uint8_t *rlane = s_lane[threadIdx.x >> 5];
+  // listed rows: {index of the row's word (+ 2^31: only the cells outside the
+  // main component), columns within reach, fine cell, its root}
+  __shared__ uint4 s_row[kT / 32][kListSlots];
+  uint2 *pairs = s_pairs[threadIdx.x >> 5];
+  uint4 *rows = s_row[threadIdx.x >> 5];
   const GlobalUF uf{parent};
-  const uint32_t NQ = sc->qcount;
+  const uint32_t NQ = min(sc->qcount, q_cap);
   if (NQ == 0) return;
   uint32_t *next = PHASE == 0 ? &sc->next0 : &sc->next1;
   const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u;
-  // lanes per cell: the fewest (1, 2, 4, 8) that give every thread of the grid work
+  // lanes per item: the fewest (1, 2, 4, 8) that give every thread of the grid work
   int lg = 0;
   while (lg < 3 && ((uint64_t)NQ << lg) < (uint64_t)gridDim.x * blockDim.x) lg++;
-  const uint32_t G = 1u << lg, sub = lane & (G - 1);
-  // a lane's share of its cell's bits: every G-th
+  const uint32_t G = 1u << lg;
+  // a lane's share of its item's rows: every G-th
   const uint64_t share = (lg == 0 ? ~0ull : lg == 1 ? 0x5555555555555555ull
-                          : lg == 2 ? 0x1111111111111111ull : 0x0101010101010101ull) << sub;
+                          : lg == 2 ? 0x1111111111111111ull : 0x0101010101010101ull)
+                         << (lane & (G - 1));
   uint32_t npair = 0, nrow = 0;
   BfStats st;
   while (true) {
     uint32_t q0 = 0;
     if (lane == 0) q0 = atomicAdd(next, 32u >> lg);
     q0 = __shfl_sync(0xffffffffu, q0, 0);
-    // past the last cells, the pairs still listed are tested
-    const bool last = q0 >= NQ;
+    const bool last = q0 >= NQ;  // past the last items, what is left in the lists
     const uint32_t qi = q0 + (lane >> lg);
-    const bool act = qi < NQ && !last;
-    const uint32_t a = queue[act ? qi : 0u];
-    const BoxDev &bx = A.boxes[A.run_box[a]];
-    const Geom &g = bx.g;
-    const int k = g.k, W = PHASE == 0 ? 1 : g.W;
-    const uint64_t pg = A.run_g[a];
-    const int gx = (int)(pg & kM21), gy = (int)((pg >> 21) & kM21), gz = (int)(pg >> 42);
-    const int tx = div_k(gx, g), ty = div_k(gy, g), tz = div_k(gz, g);
-    const int sx = gx - tx * k, sy = gy - ty * k, sz = gz - tz * k;
-    const uint32_t ra = __ldcg(parent + a);
-    uint2 tr = make_uint2(0u, 0u), tr_next = tr;  // range and slot of a neighbour top cell
-    uint32_t slot = kNone, slot_next = kNone;
-    auto fetch = [&](int nb, uint2 &range, uint32_t &sl) {
-      const int ox = kFwd[nb][0], oy = kFwd[nb][1], oz = kFwd[nb][2];
-      const int ux = tx + ox, uy = ty + oy, uz = tz + oz;
-      range = make_uint2(0u, 0u);
-      sl = kNone;
-      if (act && !(ux < 0 || uy < 0 || ux >= g.T[0] || uy >= g.T[1] || uz >= g.T[2]) &&
-          reaches(sx, ox, k, W) && reaches(sy, oy, k, W) && reaches(sz, oz, k, W)) {
-        const uint64_t tb = bx.top_base + ((uint64_t)uz * g.T[1] + uy) * g.T[0] + ux;
-        range = top_range[tb];
-        sl = top_slot[tb];
-      }
-    };
-    if (!last) fetch(0, tr, slot);
-#pragma unroll 1
-    for (int nb = last ? 14 : 0; nb < 15; nb++) {  // (nb = 14: what is left in the lists)
-      if (nb < 13) fetch(nb + 1, tr_next, slot_next);
-      // items of this neighbour: fine cells (sparse), or rows of the window (dense)
-      const uint32_t r0 = nb == 0 ? a + 1 : tr.x;
-      const uint2 *gr = nullptr;
-      int cx = 0, cy = 0, cz = 0;         // a in the neighbour's own fine coordinates
-      int y0 = 0, ny = 1, z0 = 0, nz = 0;  // the window's rows there
-      uint32_t cnt = 0, chunk = 32;       // items (rows or cells) and how many at a time
-      if (nb < 14 && r0 < tr.y) {
-        if (slot == kNone) {
-          cnt = tr.y - r0;
-        } else if (nb != 0) {  // pairs inside a dense top cell are k_befriend_dense's
-          gr = grows + (uint64_t)slot * rows_stride;
-          cx = sx - kFwd[nb][0] * k;
-          cy = sy - kFwd[nb][1] * k;
-          cz = sz - kFwd[nb][2] * k;
-          y0 = max(cy - W, 0);
-          ny = min(cy + W, k - 1) - y0 + 1;
-          z0 = max(cz - W, 0);
-          nz = min(cz + W, k - 1) - z0 + 1;
-          cnt = (uint32_t)(ny * nz);
-          // whole planes, as many as kPlanes and 64 bits take
-          chunk = (uint32_t)ny * min((64u * kDiv[ny]) >> 16, (uint32_t)kPlanes);
+    const uint4 *gr = nullptr;
+    bool rest = false;                   // only cells outside its main component
+    uint32_t a = 0, ra = 0, cnt = 0, chunk = 32, reach = 0, inner = 0;
+    int k = 1, cx = 0, cy = 0, cz = 0;   // a in the neighbour's own fine coordinates
+    int y0 = 0, ny = 1, z0 = 0;          // the window's rows there
+    if (qi < NQ && !last) {
+      a = q_cell[qi];
+      const uint32_t it = q_top[qi], nb = it >> 28;
+      gr = grows + (uint64_t)(it & 0x0fffffffu) * rows_stride;
+      const Geom &g = A.boxes[A.run_box[a]].g;
+      k = g.k;
+      const int W = PHASE == 0 ? 1 : g.W;
+      const uint64_t pg = A.run_g[a];
+      const int gx = (int)(pg & kM21), gy = (int)((pg >> 21) & kM21), gz = (int)(pg >> 42);
+      cx = gx - (div_k(gx, g) + kFwd[nb][0]) * k;
+      cy = gy - (div_k(gy, g) + kFwd[nb][1]) * k;
+      cz = gz - (div_k(gz, g) + kFwd[nb][2]) * k;
+      const int x0 = max(cx - W, 0), x1 = min(cx + W, k - 1);
+      y0 = max(cy - W, 0);
+      ny = min(cy + W, k - 1) - y0 + 1;
+      z0 = max(cz - W, 0);
+      const int nz = min(cz + W, k - 1) - z0 + 1;
+      if (x0 <= x1 && ny > 0 && nz > 0) {  // (PHASE 0 may not reach the neighbour)
+        reach = bit_span(x0, x1);
+        // the near columns, which were PHASE 0's in the rows within one row of a
+        if (PHASE == 1 && cx >= -1 && cx <= k)
+          inner = bit_span(max(cx - 1, 0), min(cx + 1, k - 1));
+        // cells of the neighbour's main component are joined to a already?
+        ra = __ldcg(parent + a);
+        uint32_t rm = __ldcg(parent + reinterpret_cast<const uint32_t *>(gr)[2 * k]);
+        st.steps += 2;
+        if (rm != ra) {
+          rm = uf_find_n(parent, rm, st.steps);
+          if (rm != ra) ra = uf_find_n(parent, ra, st.steps);
         }
+        rest = rm == ra;
+        cnt = (uint32_t)(ny * nz);
+        // whole planes, as many as kPlanes and 64 bits take
+        chunk = (uint32_t)ny * min((64u * kDiv[ny]) >> 16, (uint32_t)kPlanes);
       }
-      const uint32_t reach = gr ? bit_span(max(cx - W, 0), min(cx + W, k - 1)) : 0u;
-      // the near columns, which were PHASE 0's in the rows within one row of a
-      const uint32_t inner = PHASE == 1 && gr && cx >= -1 && cx <= k
-                                 ? bit_span(max(cx - 1, 0), min(cx + 1, k - 1)) : 0u;
-      for (uint32_t i0 = 0; nb == 14 || __any_sync(0xffffffffu, i0 < cnt); i0 += chunk) {
-        uint64_t todo = 0;  // bit i: item i0 + i is to be listed
-        if (gr && i0 < cnt) {
-          const uint32_t *planes = reinterpret_cast<const uint32_t *>(gr);
-          const uint32_t span = bit_span(0, ny - 1);
+    }
+    for (uint32_t i0 = 0; __any_sync(0xffffffffu, i0 < cnt) || (last && i0 == 0); i0 += chunk) {
+      uint64_t todo = 0;  // bit i: row i0 + i of the window is to be listed
+      if (i0 < cnt) {
+        const int zz = (int)((i0 * kDiv[ny]) >> 16);
+        const uint32_t *planes =
+            reinterpret_cast<const uint32_t *>(gr) + (rest ? k : 0) + z0 + zz;
+        const uint32_t span = bit_span(0, ny - 1), m = min(chunk, cnt - i0);
 #pragma unroll
-          for (int u = 0; u < kPlanes; u++)
-            if (u * ny < (int)min(chunk, cnt - i0)) {
-              const int z = z0 + (int)((i0 * kDiv[ny]) >> 16) + u;
-              todo |= (uint64_t)((planes[z] >> y0) & span) << (u * ny);
-            }
-          todo &= share;
-          st.window += __popcll(todo);
-        } else if (i0 < cnt) {
-          const uint32_t n = min(cnt - i0, 32u);
-#pragma unroll 4
-          for (uint32_t u = sub; u < n; u += G) {
-            const uint64_t qg = A.run_g[r0 + i0 + u];
-            const int cheb =
-                max(abs((int)(qg & kM21) - gx),
-                    max(abs((int)((qg >> 21) & kM21) - gy), abs((int)(qg >> 42) - gz)));
-            if (cheb <= W && (PHASE == 0 || cheb > 1)) todo |= 1ull << u;
-            st.scan++;
-          }
-        }
-        while (true) {
-          bool add = todo != 0;
-          uint2 e = make_uint2(0u, 0u);
-          if (add) {
-            const uint32_t i = i0 + (uint32_t)__ffsll((long long)todo) - 1u;
-            todo &= todo - 1u;
-            if (gr) {
-              const int zz = (int)((i * kDiv[ny]) >> 16), z = z0 + zz, y = y0 + (int)i - zz * ny;
-              e.x = (uint32_t)(gr - grows) + (uint32_t)((k + 1) / 2 + z * k + y);
-              e.y = PHASE == 1 && max(abs(y - cy), abs(z - cz)) <= 1 ? reach & ~inner : reach;
-              add = e.y != 0;
-            } else {
-              e.x = r0 + i;
-            }
-          }
-          const uint32_t m = __ballot_sync(0xffffffffu, add);
-          if (add) {
-            const uint32_t at = nrow + __popc(m & below);
-            rows[at] = e;
-            rlane[at] = (uint8_t)lane;
-          }
-          nrow += __popc(m);
-          const bool more = __any_sync(0xffffffffu, todo != 0);
-          if (nrow >= 32 || nb == 14) {
-            // the last 32 listed rows, one per lane
-            __syncwarp();
-            const uint32_t n = min(nrow, 32u);
-            nrow -= n;
-            uint32_t bits = 0, occ = 0, first = 0;
-            int own = 0;
-            if (lane < n) {
-              const uint2 w = rows[nrow + lane];
-              own = rlane[nrow + lane];
-              if (w.y) {
-                const uint2 word = grows[w.x];
-                occ = word.x;
-                bits = occ & w.y;
-                first = word.y;
-              } else {
-                bits = 1;
-                first = w.x;
-              }
-            }
-            const uint32_t ca = __shfl_sync(0xffffffffu, a, own);
-            uint32_t cr = __shfl_sync(0xffffffffu, ra, own);
-            do {
-              bool apart = false;
-              uint32_t b = 0;
-              if (bits) {
-                b = first + __popc(occ & ((bits & -bits) - 1u));
-                bits &= bits - 1u;
-                st.cand++;
-                st.steps++;
-                // (PHASE 1: the cached parent may be an older one, which is still
-                // in the candidate's component)
-                uint32_t rb = PHASE == 1 ? __ldca(parent + b) : __ldcg(parent + b);
-                if (rb != cr && rb != b) rb = uf_find_n(parent, rb, st.steps);
-                // cr may have been hooked since; it stays in its cell's component
-                if (rb != cr) cr = uf_find_n(parent, cr, st.steps);
-                apart = rb != cr;
-                if (!apart) st.skips++;
-              }
-              push_pairs<PT, FP32, VL>(A, uf, pairs, npair, apart, ca, b, last, st);
-            } while (__any_sync(0xffffffffu, bits != 0));
-            __syncwarp();
-          }
-          if (!more) break;
-        }
-        if (nb == 14) break;
+        for (int u = 0; u < kPlanes; u++)
+          if (u * ny < (int)m) todo |= (uint64_t)((planes[u] >> y0) & span) << (u * ny);
+        todo &= share;
+        st.window += __popcll(todo);
       }
-      tr = tr_next;
-      slot = slot_next;
+      const bool end_items = !__any_sync(0xffffffffu, i0 < cnt && i0 + chunk < cnt);
+      do {
+        bool add = todo != 0;
+        uint4 e = make_uint4(0u, 0u, a, ra);
+        if (add) {
+          const uint32_t i = i0 + (uint32_t)__ffsll((long long)todo) - 1u;
+          todo &= todo - 1u;
+          const int zz = (int)((i * kDiv[ny]) >> 16), z = z0 + zz, y = y0 + (int)i - zz * ny;
+          e.x = (uint32_t)(gr - grows) + (uint32_t)(row_head(k) + z * k + y) +
+                (rest ? 0x80000000u : 0u);
+          e.y = PHASE == 1 && max(abs(y - cy), abs(z - cz)) <= 1 ? reach & ~inner : reach;
+          add = e.y != 0;
+        }
+        const uint32_t m = __ballot_sync(0xffffffffu, add);
+        if (add) rows[nrow + __popc(m & below)] = e;
+        nrow += __popc(m);
+        const bool flush = last && end_items && !__any_sync(0xffffffffu, todo != 0);
+        if (nrow < 32 && !flush) continue;
+        // the last 32 listed rows, one per lane
+        __syncwarp();
+        const uint32_t n = min(nrow, 32u);
+        nrow -= n;
+        uint32_t bits = 0, occ = 0, first = 0, ca = 0, cr = 0;
+        if (lane < n) {
+          const uint4 w = rows[nrow + lane];
+          const uint4 word = grows[w.x & 0x7fffffffu];
+          occ = word.x;
+          bits = (w.x >> 31 ? word.z : occ) & w.y;
+          first = word.y;
+          ca = w.z;
+          cr = w.w;
+        }
+        do {
+          bool apart = false;
+          uint32_t b = 0;
+          if (bits) {
+            b = first + __popc(occ & ((bits & -bits) - 1u));
+            bits &= bits - 1u;
+            st.cand++;
+            st.steps++;
+            // (PHASE 1: the cached parent may be an older one, which is still
+            // in the candidate's component)
+            uint32_t rb = PHASE == 1 ? __ldca(parent + b) : __ldcg(parent + b);
+            if (rb != cr && rb != b) rb = uf_find_n(parent, rb, st.steps);
+            // cr may have been hooked since; it stays in its cell's component
+            if (rb != cr) cr = uf_find_n(parent, cr, st.steps);
+            apart = rb != cr;
+            if (!apart) st.skips++;
+          }
+          const bool more = __any_sync(0xffffffffu, bits != 0);
+          push_pairs<PT, FP32, VL>(A, uf, pairs, npair, apart, ca, b, flush && !more, st);
+        } while (__any_sync(0xffffffffu, bits != 0));
+        __syncwarp();
+      } while (__any_sync(0xffffffffu, todo != 0));
     }
     if (last) break;
   }
@@ -1913,10 +1964,11 @@ template <class K> unsigned rg(K *kernel, int64_t n) {
 }
 
 // Shared-memory words of one dense top cell: k^3 parents, k^2 bit rows, k^2
-// row prefixes and the count of components.
+// row prefixes, k^2 rows of the cells outside the main component, the count of
+// components and the main one's root.
 uint64_t dense_words(uint64_t k3all) {
   const uint64_t k = (uint64_t)std::llround(std::cbrt((double)k3all));
-  return k3all + 2 * k * k + 1;
+  return k3all + 3 * k * k + 2;
 }
 
 // Warps per CTA of the dense-top kernel: up to 4, each with the words of one
@@ -1926,16 +1978,16 @@ int dense_warps_per_cta(uint64_t k3all) {
   return (int)std::max<uint64_t>(1, std::min<uint64_t>(4, (200u << 10) / per));
 }
 
-// 8-byte words of a dense top cell's occupancy: k plane words of 4 bytes, k^2 rows.
+// 16-byte words of a dense top cell's occupancy: planes, then k^2 rows.
 uint64_t rows_per_top(uint64_t k3all) {
   const uint64_t k = (uint64_t)std::llround(std::cbrt((double)k3all));
-  return (k + 1) / 2 + k * k;
+  return row_head((int)k) + k * k;
 }
 
 // Dense top cells whose planes and rows fit in 4 bytes per processed
 // particle plus 1 GiB.
 int64_t rows_cap_for(int64_t np_cap, uint64_t k3all) {
-  return (int64_t)(((uint64_t)np_cap * 4 + (1ull << 30)) / (rows_per_top(k3all) * 8));
+  return (int64_t)(((uint64_t)np_cap * 4 + (1ull << 30)) / (rows_per_top(k3all) * sizeof(uint4)));
 }
 
 bool capturing(cudaStream_t s) {
@@ -2083,9 +2135,11 @@ void Plan::issue(bool want_member, cudaStream_t s, bool timed) {
   CMH_LAUNCHED();
   mark(2);
   // ---- befriending: dense top cells inside (CTA each) on a second stream
-  // while the sparse fast path runs (both join cells through the lock-free
-  // union-find), then the queued cells' warp path, near then far ----
-  uint32_t *queue = b_rtmp1.as<uint32_t>();  // the keep scan's, free since the emission
+  // while the sparse path runs (both join cells through the lock-free
+  // union-find), then the queued items of dense neighbours, near then far ----
+  // the queue lies in the ingest scans' arrays, free since the emission
+  uint32_t *q_cell = b_rtmp1.as<uint32_t>(), *q_top = b_rtmp2.as<uint32_t>();
+  const uint32_t q_cap = (uint32_t)npc;
   const int dwpc = dense_warps_per_cta(k3all);
   const uint32_t kmax = (uint32_t)std::llround(std::cbrt((double)k3all)), kk = kmax * kmax;
   const uint32_t rows_stride = (uint32_t)rows_per_top(k3all);
@@ -2103,22 +2157,21 @@ void Plan::issue(bool want_member, cudaStream_t s, bool timed) {
                               b_spos.as<SPos<PT>>(), svl, c};
     k_befriend_dense<PT, FP, VL><<<gd, 32 * dwpc, dsm, bf_stream>>>(
         pa, k3all, b_dense_range.as<uint2>(), b_dense_big.as<uint32_t>(), sc, (uint32_t)nd_cap,
-        b_rows.as<uint2>(), kk, rows_stride, b_parent.as<uint32_t>(), (uint32_t)dense_words(k3all));
+        b_rows.as<uint4>(), kk, rows_stride, b_parent.as<uint32_t>(), (uint32_t)dense_words(k3all));
     CMH_LAUNCHED();
     CMH_CUDA(cudaEventRecord(ev_join, bf_stream));
-    k_befriend_simple<PT, FP, VL><<<rg(k_befriend_simple<PT, FP, VL>, npc), kT, 0, s>>>(
-        pa, sc, b_top_range.as<uint2>(), b_top_slot.as<uint32_t>(), b_parent.as<uint32_t>(), queue);
+    k_befriend_sparse<PT, FP, VL><<<rg(k_befriend_sparse<PT, FP, VL>, npc), kT, 0, s>>>(
+        pa, sc, b_top_range.as<uint2>(), b_top_slot.as<uint32_t>(), b_parent.as<uint32_t>(),
+        q_cell, q_top, q_cap);
     CMH_LAUNCHED();
     CMH_CUDA(cudaStreamWaitEvent(s, ev_join, 0));
-    k_befriend<PT, FP, VL, 0><<<rg(k_befriend<PT, FP, VL, 0>, npc * 8), kT, 0, s>>>(
-        pa, queue, sc, b_top_range.as<uint2>(), b_top_slot.as<uint32_t>(), b_rows.as<uint2>(),
-        rows_stride, b_parent.as<uint32_t>());
+    k_befriend_cross<PT, FP, VL, 0><<<rg(k_befriend_cross<PT, FP, VL, 0>, npc * 8), kT, 0, s>>>(
+        pa, q_cell, q_top, q_cap, sc, b_rows.as<uint4>(), rows_stride, b_parent.as<uint32_t>());
     CMH_LAUNCHED();
     k_compress<<<rg(k_compress, npc), kT, 0, s>>>(b_parent.as<uint32_t>(), sc);
     CMH_LAUNCHED();
-    k_befriend<PT, FP, VL, 1><<<rg(k_befriend<PT, FP, VL, 1>, npc * 8), kT, 0, s>>>(
-        pa, queue, sc, b_top_range.as<uint2>(), b_top_slot.as<uint32_t>(), b_rows.as<uint2>(),
-        rows_stride, b_parent.as<uint32_t>());
+    k_befriend_cross<PT, FP, VL, 1><<<rg(k_befriend_cross<PT, FP, VL, 1>, npc * 8), kT, 0, s>>>(
+        pa, q_cell, q_top, q_cap, sc, b_rows.as<uint4>(), rows_stride, b_parent.as<uint32_t>());
     CMH_LAUNCHED();
   };
   if (fp32 && varlink) befriend(std::true_type{}, std::true_type{});
@@ -2305,7 +2358,7 @@ void Plan::prepare(const std::vector<BoxSpec> &specs, bool want_member) {
   b_top_slot.ensure(n_top * 4);
   b_rtmp1.ensure(npc * 4);
   b_rtmp2.ensure(npc * 4);
-  b_rows.ensure((size_t)nd_cap * rows_per_top(k3all) * sizeof(uint2));
+  b_rows.ensure((size_t)nd_cap * rows_per_top(k3all) * sizeof(uint4));
   b_dense_range.ensure((size_t)nd_cap * sizeof(uint2));
   b_dense_big.ensure((size_t)nd_cap * sizeof(uint32_t));
   b_parent.ensure(npc * 4);

@@ -113,9 +113,9 @@ typedef struct cmh_stats {
   int64_t n_unions;        /* ... joined by a linked particle pair            */
   int64_t n_find_steps;    /* union-find parent loads while befriending       */
   int64_t n_scan_iters;    /* fine cells scanned in sparse top cells          */
-  int64_t n_window_iters;  /* window slots visited in dense top cells         */
+  int64_t n_window_iters;  /* rows of fine cells visited in dense top cells   */
   int64_t n_dense_tops;    /* top cells joined in shared memory (dense)       */
-  int64_t n_queued;        /* fine cells sent to the warp-per-cell path       */
+  int64_t n_queued;        /* (fine cell, dense top cell in reach) pairs      */
   int64_t n_big_tops;      /* dense top cells joined by a whole CTA           */
 } cmh_stats;
 
