@@ -981,10 +981,12 @@ __device__ __forceinline__ void dense_top(const PairArgs<PT, FP32> &A, uint32_t 
     sync();
   };
   uint32_t npair = 0;
-  for (int pass = 0; pass < 2; pass++) {
-    // pass 0: cells at Chebyshev distance 1; pass 1: those at 2 and more
-    const int Wp = pass == 0 ? 1 : W;
-    if (pass == 1) find_main();
+  for (int pass = 0; pass < 3; pass++) {
+    // pass 0: cells that share a face; pass 1: the others at Chebyshev distance
+    // 1; pass 2: those at 2 and more.  Inside a clump the faces join nearly
+    // everything, which leaves the other passes little to test.
+    const int Wp = pass == 2 ? W : 1;
+    if (pass >= 1) find_main();
     for (uint32_t i0 = tid & ~31u;; i0 += nt) {
       // past the warp's cells (or once one component is left; one answer for
       // the whole warp) the pairs still listed are tested
@@ -1001,18 +1003,21 @@ __device__ __forceinline__ void dense_top(const PairArgs<PT, FP32> &A, uint32_t 
         sz = gz - div_k(gz, g) * k;
         ri = lfind(lpar, i);  // may go stale: re-found before a pair is listed
       }
-      const bool main = pass == 1 && act && ri == lfind(lpar, *vmain);
-      // columns within reach, and the near ones (|dx| <= 1)
+      const bool main = pass >= 1 && act && ri == lfind(lpar, *vmain);
+      // columns within reach, the near ones (|dx| <= 1) and a's own
       const uint32_t reach = bit_span(max(sx - W, 0), min(sx + W, k - 1));
       const uint32_t near = bit_span(max(sx - 1, 0), min(sx + 1, k - 1));
-      const uint32_t after = sx == 31 ? 0u : (0xffffffffu << (sx + 1));
+      const uint32_t own = 1u << sx, after = sx == 31 ? 0u : (0xffffffffu << (sx + 1));
       // the forward rows (dz, dy) in order, from (0, 0) to (Wp, Wp)
       for (int dz = 0, dy = 0; dz <= (last ? 0 : Wp); dy == Wp ? (dz++, dy = -Wp) : dy++) {
-        const int ty = sy + dy, tz = sz + dz;
+        const int ty = sy + dy, tz = sz + dz, off = abs(dy) + dz;  // off 0: a's own row
+        if (pass == 0 && off > 1 && !last) continue;
         uint32_t occ = 0, bits = 0, before = 0;
         if (act && ty >= 0 && ty < k && tz < k) {
-          uint32_t m = pass == 0 ? near : max(abs(dy), dz) <= 1 ? reach & ~near : reach;
-          if (dz == 0 && dy == 0) m &= after;  // forward only in a's own row
+          uint32_t m = max(abs(dy), dz) > 1 ? reach : pass == 2 ? reach & ~near : near;
+          if (pass == 0 && off == 1) m = own;
+          if (pass == 1 && off <= 1) m &= off == 0 ? 0u : ~own;
+          if (off == 0) m &= after;  // forward only
           const uint32_t row = (uint32_t)(tz * k + ty);
           occ = rows[row];
           bits = (main ? rest[row] : occ) & m;
