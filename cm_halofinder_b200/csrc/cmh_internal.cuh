@@ -92,34 +92,51 @@ struct SortWaits {
   uint32_t stall_tile = 0xffffffffu;
 };
 
-// Stable LSD radix sort of (key u64, value u32) pairs on the low `bits` key
-// bits.  Result lands in keys/vals (the alt buffers are scratch); `tmp`
-// holds the digit counts and the tiles' look-back states.
+// The digits of a sort's passes: shift in the original key and width (8 or
+// 9 bits); pass p's digit counts take kRadixBins words from kRadixBins p on.
+constexpr int kRadixBins = 512;
+constexpr int kRadixPasses = 8;
+struct PassDigits {
+  int passes;
+  int shift[kRadixPasses];
+  int width[kRadixPasses];
+};
+
+// The order of n records by the low `bits` bits (at least one pass is made) of
+// a 64-bit key that each holds `key_at` bytes in: the records' indices, in
+// stable key order, end in vals_b after an odd number of passes, else in
+// vals_a.  Both key buffers are scratch: the first pass reads the records and
+// their indices need no array, and the later passes move 32-bit key words,
+// with 9-bit digits where that saves a pass.
+// The caller counts the digits of radix_order_plan(bits) of all records into
+// the counts as it writes them.
 // `n` sizes the launches; with `n_dev` set, the element count is read from
 // device memory (at most n), so the sort needs no host synchronisation.
-// `tmp` must already hold radix_sort_scratch(n) bytes when the sort is
-// captured in a graph; `giveups` (device) counts capped look-back waits.
-// With copy_back false and an odd number of 8-bit passes the result stays in
-// keys_alt/vals_alt (no copy).
-void radix_sort_u64_u32(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt,
-                        uint32_t *vals_alt, int64_t n, const uint32_t *n_dev, int bits,
-                        DevBuf &tmp, unsigned int *giveups, cudaStream_t s,
-                        bool copy_back = true, SortWaits waits = SortWaits{});
-// The values of the same sort, in key order, without the sorted keys: both
-// key buffers end as scratch (the later passes move 32-bit key words, with
-// 9-bit digits where that saves a pass), and the values end in vals_alt
-// after an odd number of passes (radix_order_passes), else in vals.
-int radix_order_passes(int bits);
-void radix_order_u64_u32(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt,
-                         uint32_t *vals_alt, int64_t n, const uint32_t *n_dev, int bits,
-                         DevBuf &tmp, unsigned int *giveups, cudaStream_t s,
-                         SortWaits waits = SortWaits{});
-// Same for 32-bit keys.
+// `giveups` (device) counts capped look-back waits.
+//
+// Scratch: kRadixCounts cleared words of digit counts (and what follows from
+// them), and the tiles' look-back states -- radix_state_bytes(n) bytes that the
+// sort clears before each pass, or, where every pass has its own
+// (radix_states_apart: up to 64 MB in all), the bytes it gives, cleared by the
+// caller.
+constexpr int kRadixCounts = 2 * kRadixPasses * kRadixBins + kRadixPasses;
+struct RadixTmp {
+  uint64_t *state;
+  uint32_t *counts;
+  bool apart;
+};
+size_t radix_state_bytes(int64_t n);
+bool radix_states_apart(int64_t n, int bits, size_t *bytes);
+PassDigits radix_order_plan(int bits);
+void radix_order_records(const void *records, uint32_t stride, uint32_t key_at, uint64_t *keys_a,
+                         uint32_t *vals_a, uint64_t *keys_b, uint32_t *vals_b, int64_t n,
+                         const uint32_t *n_dev, int bits, RadixTmp tmp, unsigned int *giveups,
+                         cudaStream_t s, SortWaits waits = SortWaits{});
+// Stable LSD radix sort of (key, value) pairs, 32-bit keys; the result lands in
+// keys/vals (the alt buffers are scratch).
 void radix_sort_u32_u32(uint32_t *keys, uint32_t *vals, uint32_t *keys_alt,
                         uint32_t *vals_alt, int64_t n, const uint32_t *n_dev, int bits,
-                        DevBuf &tmp, unsigned int *giveups, cudaStream_t s,
+                        RadixTmp tmp, unsigned int *giveups, cudaStream_t s,
                         SortWaits waits = SortWaits{});
-// Scratch bytes of a sort of up to n keys.
-size_t radix_sort_scratch(int64_t n);
 
 }  // namespace cmh

@@ -20,6 +20,23 @@ template <> struct __align__(16) SPos<double> {
   uint32_t src, pad;
 };
 
+// Processed particle as the ingest emits it: position, source, sort key and
+// processing index in one record (a whole 32-byte sector for float positions),
+// so that a record goes to its place in one write and is gathered in one read.
+template <class PT> struct PRec;
+template <> struct __align__(32) PRec<float> {
+  float x, y, z;
+  uint32_t src;
+  uint64_t key;
+  uint32_t proc, pad;
+};
+template <> struct __align__(16) PRec<double> {
+  double x, y, z;
+  uint64_t key;
+  uint32_t src, proc;
+  uint64_t pad;
+};
+
 // Geometry and run parameters of one domain, passed by value to kernels.
 struct Geom {
   double lo[3], hi[3];   // Lmin, Lmax
@@ -39,6 +56,11 @@ struct Geom {
   int W;                 // fine-cell reach: cells more than W apart never link
   int G[3];              // fine cells per axis
   int T[3];              // top cells per axis
+  // Ingest, in the position type's own values: a particle is inside the domain
+  // when dom_lo <= x <= dom_hi on every axis; its image by -L (+L) along an
+  // axis stays in the shell when x >= img_lo (x <= img_hi).  Both hold exactly:
+  // the image's stored coordinate is monotonic in x.
+  double dom_lo[3], dom_hi[3], img_lo[3], img_hi[3];
   uint64_t k3;           // k^3
   uint32_t kmul;         // floor(2^32 / k) + 1: x / k == umulhi(x, kmul) for x < 2^27
   int props;             // CMH_PROP_* bits
@@ -63,6 +85,10 @@ struct BoxDev {
   uint64_t top_base;    // first index of the box's top cells in the run's tables
   uint32_t n;           // input particles of the box
   int vel_f64;          // velocities are double
+  uint32_t tile_base;   // first ingest tile of the box
+  uint32_t bucket_base; // first bucket of the box
+  uint32_t nbucket;     // its buckets, and their count over the padded box's height
+  float bucket_scale;
 };
 
 // Device-side sizes of one run: nothing is read back by the host until the
@@ -210,7 +236,7 @@ __device__ __forceinline__ int div_k(int x, const Geom &g) {
 // along the axis, far inside the 2^-20 margin that sizes h.
 __device__ __forceinline__ int fine_index(double x, double rmin, double inv_h, int G) {
   double q = __dmul_rn(__dsub_rn(x, rmin), inv_h);
-  int g = (int)floor(q);
+  int g = __double2int_rd(q);
   g = g < 0 ? 0 : g;
   return g >= G ? G - 1 : g;
 }

@@ -41,6 +41,15 @@ struct Plan : public cmh_plan {
   // shape of the current run
   std::vector<BoxDev> boxes_host;
   int64_t n_total = 0;
+  int ingest_per = 1;    // particles per thread of the ingest
+  uint32_t n_tiles = 0;  // ingest tiles of the boxes
+  int n_buckets = 1;     // buckets of the emission
+  // byte offsets in `scal` of the counters, the per-box numbers, the buckets and
+  // the sorts' digit counts, and its bytes
+  size_t at_ctr = 0, at_boxd = 0, at_bucket = 0, at_counts = 0, small_bytes = 0;
+  std::vector<unsigned char> small_host;
+  bool cell_states_apart = false;  // each pass of the cell sort has its own tile states
+  size_t cell_state_bytes = 0;
   uint64_t n_top = 0, k3all = 1;
   int key_bits = 0, hs = 7, props = 0;
   bool varlink = false;             // some box has a variable linking length
@@ -58,7 +67,7 @@ struct Plan : public cmh_plan {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaStream_t bf_stream = nullptr;  // the dense top cells' kernel, beside the sparse one
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  cudaEvent_t ev_cleared = nullptr, ev_emitted = nullptr, ev_cleared2 = nullptr;
+  cudaEvent_t ev_cleared = nullptr;
   cudaEvent_t stage_ev[7] = {};  // boundaries between the eight stages
   // the recorded graphs of the last two run shapes (two, so that runs that
   // alternate between the two host-input buffers both replay)
@@ -99,11 +108,11 @@ struct Plan : public cmh_plan {
   const uint64_t *samp_ids = nullptr;
 
   // workspace
-  DevBuf scal, ctr, scan_tmp, scan_tmp2, sort_tmp, ltab_dev, b_boxes, b_boxd;
-  DevBuf b_keys, b_keys_alt, b_vals, b_vals_alt, b_ppos, b_spos, b_svl;
-  DevBuf b_run_start, b_run_box, b_top_range, b_top_slot, b_rtmp1, b_rtmp2;
+  DevBuf scal, scan_tmp, sort_tmp, b_tiles, ltab_dev, b_boxes;
+  DevBuf b_keys, b_keys_alt, b_vals, b_vals_alt, b_recs, b_spos, b_svl;
+  DevBuf b_run_box, b_top_range, b_top_slot;
   DevBuf b_rows, b_dense_range, b_dense_big;
-  DevBuf b_parent, b_count, b_head, b_cand_of_root, b_cand_root, b_sums, b_warn;
+  DevBuf b_count, b_head, b_cand_of_root, b_cand_root, b_sums, b_warn;
   DevBuf b_okeys, b_ovals, b_okeys_alt, b_ovals_alt;
   DevBuf b_props, b_head_out, b_cat_of_cand, b_member, b_member_proc, b_member_pos;
   DevBuf in_pos[2], in_vel[2];  // device copies of host-resident particles
@@ -111,10 +120,10 @@ struct Plan : public cmh_plan {
 
   // every workspace buffer, for release and for the graph signature
   template <class F> void each_buf(F f) {
-    DevBuf *all[] = {&scal, &ctr, &scan_tmp, &scan_tmp2, &sort_tmp, &ltab_dev, &b_boxes, &b_boxd,
-                     &b_keys, &b_keys_alt, &b_vals, &b_vals_alt, &b_ppos, &b_spos, &b_svl,
-                     &b_run_start, &b_run_box, &b_top_range, &b_top_slot,
-                     &b_rtmp1, &b_rtmp2, &b_rows, &b_dense_range, &b_dense_big, &b_parent, &b_count,
+    DevBuf *all[] = {&scal, &scan_tmp, &sort_tmp, &b_tiles, &ltab_dev, &b_boxes,
+                     &b_keys, &b_keys_alt, &b_vals, &b_vals_alt, &b_recs, &b_spos, &b_svl,
+                     &b_run_box, &b_top_range, &b_top_slot,
+                     &b_rows, &b_dense_range, &b_dense_big, &b_count,
                      &b_head, &b_cand_of_root, &b_cand_root, &b_sums, &b_warn,
                      &b_okeys, &b_ovals, &b_okeys_alt, &b_ovals_alt, &b_props,
                      &b_head_out, &b_cat_of_cand, &b_member, &b_member_proc, &b_member_pos,

@@ -23,8 +23,8 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kIPT = 16;
 constexpr int kTile = kThreads * kIPT;  // 4096
 constexpr int kBins = 256;      // 8-bit digits
-constexpr int kMaxBins = 512;   // 9-bit digits
-constexpr int kMaxPasses = 8;
+constexpr int kMaxBins = kRadixBins;  // 9-bit digits
+constexpr int kMaxPasses = kRadixPasses;
 // Tile states of the look-back, one 64-bit word per (tile, digit): the flag
 // in the high half, the count in the low half, written in one store.
 constexpr uint64_t kAggregate = 1ull << 32;  // count = the tile's own keys of the digit
@@ -34,14 +34,6 @@ template <int BINS = kBins, class K>
 __device__ __forceinline__ uint32_t digit_of(K k, int shift) {
   return (uint32_t)(k >> shift) & (BINS - 1);
 }
-
-// The digits of a sort's passes: shift in the original key and width (8 or
-// 9 bits).
-struct PassDigits {
-  int passes;
-  int shift[kMaxPasses];
-  int width[kMaxPasses];
-};
 
 __device__ __forceinline__ uint32_t warp_inclusive(uint32_t v) {
   const int lane = threadIdx.x & 31;
@@ -54,11 +46,22 @@ __device__ __forceinline__ uint32_t warp_inclusive(uint32_t v) {
 }
 
 
+// Where a pass reads its keys: an array, or a field of records `stride` bytes
+// apart (their values are then the records' indices).
+template <class K>
+struct KeySource {
+  const K *keys;
+  uint32_t stride;  // bytes from one key to the next
+  __device__ __forceinline__ K operator[](int64_t i) const {
+    return *reinterpret_cast<const K *>(reinterpret_cast<const unsigned char *>(keys) +
+                                        (uint64_t)i * stride);
+  }
+};
+
 // All digit histograms of the sort in one read of the keys: pass p's
 // counters at ghist[kMaxBins p].
 template <class K>
-__global__ void __launch_bounds__(kThreads) k_rs_upfront(const K *__restrict__ keys,
-                                                         int64_t n_cap,
+__global__ void __launch_bounds__(kThreads) k_rs_upfront(KeySource<K> keys, int64_t n_cap,
                                                          const uint32_t *__restrict__ n_dev,
                                                          PassDigits pd,
                                                          uint32_t *__restrict__ ghist) {
@@ -145,7 +148,7 @@ __device__ __forceinline__ uint64_t load_state(const uint64_t *p) {
 // 4 CTAs per SM.
 template <class K, class KO, int BINS>
 __global__ void __launch_bounds__(kSThreads, (sizeof(K) == 4 && BINS == BINS) ? 4 : 3) k_rs_scatter(
-    const K *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
+    KeySource<K> keys_in, const uint32_t *__restrict__ vals_in,
     KO *__restrict__ keys_out, uint32_t *__restrict__ vals_out, int64_t n_cap,
     const uint32_t *__restrict__ n_dev, int shift, int out_shift,
     const uint32_t *__restrict__ goff,
@@ -170,7 +173,7 @@ __global__ void __launch_bounds__(kSThreads, (sizeof(K) == 4 && BINS == BINS) ? 
     const int64_t i = base + (int64_t)warp * 32 * kSIPT + j * 32 + lane;
     const bool valid = i < n;
     k[j] = valid ? keys_in[i] : K(0);
-    v[j] = valid ? vals_in[i] : 0u;
+    v[j] = valid ? (vals_in ? vals_in[i] : (uint32_t)i) : 0u;
   }
   // the tile's digit counts first, published before the ranking so that
   // the higher tiles' look-back finds them early
@@ -301,7 +304,7 @@ PassDigits plan_passes(int bits, bool narrow, int *wide) {
   PassDigits pd{};
   int m = (bits + 7) / 8, nine = 0, q = 0;
   if (narrow) {
-    m = std::min((bits + 7) / 8, std::max(1, (bits - 32 + 7) / 8));
+    m = std::max(1, std::min((bits + 7) / 8, (bits - 32 + 7) / 8));
     const int rest = std::max(0, bits - 8 * m);
     const int q8 = (rest + 7) / 8, q9 = (rest + 8) / 9;
     q = q9 < q8 ? q9 : q8;
@@ -321,116 +324,126 @@ PassDigits plan_passes(int bits, bool narrow, int *wide) {
 // With `narrow` (64-bit keys whose sorted order, not their sorted copy, is
 // wanted) the first m passes read 64-bit keys; pass m-1 writes key >> 8m as
 // 32-bit words and the later passes sort those on the digits that are left.
+// The first pass reads `src` (and vals, or takes the indices when vals is
+// null) and writes the b buffers, the next the a buffers, and so on in turn.
 template <class K>
-void radix_sort_impl(K *keys, uint32_t *vals, K *keys_alt, uint32_t *vals_alt, int64_t n,
-                     const uint32_t *n_dev, int bits, DevBuf &tmp, unsigned int *giveups,
-                     cudaStream_t s, bool copy_back, bool narrow, SortWaits waits) {
-  if (bits <= 0) return;
+int radix_passes_run(KeySource<K> first, const uint32_t *first_vals, K *keys_a, uint32_t *vals_a,
+                     K *keys_b, uint32_t *vals_b, int64_t n, const uint32_t *n_dev, int bits,
+                     RadixTmp tmp, unsigned int *giveups, cudaStream_t s, bool narrow,
+                     bool counted, SortWaits waits) {
   if (bits > (int)(8 * sizeof(K)) || (bits + 7) / 8 > kMaxPasses)
     fail(CMH_ERR_INVALID_ARGUMENT, "radix sort: key bits out of range");
-  if (narrow && (copy_back || sizeof(K) != 8))
-    fail(CMH_ERR_INVALID_ARGUMENT, "radix sort: narrowing applies to 64-bit keys left unsorted");
   int m = 0;
   const PassDigits pd = plan_passes(bits, narrow, &m);
   const int passes = pd.passes;
-  if (n <= 1) {
-    // nothing to order; still leave the data where the caller expects it
-    if (!copy_back && passes % 2 == 1 && n == 1) {
-      CMH_CUDA(cudaMemcpyAsync(keys_alt, keys, sizeof(K), cudaMemcpyDeviceToDevice, s));
-      CMH_CUDA(cudaMemcpyAsync(vals_alt, vals, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-    }
-    return;
-  }
   const int64_t ntiles = (n + kTile - 1) / kTile;
   if (ntiles >= 0xffffffffll) fail(CMH_ERR_CAPACITY, "radix sort: too many tiles");
-  // tmp: tile states (ntiles x 512 u64) | digit counts | digit offsets | tile counters
-  const size_t state_bytes = (size_t)ntiles * kMaxBins * sizeof(uint64_t);
-  const size_t small = (size_t)(2 * kMaxPasses * kMaxBins + kMaxPasses) * sizeof(uint32_t);
-  tmp.ensure(radix_sort_scratch(n));
-  uint64_t *state = tmp.as<uint64_t>();
-  uint32_t *ghist = reinterpret_cast<uint32_t *>(tmp.as<unsigned char>() + state_bytes);
+  uint64_t *state = tmp.state;
+  uint32_t *ghist = tmp.counts;  // digit counts | digit offsets | tile counters
   uint32_t *goff = ghist + kMaxPasses * kMaxBins;
   uint32_t *tile_ctr = goff + kMaxPasses * kMaxBins;
   set_scatter_smem(s);
-  CMH_CUDA(cudaMemsetAsync(ghist, 0, small, s));
-  k_rs_upfront<K><<<grid_resident(reinterpret_cast<const void *>(k_rs_upfront<K>), kThreads, 0,
-                                  n),
-                    kThreads, 0, s>>>(keys, n, n_dev, pd, ghist);
-  CMH_LAUNCHED();
+  if (!counted) {
+    k_rs_upfront<K><<<grid_resident(reinterpret_cast<const void *>(k_rs_upfront<K>), kThreads, 0,
+                                    n),
+                      kThreads, 0, s>>>(first, n, n_dev, pd, ghist);
+    CMH_LAUNCHED();
+  }
   k_rs_offsets<<<passes, kMaxBins, 0, s>>>(ghist, goff);
   CMH_LAUNCHED();
-  void *src_k = keys, *dst_k = keys_alt;
-  uint32_t *src_v = vals, *dst_v = vals_alt;
+  const void *src_k = first.keys;
+  const uint32_t *src_v = first_vals;
+  uint32_t src_stride = first.stride;
+  void *out_k[2] = {keys_b, keys_a};
+  uint32_t *out_v[2] = {vals_b, vals_a};
   for (int p = 0; p < passes; p++) {
     const int bins = 1 << pd.width[p];
-    CMH_CUDA(cudaMemsetAsync(state, 0, (size_t)ntiles * bins * sizeof(uint64_t), s));
+    if (!tmp.apart)
+      CMH_CUDA(cudaMemsetAsync(state, 0, (size_t)ntiles * bins * sizeof(uint64_t), s));
     const uint32_t *go = goff + p * kMaxBins;
+    void *dst_k = out_k[p % 2];
+    uint32_t *dst_v = out_v[p % 2];
     // the stall hook applies to the first pass only
     const SortWaits wp{waits.spin_cap, p == 0 ? waits.stall_tile : 0xffffffffu};
+    const KeySource<K> sk{static_cast<const K *>(src_k), src_stride};
+    const KeySource<uint32_t> s4{static_cast<const uint32_t *>(src_k), src_stride};
     if (p < m && !(narrow && p == m - 1)) {
       k_rs_scatter<K, K, kBins><<<(unsigned)ntiles, kSThreads, sizeof(ScatterSmem<K, kBins>), s>>>(
-          static_cast<const K *>(src_k), src_v, static_cast<K *>(dst_k), dst_v, n, n_dev,
-          pd.shift[p], 0, go, state, tile_ctr + p, giveups, wp);
+          sk, src_v, static_cast<K *>(dst_k), dst_v, n, n_dev, pd.shift[p], 0, go, state,
+          tile_ctr + p, giveups, wp);
+      src_stride = sizeof(K);
     } else if (p < m) {
       k_rs_scatter<K, uint32_t, kBins>
           <<<(unsigned)ntiles, kSThreads, sizeof(ScatterSmem<K, kBins>), s>>>(
-              static_cast<const K *>(src_k), src_v, static_cast<uint32_t *>(dst_k), dst_v, n,
-              n_dev, pd.shift[p], 8 * m, go, state, tile_ctr + p, giveups, wp);
+              sk, src_v, static_cast<uint32_t *>(dst_k), dst_v, n, n_dev, pd.shift[p], 8 * m, go,
+              state, tile_ctr + p, giveups, wp);
+      src_stride = sizeof(uint32_t);
     } else if (bins == kMaxBins) {
       k_rs_scatter<uint32_t, uint32_t, kMaxBins>
           <<<(unsigned)ntiles, kSThreads, sizeof(ScatterSmem<uint32_t, kMaxBins>), s>>>(
-              static_cast<const uint32_t *>(src_k), src_v, static_cast<uint32_t *>(dst_k), dst_v,
-              n, n_dev, pd.shift[p] - 8 * m, 0, go, state, tile_ctr + p, giveups, wp);
+              s4, src_v, static_cast<uint32_t *>(dst_k), dst_v, n, n_dev, pd.shift[p] - 8 * m, 0,
+              go, state, tile_ctr + p, giveups, wp);
     } else {
       k_rs_scatter<uint32_t, uint32_t, kBins>
           <<<(unsigned)ntiles, kSThreads, sizeof(ScatterSmem<uint32_t, kBins>), s>>>(
-              static_cast<const uint32_t *>(src_k), src_v, static_cast<uint32_t *>(dst_k), dst_v,
-              n, n_dev, pd.shift[p] - 8 * m, 0, go, state, tile_ctr + p, giveups, wp);
+              s4, src_v, static_cast<uint32_t *>(dst_k), dst_v, n, n_dev, pd.shift[p] - 8 * m, 0,
+              go, state, tile_ctr + p, giveups, wp);
     }
     CMH_LAUNCHED();
-    std::swap(src_k, dst_k);
-    std::swap(src_v, dst_v);
+    if (tmp.apart) state += (size_t)ntiles * bins;
+    src_k = dst_k;
+    src_v = dst_v;
   }
-  if (src_k != keys && copy_back) {
-    CMH_CUDA(cudaMemcpyAsync(keys, src_k, (size_t)n * sizeof(K), cudaMemcpyDeviceToDevice, s));
-    CMH_CUDA(cudaMemcpyAsync(vals, src_v, (size_t)n * sizeof(uint32_t),
-                             cudaMemcpyDeviceToDevice, s));
-  }
+  return passes;
 }
 
 }  // namespace
 
-size_t radix_sort_scratch(int64_t n) {
+size_t radix_state_bytes(int64_t n) {
   const int64_t ntiles = (std::max<int64_t>(n, 1) + kTile - 1) / kTile;
-  return (size_t)ntiles * kMaxBins * sizeof(uint64_t) +
-         (size_t)(2 * kMaxPasses * kMaxBins + kMaxPasses) * sizeof(uint32_t);
+  return (size_t)ntiles * kMaxBins * sizeof(uint64_t);
 }
 
-int radix_order_passes(int bits) {
+bool radix_states_apart(int64_t n, int bits, size_t *bytes) {
   int m = 0;
-  return bits > 0 ? plan_passes(bits, true, &m).passes : 0;
+  const PassDigits pd = plan_passes(bits, true, &m);
+  const int64_t ntiles = (std::max<int64_t>(n, 1) + kTile - 1) / kTile;
+  size_t all = 0;
+  for (int p = 0; p < pd.passes; p++) all += ((size_t)ntiles << pd.width[p]) * sizeof(uint64_t);
+  const bool apart = all <= (64u << 20);
+  *bytes = apart ? all : radix_state_bytes(n);
+  return apart;
 }
 
-void radix_sort_u64_u32(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt,
-                        uint32_t *vals_alt, int64_t n, const uint32_t *n_dev, int bits,
-                        DevBuf &tmp, unsigned int *giveups, cudaStream_t s, bool copy_back,
-                        SortWaits waits) {
-  radix_sort_impl<uint64_t>(keys, vals, keys_alt, vals_alt, n, n_dev, bits, tmp, giveups, s,
-                            copy_back, false, waits);
+PassDigits radix_order_plan(int bits) {
+  int m = 0;
+  return plan_passes(bits, true, &m);
 }
 
-void radix_order_u64_u32(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt,
-                         uint32_t *vals_alt, int64_t n, const uint32_t *n_dev, int bits,
-                         DevBuf &tmp, unsigned int *giveups, cudaStream_t s, SortWaits waits) {
-  radix_sort_impl<uint64_t>(keys, vals, keys_alt, vals_alt, n, n_dev, bits, tmp, giveups, s,
-                            false, true, waits);
+void radix_order_records(const void *records, uint32_t stride, uint32_t key_at, uint64_t *keys_a,
+                         uint32_t *vals_a, uint64_t *keys_b, uint32_t *vals_b, int64_t n,
+                         const uint32_t *n_dev, int bits, RadixTmp tmp, unsigned int *giveups,
+                         cudaStream_t s, SortWaits waits) {
+  const KeySource<uint64_t> src{
+      reinterpret_cast<const uint64_t *>(static_cast<const unsigned char *>(records) + key_at),
+      stride};
+  radix_passes_run<uint64_t>(src, nullptr, keys_a, vals_a, keys_b, vals_b, n, n_dev, bits, tmp,
+                             giveups, s, true, true, waits);
 }
 
 void radix_sort_u32_u32(uint32_t *keys, uint32_t *vals, uint32_t *keys_alt,
                         uint32_t *vals_alt, int64_t n, const uint32_t *n_dev, int bits,
-                        DevBuf &tmp, unsigned int *giveups, cudaStream_t s, SortWaits waits) {
-  radix_sort_impl<uint32_t>(keys, vals, keys_alt, vals_alt, n, n_dev, bits, tmp, giveups, s,
-                            true, false, waits);
+                        RadixTmp tmp, unsigned int *giveups, cudaStream_t s, SortWaits waits) {
+  if (bits <= 0 || n <= 1) return;
+  const KeySource<uint32_t> src{keys, sizeof(uint32_t)};
+  const int passes = radix_passes_run<uint32_t>(src, vals, keys, vals, keys_alt, vals_alt, n,
+                                                n_dev, bits, tmp, giveups, s, false, false, waits);
+  if (passes % 2 == 1) {
+    CMH_CUDA(cudaMemcpyAsync(keys, keys_alt, (size_t)n * sizeof(uint32_t),
+                             cudaMemcpyDeviceToDevice, s));
+    CMH_CUDA(cudaMemcpyAsync(vals, vals_alt, (size_t)n * sizeof(uint32_t),
+                             cudaMemcpyDeviceToDevice, s));
+  }
 }
 
 }  // namespace cmh
