@@ -115,28 +115,19 @@ struct PassDigits {
 // `giveups` (device) counts capped look-back waits.
 //
 // Scratch: kRadixCounts cleared words of digit counts (and what follows from
-// them), and the tiles' look-back states -- radix_state_bytes(n) bytes that the
-// sort clears before each pass, or, where every pass has its own
-// (radix_states_apart: up to 64 MB in all), the bytes it gives, cleared by the
-// caller.
+// them), and the tiles' look-back states: the bytes that radix_states_apart
+// gives.  Where it returns true (up to 64 MB in all) every pass has its own and
+// the caller clears them; else the sort clears them before each pass.
 constexpr int kRadixCounts = 2 * kRadixPasses * kRadixBins + kRadixPasses;
 struct RadixTmp {
   uint64_t *state;
   uint32_t *counts;
   bool apart;
 };
-size_t radix_state_bytes(int64_t n);
 bool radix_states_apart(int64_t n, int bits, size_t *bytes);
 PassDigits radix_order_plan(int bits);
 void radix_order_records(const void *records, uint32_t stride, uint32_t key_at, uint64_t *keys_a,
                          uint32_t *vals_a, uint64_t *keys_b, uint32_t *vals_b, int64_t n,
                          const uint32_t *n_dev, int bits, RadixTmp tmp, unsigned int *giveups,
                          cudaStream_t s, SortWaits waits = SortWaits{});
-// Stable LSD radix sort of (key, value) pairs, 32-bit keys; the result lands in
-// keys/vals (the alt buffers are scratch).
-void radix_sort_u32_u32(uint32_t *keys, uint32_t *vals, uint32_t *keys_alt,
-                        uint32_t *vals_alt, int64_t n, const uint32_t *n_dev, int bits,
-                        RadixTmp tmp, unsigned int *giveups, cudaStream_t s,
-                        SortWaits waits = SortWaits{});
-
 }  // namespace cmh

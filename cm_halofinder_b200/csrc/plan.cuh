@@ -45,7 +45,7 @@ struct Plan : public cmh_plan {
   uint32_t n_tiles = 0;  // ingest tiles of the boxes
   int n_buckets = 1;     // buckets of the emission
   // byte offsets in `scal` of the counters, the per-box numbers, the buckets and
-  // the sorts' digit counts, and its bytes
+  // the sort's digit counts, and its bytes
   size_t at_ctr = 0, at_boxd = 0, at_bucket = 0, at_counts = 0, small_bytes = 0;
   std::vector<unsigned char> small_host;
   bool cell_states_apart = false;  // each pass of the cell sort has its own tile states
@@ -113,7 +113,7 @@ struct Plan : public cmh_plan {
   DevBuf b_run_box, b_top_range, b_top_slot;
   DevBuf b_rows, b_dense_range, b_dense_big;
   DevBuf b_count, b_head, b_cand_of_root, b_cand_root, b_sums, b_warn;
-  DevBuf b_okeys, b_ovals, b_okeys_alt, b_ovals_alt;
+  DevBuf b_own_head, b_own_cand, b_marks;
   DevBuf b_props, b_head_out, b_cat_of_cand, b_member, b_member_proc, b_member_pos;
   DevBuf in_pos[2], in_vel[2];  // device copies of host-resident particles
   DevBuf b_samp;          // per input particle: 0, 1 (kept, in a halo), 2 (kept, outside)
@@ -125,7 +125,7 @@ struct Plan : public cmh_plan {
                      &b_run_box, &b_top_range, &b_top_slot,
                      &b_rows, &b_dense_range, &b_dense_big, &b_count,
                      &b_head, &b_cand_of_root, &b_cand_root, &b_sums, &b_warn,
-                     &b_okeys, &b_ovals, &b_okeys_alt, &b_ovals_alt, &b_props,
+                     &b_own_head, &b_own_cand, &b_marks, &b_props,
                      &b_head_out, &b_cat_of_cand, &b_member, &b_member_proc, &b_member_pos,
                      &in_pos[0], &in_vel[0], &in_pos[1], &in_vel[1], &b_samp};
     for (DevBuf *b : all) f(*b);

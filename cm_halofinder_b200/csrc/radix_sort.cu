@@ -1,13 +1,13 @@
-// Stable LSD radix sort of (key, value) pairs, 8-bit digits.
+// Order of records by a 64-bit key: stable LSD radix sort of (key, index) pairs.
 //
-// One read of the keys counts the digits of every pass (k_rs_upfront), which
-// gives each digit's start in the output.  Each pass is then a single
-// kernel: each 4096-key tile ranks its keys stably with warp match/ballot
+// The emission of the records has counted the digits of every pass, which
+// gives each digit's start in the output (k_rs_offsets).  Each pass is then a single
+// kernel: each 4096-key tile ranks its keys stably with warp ballot
 // counters, learns how many keys of each digit the lower tiles hold by
 // decoupled look-back over published tile states, stages its keys in shared
 // memory in digit order and writes each digit's run contiguously
-// (coalesced).  A sort of 64-bit keys whose sorted keys are not wanted
-// narrows them to 32-bit words at the first pass after which at most 32 key
+// (coalesced).  Only the order is wanted: the keys are
+// narrowed to 32-bit words at the first pass after which at most 32 key
 // bits remain (the consumed low digits are dropped), so that the later
 // passes move 8 bytes per pair instead of 12; and those 32-bit passes use
 // 9-bit digits where that saves a pass (26 bits: 9 + 9 + 8, not 8 + 8 + 8 + 2).
@@ -18,10 +18,7 @@
 namespace cmh {
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kWarps = kThreads / 32;
-constexpr int kIPT = 16;
-constexpr int kTile = kThreads * kIPT;  // 4096
+constexpr int kTile = 4096;
 constexpr int kBins = 256;      // 8-bit digits
 constexpr int kMaxBins = kRadixBins;  // 9-bit digits
 constexpr int kMaxPasses = kRadixPasses;
@@ -57,29 +54,6 @@ struct KeySource {
                                         (uint64_t)i * stride);
   }
 };
-
-// All digit histograms of the sort in one read of the keys: pass p's
-// counters at ghist[kMaxBins p].
-template <class K>
-__global__ void __launch_bounds__(kThreads) k_rs_upfront(KeySource<K> keys, int64_t n_cap,
-                                                         const uint32_t *__restrict__ n_dev,
-                                                         PassDigits pd,
-                                                         uint32_t *__restrict__ ghist) {
-  __shared__ uint32_t h[kMaxPasses * kMaxBins];
-  const int64_t n = n_dev ? (int64_t)*n_dev : n_cap;
-  for (int i = threadIdx.x; i < pd.passes * kMaxBins; i += kThreads) h[i] = 0;
-  __syncthreads();
-  for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * kThreads) {
-    const K k = keys[i];
-    for (int p = 0; p < pd.passes; p++)
-      atomicAdd(&h[p * kMaxBins + ((uint32_t)(k >> pd.shift[p]) & ((1u << pd.width[p]) - 1u))],
-                1u);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < pd.passes * kMaxBins; i += kThreads)
-    if (h[i]) atomicAdd(&ghist[i], h[i]);
-}
 
 // Exclusive prefix over the digits of each pass (one CTA of kMaxBins
 // threads per pass; unused digits count 0).
@@ -295,21 +269,17 @@ void set_scatter_smem(cudaStream_t s) {
   done[dev] = true;
 }
 
-// The passes of a sort of `bits`-bit keys.  Plain: 8-bit digits.  Narrowed:
-// m 8-bit passes over the 64-bit keys, m the fewest after which at most 32
-// bits remain, then the 32-bit passes over the R bits left, with 9-bit
-// digits on the first R - 8 ceil(R / 9) of them when that takes fewer passes
-// than 8-bit digits.  *wide receives m.
-PassDigits plan_passes(int bits, bool narrow, int *wide) {
+// The passes of a sort of `bits`-bit keys: m 8-bit passes over the 64-bit keys,
+// m the fewest (at least one) after which at most 32 bits remain, then the
+// 32-bit passes over the R bits left, with 9-bit digits on the first
+// R - 8 ceil(R / 9) of them when that takes fewer passes than 8-bit digits.
+// *wide receives m.
+PassDigits plan_passes(int bits, int *wide) {
   PassDigits pd{};
-  int m = (bits + 7) / 8, nine = 0, q = 0;
-  if (narrow) {
-    m = std::max(1, std::min((bits + 7) / 8, (bits - 32 + 7) / 8));
-    const int rest = std::max(0, bits - 8 * m);
-    const int q8 = (rest + 7) / 8, q9 = (rest + 8) / 9;
-    q = q9 < q8 ? q9 : q8;
-    nine = q9 < q8 ? rest - 8 * q9 : 0;
-  }
+  const int m = std::max(1, std::min((bits + 7) / 8, (bits - 32 + 7) / 8));
+  const int rest = std::max(0, bits - 8 * m);
+  const int q8 = (rest + 7) / 8, q9 = (rest + 8) / 9;
+  const int q = std::min(q8, q9), nine = q9 < q8 ? rest - 8 * q9 : 0;
   pd.passes = m + q;
   int shift = 0;
   for (int p = 0; p < pd.passes; p++) {
@@ -321,21 +291,32 @@ PassDigits plan_passes(int bits, bool narrow, int *wide) {
   return pd;
 }
 
-// With `narrow` (64-bit keys whose sorted order, not their sorted copy, is
-// wanted) the first m passes read 64-bit keys; pass m-1 writes key >> 8m as
-// 32-bit words and the later passes sort those on the digits that are left.
-// The first pass reads `src` (and vals, or takes the indices when vals is
-// null) and writes the b buffers, the next the a buffers, and so on in turn.
-template <class K>
-int radix_passes_run(KeySource<K> first, const uint32_t *first_vals, K *keys_a, uint32_t *vals_a,
-                     K *keys_b, uint32_t *vals_b, int64_t n, const uint32_t *n_dev, int bits,
-                     RadixTmp tmp, unsigned int *giveups, cudaStream_t s, bool narrow,
-                     bool counted, SortWaits waits) {
-  if (bits > (int)(8 * sizeof(K)) || (bits + 7) / 8 > kMaxPasses)
-    fail(CMH_ERR_INVALID_ARGUMENT, "radix sort: key bits out of range");
+}  // namespace
+
+bool radix_states_apart(int64_t n, int bits, size_t *bytes) {
   int m = 0;
-  const PassDigits pd = plan_passes(bits, narrow, &m);
-  const int passes = pd.passes;
+  const PassDigits pd = plan_passes(bits, &m);
+  const int64_t ntiles = (std::max<int64_t>(n, 1) + kTile - 1) / kTile;
+  size_t all = 0;
+  for (int p = 0; p < pd.passes; p++) all += ((size_t)ntiles << pd.width[p]) * sizeof(uint64_t);
+  const bool apart = all <= (64u << 20);
+  *bytes = apart ? all : (size_t)ntiles * kMaxBins * sizeof(uint64_t);
+  return apart;
+}
+
+PassDigits radix_order_plan(int bits) {
+  int m = 0;
+  return plan_passes(bits, &m);
+}
+
+void radix_order_records(const void *records, uint32_t stride, uint32_t key_at, uint64_t *keys_a,
+                         uint32_t *vals_a, uint64_t *keys_b, uint32_t *vals_b, int64_t n,
+                         const uint32_t *n_dev, int bits, RadixTmp tmp, unsigned int *giveups,
+                         cudaStream_t s, SortWaits waits) {
+  int m = 0;
+  const PassDigits pd = plan_passes(bits, &m);
+  if (bits > 64 || pd.passes > kMaxPasses)
+    fail(CMH_ERR_INVALID_ARGUMENT, "radix sort: key bits out of range");
   const int64_t ntiles = (n + kTile - 1) / kTile;
   if (ntiles >= 0xffffffffll) fail(CMH_ERR_CAPACITY, "radix sort: too many tiles");
   uint64_t *state = tmp.state;
@@ -343,20 +324,17 @@ int radix_passes_run(KeySource<K> first, const uint32_t *first_vals, K *keys_a, 
   uint32_t *goff = ghist + kMaxPasses * kMaxBins;
   uint32_t *tile_ctr = goff + kMaxPasses * kMaxBins;
   set_scatter_smem(s);
-  if (!counted) {
-    k_rs_upfront<K><<<grid_resident(reinterpret_cast<const void *>(k_rs_upfront<K>), kThreads, 0,
-                                    n),
-                      kThreads, 0, s>>>(first, n, n_dev, pd, ghist);
-    CMH_LAUNCHED();
-  }
-  k_rs_offsets<<<passes, kMaxBins, 0, s>>>(ghist, goff);
+  k_rs_offsets<<<pd.passes, kMaxBins, 0, s>>>(ghist, goff);
   CMH_LAUNCHED();
-  const void *src_k = first.keys;
-  const uint32_t *src_v = first_vals;
-  uint32_t src_stride = first.stride;
+  // the first pass reads the records (their indices are the values) and writes
+  // the b buffers, the next the a buffers, and so on in turn; pass m - 1 writes
+  // key >> 8 m as 32-bit words and the later passes sort those
+  const void *src_k = static_cast<const unsigned char *>(records) + key_at;
+  const uint32_t *src_v = nullptr;
+  uint32_t src_stride = stride;
   void *out_k[2] = {keys_b, keys_a};
   uint32_t *out_v[2] = {vals_b, vals_a};
-  for (int p = 0; p < passes; p++) {
+  for (int p = 0; p < pd.passes; p++) {
     const int bins = 1 << pd.width[p];
     if (!tmp.apart)
       CMH_CUDA(cudaMemsetAsync(state, 0, (size_t)ntiles * bins * sizeof(uint64_t), s));
@@ -365,17 +343,18 @@ int radix_passes_run(KeySource<K> first, const uint32_t *first_vals, K *keys_a, 
     uint32_t *dst_v = out_v[p % 2];
     // the stall hook applies to the first pass only
     const SortWaits wp{waits.spin_cap, p == 0 ? waits.stall_tile : 0xffffffffu};
-    const KeySource<K> sk{static_cast<const K *>(src_k), src_stride};
+    const KeySource<uint64_t> s8{static_cast<const uint64_t *>(src_k), src_stride};
     const KeySource<uint32_t> s4{static_cast<const uint32_t *>(src_k), src_stride};
-    if (p < m && !(narrow && p == m - 1)) {
-      k_rs_scatter<K, K, kBins><<<(unsigned)ntiles, kSThreads, sizeof(ScatterSmem<K, kBins>), s>>>(
-          sk, src_v, static_cast<K *>(dst_k), dst_v, n, n_dev, pd.shift[p], 0, go, state,
-          tile_ctr + p, giveups, wp);
-      src_stride = sizeof(K);
+    if (p < m - 1) {
+      k_rs_scatter<uint64_t, uint64_t, kBins>
+          <<<(unsigned)ntiles, kSThreads, sizeof(ScatterSmem<uint64_t, kBins>), s>>>(
+              s8, src_v, static_cast<uint64_t *>(dst_k), dst_v, n, n_dev, pd.shift[p], 0, go,
+              state, tile_ctr + p, giveups, wp);
+      src_stride = sizeof(uint64_t);
     } else if (p < m) {
-      k_rs_scatter<K, uint32_t, kBins>
-          <<<(unsigned)ntiles, kSThreads, sizeof(ScatterSmem<K, kBins>), s>>>(
-              sk, src_v, static_cast<uint32_t *>(dst_k), dst_v, n, n_dev, pd.shift[p], 8 * m, go,
+      k_rs_scatter<uint64_t, uint32_t, kBins>
+          <<<(unsigned)ntiles, kSThreads, sizeof(ScatterSmem<uint64_t, kBins>), s>>>(
+              s8, src_v, static_cast<uint32_t *>(dst_k), dst_v, n, n_dev, pd.shift[p], 8 * m, go,
               state, tile_ctr + p, giveups, wp);
       src_stride = sizeof(uint32_t);
     } else if (bins == kMaxBins) {
@@ -393,56 +372,6 @@ int radix_passes_run(KeySource<K> first, const uint32_t *first_vals, K *keys_a, 
     if (tmp.apart) state += (size_t)ntiles * bins;
     src_k = dst_k;
     src_v = dst_v;
-  }
-  return passes;
-}
-
-}  // namespace
-
-size_t radix_state_bytes(int64_t n) {
-  const int64_t ntiles = (std::max<int64_t>(n, 1) + kTile - 1) / kTile;
-  return (size_t)ntiles * kMaxBins * sizeof(uint64_t);
-}
-
-bool radix_states_apart(int64_t n, int bits, size_t *bytes) {
-  int m = 0;
-  const PassDigits pd = plan_passes(bits, true, &m);
-  const int64_t ntiles = (std::max<int64_t>(n, 1) + kTile - 1) / kTile;
-  size_t all = 0;
-  for (int p = 0; p < pd.passes; p++) all += ((size_t)ntiles << pd.width[p]) * sizeof(uint64_t);
-  const bool apart = all <= (64u << 20);
-  *bytes = apart ? all : radix_state_bytes(n);
-  return apart;
-}
-
-PassDigits radix_order_plan(int bits) {
-  int m = 0;
-  return plan_passes(bits, true, &m);
-}
-
-void radix_order_records(const void *records, uint32_t stride, uint32_t key_at, uint64_t *keys_a,
-                         uint32_t *vals_a, uint64_t *keys_b, uint32_t *vals_b, int64_t n,
-                         const uint32_t *n_dev, int bits, RadixTmp tmp, unsigned int *giveups,
-                         cudaStream_t s, SortWaits waits) {
-  const KeySource<uint64_t> src{
-      reinterpret_cast<const uint64_t *>(static_cast<const unsigned char *>(records) + key_at),
-      stride};
-  radix_passes_run<uint64_t>(src, nullptr, keys_a, vals_a, keys_b, vals_b, n, n_dev, bits, tmp,
-                             giveups, s, true, true, waits);
-}
-
-void radix_sort_u32_u32(uint32_t *keys, uint32_t *vals, uint32_t *keys_alt,
-                        uint32_t *vals_alt, int64_t n, const uint32_t *n_dev, int bits,
-                        RadixTmp tmp, unsigned int *giveups, cudaStream_t s, SortWaits waits) {
-  if (bits <= 0 || n <= 1) return;
-  const KeySource<uint32_t> src{keys, sizeof(uint32_t)};
-  const int passes = radix_passes_run<uint32_t>(src, vals, keys, vals, keys_alt, vals_alt, n,
-                                                n_dev, bits, tmp, giveups, s, false, false, waits);
-  if (passes % 2 == 1) {
-    CMH_CUDA(cudaMemcpyAsync(keys, keys_alt, (size_t)n * sizeof(uint32_t),
-                             cudaMemcpyDeviceToDevice, s));
-    CMH_CUDA(cudaMemcpyAsync(vals, vals_alt, (size_t)n * sizeof(uint32_t),
-                             cudaMemcpyDeviceToDevice, s));
   }
 }
 

@@ -1,7 +1,8 @@
 """Domain filter, periodic images and processing order where the ingest can go
 wrong, against the oracle: coordinates within a few representable values of
 the faces and of the shell's inner edge, domains away from the origin and
-around it, sizes around a tile, unaligned device arrays, empty boxes in a
+around it, sizes around a tile and around a group of the catalog's heads,
+unaligned device arrays, empty boxes in a
 batch."""
 import numpy as np
 import pytest
