@@ -71,15 +71,6 @@ struct DevBuf {
   template <class T> T *as() const { return reinterpret_cast<T *>(p); }
 };
 
-// ---- scan.cu ---------------------------------------------------------------
-// Exclusive prefix sum of n uint32 values; `total` (device, may be null)
-// receives the sum.  Scratch is taken from `tmp` (grown as needed).  With
-// `n_dev` (device) only the first min(n, *n_dev) entries are read and
-// written; n sizes the launches.
-void exclusive_scan_u32(const uint32_t *in, uint32_t *out, int64_t n,
-                        uint32_t *total, DevBuf &tmp, cudaStream_t s,
-                        const uint32_t *n_dev = nullptr);
-
 // ---- radix_sort.cu -----------------------------------------------------------
 // Bounds of the sorts' look-back waits: a tile polls a lower tile's state at
 // most spin_cap times, then gives up (the sort's giveups counter is raised;

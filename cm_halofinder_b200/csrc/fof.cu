@@ -596,59 +596,6 @@ __device__ __forceinline__ void load_rec(const PRec<double> *from, SPos<double> 
   *proc = t.y;
 }
 
-// Cell-ordered positions, processing indices, packed fine cells (the sort
-// leaves only the order) and run-start flags (a new (box, fine cell) pair) of
-// the processed particles (their scan reads no more).  A warp takes two groups of 32 consecutive elements per step (w0 and
-// w0 + stride), with both gathers in flight before either is used.  Lane l
-// compares with lane l-1's cell; lane 0 recomputes its predecessor's.
-template <class PT>
-__global__ void __launch_bounds__(kT) k_gather_flags(const uint32_t *__restrict__ order,
-                                                     const PRec<PT> *__restrict__ recs,
-                                                     const BoxDev *__restrict__ boxes, int nbox,
-                                                     SPos<PT> *__restrict__ spos,
-                                                     uint32_t *__restrict__ perm,
-                                                     uint64_t *__restrict__ cells,
-                                                     uint32_t *__restrict__ flag,
-                                                     const DevScal *__restrict__ sc) {
-  if (sc->failed) return;  // a sort of this run gave up: its order is not valid
-  __shared__ uint64_t s_base[kMaxBoxes];
-  load_bases(boxes, nbox, s_base, false);
-  const int64_t np = sc->np;
-  const int lane = threadIdx.x & 31;
-  const int64_t st = gstride();
-  for (int64_t w0 = gtid() - lane; w0 < np; w0 += 2 * st) {
-    int64_t i[2] = {w0 + lane, w0 + st + lane};
-    uint32_t pi[2] = {0u, 0u}, pp[2] = {0u, 0u};
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      if (i[h] < np) pi[h] = order[i[h]];
-      if (lane == 0 && i[h] > 0 && i[h] < np) pp[h] = order[i[h] - 1];
-    }
-    SPos<PT> sp[2], sq[2];
-    uint32_t proc[2], unused;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      if (i[h] < np) load_rec(recs + pi[h], &sp[h], &proc[h]);
-      if (lane == 0 && i[h] > 0 && i[h] < np) load_rec(recs + pp[h], &sq[h], &unused);
-    }
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      uint64_t cell = 0;
-      int box = 0;
-      if (i[h] < np) {
-        spos[i[h]] = sp[h];
-        perm[i[h]] = proc[h];
-        cell = stored_cell<PT>(boxes, s_base, nbox, sp[h], &box);
-        cells[i[h]] = cell;
-      }
-      uint64_t pcell = __shfl_up_sync(0xffffffffu, cell, 1);
-      int pbox = __shfl_up_sync(0xffffffffu, box, 1);
-      if (lane == 0 && i[h] > 0 && i[h] < np) pcell = stored_cell<PT>(boxes, s_base, nbox, sq[h], &pbox);
-      if (i[h] < np) flag[i[h]] = (i[h] == 0 || cell != pcell || box != pbox) ? 1u : 0u;
-    }
-  }
-}
-
 __device__ __forceinline__ uint64_t top_of_run(const BoxDev &bx, uint64_t pg) {
   const Geom &g = bx.g;
   const int gx = (int)(pg & kM21), gy = (int)((pg >> 21) & kM21), gz = (int)(pg >> 42);
@@ -656,51 +603,160 @@ __device__ __forceinline__ uint64_t top_of_run(const BoxDev &bx, uint64_t pg) {
          ((uint64_t)div_k(gz, g) * g.T[1] + (uint64_t)div_k(gy, g)) * g.T[0] + div_k(gx, g);
 }
 
-// Run of every processed particle, and per run its first particle, packed
-// fine cell, box and initial parent (itself); the range of runs of every
-// occupied top cell ([first, last + 1), written where the top cell changes
-// between neighbouring particles; top_range starts zeroed).
+// Tile states of the run count's look-back, as the sort's: the flag in the high
+// half, the count in the low half.
+constexpr uint64_t kTileOwn = 1ull << 32;   // the tile's own runs
+constexpr uint64_t kTileAll = 2ull << 32;   // the runs up to and with this tile
+
+// Runs before `tile`: one warp adds up the lower tiles' published states, 32 at
+// a time, back to the first inclusive one.  Every lower tile publishes its own
+// count before it waits, so every wait ends; a wait is capped all the same
+// (`polls` reads) and then raises *failed.
+__device__ __forceinline__ uint32_t runs_before(const uint64_t *state, uint32_t tile,
+                                                uint32_t polls, unsigned int *failed) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t sum = 0, left = polls;
+  int64_t top = (int64_t)tile - 1;
+  while (top >= 0) {
+    const int64_t j = top - (int64_t)lane;
+    uint64_t w = kTileAll;  // (below tile 0: nothing)
+    if (j >= 0) w = *reinterpret_cast<const volatile uint64_t *>(state + j);
+    const uint32_t all = __ballot_sync(0xffffffffu, (w >> 32) == 2);
+    const uint32_t none = __ballot_sync(0xffffffffu, (w >> 32) == 0);
+    const int first = all ? __ffs(all) - 1 : 31;  // the nearest inclusive state
+    const uint32_t need = first == 31 ? 0xffffffffu : (2u << first) - 1u;
+    if (none & need) {
+      if (left-- == 0) {
+        if (lane == 0) atomicAdd(failed, 1u);
+        return sum;
+      }
+      continue;
+    }
+    sum += __reduce_add_sync(0xffffffffu, (need >> lane) & 1u ? (uint32_t)w : 0u);
+    if (all) break;
+    top -= 32;
+    left = polls;
+  }
+  return sum;
+}
+
+// The records in cell order and their runs (of equal box and fine cell), in one
+// sweep: positions, processing indices and runs of the particles; per run its
+// first particle, packed fine cell (the sort leaves only the order: it is
+// recomputed), box and initial parent (itself); the range of runs of every
+// occupied top cell (top_range starts zeroed; where the top cell changes
+// between two particles, the new one's first run is the old one's end).  A tile
+// counts its run starts, publishes the count and learns the lower tiles' by
+// look-back.  A gather, a three-kernel scan of start flags and a kernel for the
+// runs moved 40 bytes more per particle: 0.60 ms on the 256^3 box, this 0.37;
+// 512^3 box 5.9 and 2.9 ms.
+//
+// A warp has 128 consecutive elements, 32 at a time; lane l compares with lane
+// l - 1's cell, lane 0 with the last of the 32 before (before the first 32 it
+// recomputes its predecessor's).
+constexpr int kRunPer = 4;
+constexpr int kRunTile = kT * kRunPer;
+
 template <class PT>
-__global__ void __launch_bounds__(kT) k_runs(const uint64_t *__restrict__ cells,
-                                             const uint32_t *__restrict__ flag,
-                                             const uint32_t *__restrict__ run_scan,
-                                             const SPos<PT> *__restrict__ spos,
-                                             const BoxDev *__restrict__ boxes, int nbox,
-                                             DevScal *sc,
-                                             uint32_t *__restrict__ run_of,
-                                             uint32_t *__restrict__ run_start,
-                                             uint64_t *__restrict__ run_g,
-                                             uint16_t *__restrict__ run_box,
-                                             uint32_t *__restrict__ parent,
-                                             uint32_t *__restrict__ top_range) {
+__global__ void __launch_bounds__(kT) k_gather_runs(
+    const uint32_t *__restrict__ order, const PRec<PT> *__restrict__ recs,
+    const BoxDev *__restrict__ boxes, int nbox, SPos<PT> *__restrict__ spos,
+    uint32_t *__restrict__ perm, uint32_t *__restrict__ run_of, uint32_t *__restrict__ run_start,
+    uint64_t *__restrict__ run_g, uint16_t *__restrict__ run_box, uint32_t *__restrict__ parent,
+    uint32_t *__restrict__ top_range, uint64_t *state, DevScal *sc, uint32_t polls) {
   if (sc->failed) return;  // a sort of this run gave up: its order is not valid
   __shared__ uint64_t s_base[kMaxBoxes];
+  __shared__ uint32_t s_tile, s_warp[kT / 32], s_before;
+  if (threadIdx.x == 0) s_tile = atomicAdd(&sc->next_tile, 1u);
   load_bases(boxes, nbox, s_base, false);
+  const uint32_t tile = s_tile;
   const int64_t np = sc->np;
-  const uint32_t R = sc->R;
-  auto box_of = [&](int64_t i) {
-    return nbox > 1 ? box_search(s_base, nbox, (uint64_t)spos[i].src) : 0;
-  };
-  for (int64_t i = gtid(); i < np; i += gstride()) {
-    const uint32_t f = flag[i];
-    const uint32_t rid = run_scan[i] + f - 1u;
-    const bool last = i == np - 1 || flag[i + 1] != 0u;
-    run_of[i] = rid;
-    if (!f && !last) continue;
-    const uint64_t c = cells[i];
-    const int b = box_of(i);
-    const uint64_t t = top_of_run(boxes[b], c);
-    if (f) {
-      run_start[rid] = (uint32_t)i;
-      run_g[rid] = c;
-      run_box[rid] = (uint16_t)b;
-      parent[rid] = rid;
-      if (i == 0 || top_of_run(boxes[box_of(i - 1)], cells[i - 1]) != t)
-        top_range[2 * t] = rid;
+  if ((int64_t)tile * kRunTile >= np) return;  // the whole CTA leaves together
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t i0 = (int64_t)tile * kRunTile + w * (32 * kRunPer) + lane;
+  uint32_t from[kRunPer], before = 0;
+#pragma unroll
+  for (int j = 0; j < kRunPer; j++) from[j] = i0 + 32 * j < np ? order[i0 + 32 * j] : 0u;
+  const bool has_before = lane == 0 && i0 > 0 && i0 < np;
+  if (has_before) before = order[i0 - 1];
+  SPos<PT> sp[kRunPer], sq;
+  uint32_t proc[kRunPer], unused;
+#pragma unroll
+  for (int j = 0; j < kRunPer; j++)
+    if (i0 + 32 * j < np) load_rec(recs + from[j], &sp[j], &proc[j]);
+  if (has_before) load_rec(recs + before, &sq, &unused);
+  uint64_t cell[kRunPer], pcell[kRunPer];
+  int box[kRunPer], pbox[kRunPer];
+  uint32_t start[kRunPer];  // the warp's run starts
+  uint64_t last_cell = 0;
+  int last_box = 0;
+  if (has_before) last_cell = stored_cell<PT>(boxes, s_base, nbox, sq, &last_box);
+#pragma unroll
+  for (int j = 0; j < kRunPer; j++) {
+    const int64_t i = i0 + 32 * j;
+    cell[j] = 0;
+    box[j] = 0;
+    if (i < np) {
+      spos[i] = sp[j];
+      perm[i] = proc[j];
+      cell[j] = stored_cell<PT>(boxes, s_base, nbox, sp[j], &box[j]);
     }
-    if (last && (i == np - 1 || top_of_run(boxes[box_of(i + 1)], cells[i + 1]) != t))
+    pcell[j] = __shfl_up_sync(0xffffffffu, cell[j], 1);
+    pbox[j] = __shfl_up_sync(0xffffffffu, box[j], 1);
+    if (lane == 0) {
+      pcell[j] = last_cell;
+      pbox[j] = last_box;
+    }
+    last_cell = __shfl_sync(0xffffffffu, cell[j], 31);
+    last_box = __shfl_sync(0xffffffffu, box[j], 31);
+    start[j] = __ballot_sync(0xffffffffu,
+                             i < np && (i == 0 || cell[j] != pcell[j] || box[j] != pbox[j]));
+  }
+  uint32_t mine = 0;
+#pragma unroll
+  for (int j = 0; j < kRunPer; j++) mine += __popc(start[j]);
+  if (lane == 0) s_warp[w] = mine;
+  __syncthreads();
+  uint32_t in_tile = 0, wbefore = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < kT / 32; q++) {
+    if (q < w) wbefore += s_warp[q];
+    in_tile += s_warp[q];
+  }
+  if (w == 0) {
+    unsigned long long *own = reinterpret_cast<unsigned long long *>(state + tile);
+    if (lane == 0 && tile != 0) atomicExch(own, (unsigned long long)(kTileOwn | in_tile));
+    const uint32_t b = runs_before(state, tile, polls, &sc->failed);
+    if (lane == 0) {
+      atomicExch(own, (unsigned long long)(kTileAll | (b + in_tile)));
+      s_before = b;
+    }
+  }
+  __syncthreads();
+  uint32_t done = s_before + wbefore;  // runs that start before these 32
+#pragma unroll
+  for (int j = 0; j < kRunPer; j++) {
+    const int64_t i = i0 + 32 * j;
+    const uint32_t rid = done + __popc(start[j] & ((2u << lane) - 1u)) - 1u;
+    done += __popc(start[j]);
+    if (i >= np) continue;
+    run_of[i] = rid;
+    if (!((start[j] >> lane) & 1u) && i != np - 1) continue;
+    const uint64_t t = top_of_run(boxes[box[j]], cell[j]);
+    if ((start[j] >> lane) & 1u) {
+      run_start[rid] = (uint32_t)i;
+      run_g[rid] = cell[j];
+      run_box[rid] = (uint16_t)box[j];
+      parent[rid] = rid;
+      const uint64_t pt = i > 0 ? top_of_run(boxes[pbox[j]], pcell[j]) : t;
+      if (i == 0 || pt != t) top_range[2 * t] = rid;
+      if (pt != t) top_range[2 * pt + 1] = rid;
+    }
+    if (i == np - 1) {
       top_range[2 * t + 1] = rid + 1u;
-    if (i == np - 1) run_start[R] = (uint32_t)np;
+      run_start[rid + 1u] = (uint32_t)np;
+      sc->R = rid + 1u;
+    }
   }
 }
 
@@ -2411,13 +2467,13 @@ void Plan::issue(bool want_member, cudaStream_t s, bool timed) {
   uint32_t *bucket = reinterpret_cast<uint32_t *>(small + at_bucket);
   uint32_t *cell_counts = reinterpret_cast<uint32_t *>(small + at_counts);
   const BoxDev *boxes = b_boxes.as<BoxDev>();
-  // buffers whose lifetimes do not overlap share memory: the fine-cell tables,
-  // the union-find and the befriending queue lie in the records (32 bytes or
-  // more per particle), which are dead after the gather
-  uint64_t *run_g = b_recs.as<uint64_t>();
-  uint32_t *run_of = reinterpret_cast<uint32_t *>(run_g + npc);
-  uint32_t *parent = run_of + npc, *q_cell = parent + npc, *q_top = q_cell + npc;
-  uint32_t *run_start = q_top + npc;  // npc + 1
+  // buffers whose lifetimes do not overlap share memory: the fine-cell tables
+  // lie in the sort's keys, dead after its last pass, and the befriending queue
+  // in the records, dead after the gather
+  uint64_t *run_g = b_keys.as<uint64_t>();
+  uint32_t *run_of = b_keys_alt.as<uint32_t>(), *run_start = run_of + npc;  // npc + 1
+  uint32_t *parent = b_parent.as<uint32_t>();
+  uint32_t *q_cell = b_recs.as<uint32_t>(), *q_top = q_cell + npc;
   uint2 *tile_sum = b_tiles.as<uint2>();
   auto mark = [&](int q) {
     if (timed) CMH_CUDA(cudaEventRecord(q < 0 ? ev0 : (q >= 7 ? ev1 : stage_ev[q]), s));
@@ -2443,6 +2499,7 @@ void Plan::issue(bool want_member, cudaStream_t s, bool timed) {
     f.add(b_count, npc * 4, 0u);
     f.add(b_head, npc * 4, 0xffffffffu);
     f.add(b_marks, (size_t)((npc + kHeadGroup - 1) / kHeadGroup) * (kHeadGroup / 8), 0u);
+    f.add(b_run_state, (size_t)run_tiles * 8, 0u);
     if (cell_states_apart) f.add(sort_tmp, cell_state_bytes, 0u);
     if (want_member && n > 0) {
       f.add(b_member, (size_t)n * 8, 0xffffffffu);
@@ -2483,8 +2540,7 @@ void Plan::issue(bool want_member, cudaStream_t s, bool timed) {
   // copied into their buffer)
   if (vel_wait) record_external(ev_pos_free, s);
   // ---- sort ----
-  // the sort leaves the records' indices in cell order and no sorted keys:
-  // k_gather_flags recomputes the fine cells into b_keys from the positions
+  // the sort leaves the records' indices in cell order and no sorted keys;
   // a look-back that gives up raises sc->failed, and every later kernel of
   // the run then returns at once (the order would not be valid)
   const bool odd = pd.passes % 2 == 1;
@@ -2498,19 +2554,11 @@ void Plan::issue(bool want_member, cudaStream_t s, bool timed) {
                       &sc->failed, s, SortWaits{spin_cap, stall_sort ? 1u : 0xffffffffu});
   mark(1);
   // ---- runs, top-cell ranges, dense top cells ----
-  uint32_t *flag = b_keys_alt.as<uint32_t>();  // reuse: [flag | run_scan]
-  uint32_t *run_scan = flag + npc;
-  k_gather_flags<PT><<<rg(k_gather_flags<PT>, npc), kT, 0, s>>>(
-      order, b_recs.as<PRec<PT>>(), boxes, nbox, b_spos.as<SPos<PT>>(), perm,
-      b_keys.as<uint64_t>(), flag, sc);
-  CMH_LAUNCHED();
-  exclusive_scan_u32(flag, run_scan, npc, &sc->R, scan_tmp, s, &sc->np);
   CMH_CUDA(cudaStreamWaitEvent(s, ev_cleared, 0));  // the later stages' tables
-  k_runs<PT><<<rg(k_runs<PT>, npc), kT, 0, s>>>(b_keys.as<uint64_t>(), flag, run_scan,
-                                               b_spos.as<SPos<PT>>(), boxes, nbox, sc, run_of,
-                                               run_start, run_g,
-                                               b_run_box.as<uint16_t>(), parent,
-                                               b_top_range.as<uint32_t>());
+  k_gather_runs<PT><<<(unsigned)run_tiles, kT, 0, s>>>(
+      order, b_recs.as<PRec<PT>>(), boxes, nbox, b_spos.as<SPos<PT>>(), perm, run_of, run_start,
+      run_g, b_run_box.as<uint16_t>(), parent, b_top_range.as<uint32_t>(),
+      b_run_state.as<uint64_t>(), sc, spin_cap);
   CMH_LAUNCHED();
   if (varlink) {
     if (fp32)
@@ -2764,7 +2812,10 @@ void Plan::prepare(const std::vector<BoxSpec> &specs, bool want_member) {
   scal.ensure(small_bytes);
   b_boxes.ensure(sizeof(BoxDev) * nbox);
   b_keys.ensure(npc * 8);
-  b_keys_alt.ensure(npc * 8);
+  b_keys_alt.ensure(npc * 8 + 8);  // (also run_of and run_start)
+  b_parent.ensure(npc * 4);
+  run_tiles = (npc + kRunTile - 1) / kRunTile;
+  b_run_state.ensure((size_t)run_tiles * 8);
   b_vals.ensure(npc * 4);
   b_vals_alt.ensure(npc * 4);
   const bool dbl = pos_dtype == CMH_FLOAT64;
@@ -2813,15 +2864,8 @@ void Plan::prepare(const std::vector<BoxSpec> &specs, bool want_member) {
     for (const void *f : dense)
       CMH_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm));
   }
-  // pre-grow the scratch of the scans and sorts so that issue() allocates
-  // nothing (it may be captured in a graph)
+  // the sort's scratch (issue() allocates nothing: it may be captured in a graph)
   {
-    int64_t need = 0;
-    for (int64_t m = std::max(npc, nn) * 1; m > 4096;) {
-      m = (m + 4095) / 4096;
-      need += 2 * m;
-    }
-    scan_tmp.ensure((size_t)(need + 16) * sizeof(uint32_t));
     cell_states_apart = radix_states_apart(npc, key_bits, &cell_state_bytes);
     sort_tmp.ensure(cell_state_bytes);
   }

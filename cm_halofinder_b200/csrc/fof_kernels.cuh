@@ -101,7 +101,8 @@ struct DevScal {
   uint32_t overflow;               // bit 0: processed particles above capacity
   uint32_t nbig, next_big;          // dense top cells handled by a whole CTA
   uint32_t next_simple;             // fine cells taken by the sparse path
-  uint32_t failed;                  // a sort's capped look-back wait gave up: every
+  uint32_t next_tile;               // tiles taken by the gather
+  uint32_t failed;                  // a capped look-back wait gave up: every
                                     // later kernel of the run returns at once
 };
 

@@ -50,6 +50,7 @@ struct Plan : public cmh_plan {
   std::vector<unsigned char> small_host;
   bool cell_states_apart = false;  // each pass of the cell sort has its own tile states
   size_t cell_state_bytes = 0;
+  int64_t run_tiles = 0;           // tiles of the gather
   uint64_t n_top = 0, k3all = 1;
   int key_bits = 0, hs = 7, props = 0;
   bool varlink = false;             // some box has a variable linking length
@@ -108,11 +109,11 @@ struct Plan : public cmh_plan {
   const uint64_t *samp_ids = nullptr;
 
   // workspace
-  DevBuf scal, scan_tmp, sort_tmp, b_tiles, ltab_dev, b_boxes;
+  DevBuf scal, sort_tmp, b_tiles, ltab_dev, b_boxes;
   DevBuf b_keys, b_keys_alt, b_vals, b_vals_alt, b_recs, b_spos, b_svl;
   DevBuf b_run_box, b_top_range, b_top_slot;
   DevBuf b_rows, b_dense_range, b_dense_big;
-  DevBuf b_count, b_head, b_cand_of_root, b_cand_root, b_sums, b_warn;
+  DevBuf b_parent, b_run_state, b_count, b_head, b_cand_of_root, b_cand_root, b_sums, b_warn;
   DevBuf b_own_head, b_own_cand, b_marks;
   DevBuf b_props, b_head_out, b_cat_of_cand, b_member, b_member_proc, b_member_pos;
   DevBuf in_pos[2], in_vel[2];  // device copies of host-resident particles
@@ -120,10 +121,10 @@ struct Plan : public cmh_plan {
 
   // every workspace buffer, for release and for the graph signature
   template <class F> void each_buf(F f) {
-    DevBuf *all[] = {&scal, &scan_tmp, &sort_tmp, &b_tiles, &ltab_dev, &b_boxes,
+    DevBuf *all[] = {&scal, &sort_tmp, &b_tiles, &ltab_dev, &b_boxes,
                      &b_keys, &b_keys_alt, &b_vals, &b_vals_alt, &b_recs, &b_spos, &b_svl,
                      &b_run_box, &b_top_range, &b_top_slot,
-                     &b_rows, &b_dense_range, &b_dense_big, &b_count,
+                     &b_rows, &b_dense_range, &b_dense_big, &b_parent, &b_run_state, &b_count,
                      &b_head, &b_cand_of_root, &b_cand_root, &b_sums, &b_warn,
                      &b_own_head, &b_own_cand, &b_marks, &b_props,
                      &b_head_out, &b_cat_of_cand, &b_member, &b_member_proc, &b_member_pos,

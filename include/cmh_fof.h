@@ -271,8 +271,9 @@ cmh_status cmh_plan_run_batch_status(cmh_plan *plan, const cmh_fof_params *param
 /* Bounds of the device loops that retry or wait.  A union of two
  * union-find components (find both roots, hook one under the other) is
  * attempted at most union_attempts times -- it is attempted again only after
- * losing a race to another thread -- and a tile of a radix sort polls a lower
- * tile's state at most lookback_polls times after its first read.  A loop
+ * losing a race to another thread -- and a tile of the cell sort, or of the run
+ * count after it, polls a lower tile's state at most lookback_polls times after
+ * its first read.  A loop
  * that runs out makes the run return CMH_ERR_DEVICE_TIMEOUT (the plan stays
  * usable; the next run starts afresh).  Negative: the default, 2^22 each.
  * union_attempts = 0 makes every union give up at once (a test setting).
