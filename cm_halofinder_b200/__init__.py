@@ -120,17 +120,49 @@ def _dtype_code(a):
     raise TypeError("positions and velocities must be float32 or float64")
 
 
+class _Owned:
+    """A host catalog of the library's, freed with the last array on it."""
+
+    def __init__(self, cat):
+        self.free = _abi.lib().cmh_catalog_free
+        self.cat = _abi.Catalog()
+        C.memmove(C.byref(self.cat), C.byref(cat), C.sizeof(cat))
+        cat.impl = None          # the struct given is no longer its owner
+        cat.props = cat.head = cat.member = cat.member_proc = cat.member_pos = None
+
+    def __del__(self):
+        self.free(self.cat)
+
+
+# Memberships of at least this many bytes are handed over as the library's own
+# array instead of a copy.
+_HAND_OVER = 1 << 20
+
+
 def _host_catalog(cat):
+    """The host catalog as numpy arrays: copies, except a large membership,
+    which stays where the library put it (and keeps the catalog alive)."""
     nh, hs = int(cat.nhalos), int(cat.halosize)
     props = np.ctypeslib.as_array(cat.props, shape=(max(nh, 1), hs))[:nh].copy() \
         if nh else np.zeros((0, hs), np.float32)
     head = np.ctypeslib.as_array(cat.head, shape=(max(nh, 1),))[:nh].copy() \
         if nh else np.zeros(0, np.uint32)
+    stats = cat.stats.as_dict()
     member = None
     if bool(cat.member):
         n = int(cat.stats.n_in)
-        member = np.ctypeslib.as_array(cat.member, shape=(max(n, 1),))[:n].copy()
-    return Catalog(props=props, head=head, member=member, stats=cat.stats.as_dict())
+        if 8 * n >= _HAND_OVER:
+            room = (C.c_int64 * n).from_address(C.addressof(cat.member.contents))
+            room.owner = _Owned(cat)
+            member = np.frombuffer(room, np.int64)
+        else:
+            member = np.ctypeslib.as_array(cat.member, shape=(max(n, 1),))[:n].copy()
+    return Catalog(props=props, head=head, member=member, stats=stats)
+
+
+def _want(members):
+    """want_member of the C calls: the arrays here are the halo indices only."""
+    return _abi.CMH_MEMBER_INDEX if members else 0
 
 
 def fof(pos, vel, config: FofConfig, ids=None, members=False, stream=None):
@@ -149,7 +181,7 @@ def fof(pos, vel, config: FofConfig, ids=None, members=False, stream=None):
                            location=CMH_HOST)
     p = config.to_c()
     cat = _abi.Catalog()
-    _abi.check(L.cmh_fof_run(C.byref(p), C.byref(parts), C.byref(cat), int(members),
+    _abi.check(L.cmh_fof_run(C.byref(p), C.byref(parts), C.byref(cat), _want(members),
                              C.c_void_p(stream or 0)))
     try:
         return _host_catalog(cat)
@@ -210,8 +242,9 @@ class Plan:
             sp = stream.cuda_stream
         else:
             sp = int(stream)
-        _abi.check(self._L.cmh_plan_run(self._h, C.byref(parts), C.byref(cat), int(members),
-                                        loc, C.c_void_p(sp)))
+        want = _want(members) if loc == CMH_HOST else int(members)
+        _abi.check(self._L.cmh_plan_run(self._h, C.byref(parts), C.byref(cat), want, loc,
+                                        C.c_void_p(sp)))
         if loc == CMH_DEVICE:
             return cat  # raw struct: device pointers into plan-owned memory
         try:
@@ -460,7 +493,7 @@ def fof_sampled(pos, vel, config: FofConfig, samp_in, samp_out, seed, ids=None,
     cat = _abi.Catalog()
     out = _abi.Sample()
     _abi.check(L.cmh_fof_run_sampled(C.byref(p), C.byref(parts), C.byref(samp), C.byref(cat),
-                                     int(members), C.byref(out), C.c_void_p(stream or 0)))
+                                     _want(members), C.byref(out), C.c_void_p(stream or 0)))
     try:
         inh = np.ctypeslib.as_array(out.inhalo, shape=(max(out.n_inhalo, 1),))[:out.n_inhalo].copy()
         outh = np.ctypeslib.as_array(out.outhalo, shape=(max(out.n_outhalo, 1),))[

@@ -18,6 +18,7 @@ CMH_FLOAT32, CMH_FLOAT64 = 0, 1
 CMH_PLAIN_FP64, CMH_FP32_RECHECK = 0, 1
 CMH_HOST, CMH_DEVICE = 0, 1
 CMH_PROP_INERTIA, CMH_PROP_DISPERSION = 1, 2
+CMH_MEMBER_INDEX = 0x6D656D31
 CMH_OUT_UNFORMATTED, CMH_OUT_PARTICLES, CMH_OUT_PARTICLE_ID = 1, 2, 4
 CMH_TAGS_VARLINK, CMH_TAGS_INFOFILE = 1, 2
 CMH_FMT_ASCII, CMH_FMT_GADGET1, CMH_FMT_PICOLA_LIGHTCONE = 0, 1, 2

@@ -89,8 +89,32 @@ void DevBuf::ensure(size_t bytes) {
   cap = want;
 }
 
+void DevBuf::place(const DevBuf &in, size_t at, size_t bytes) {
+  p = in.as<unsigned char>() + at;
+  cap = bytes;
+  view = true;
+}
+
 void DevBuf::release() {
-  if (p) cudaFree(p);
+  if (p && !view) cudaFree(p);
+  p = nullptr;
+  cap = 0;
+}
+
+void HostBuf::ensure(size_t bytes) {
+  if (bytes <= cap) return;
+  release();
+  const size_t want = bytes + bytes / 4 + 4096;
+  if (cudaMallocHost(&p, want) != cudaSuccess) {  // (the caller then copies unpinned)
+    (void)cudaGetLastError();
+    p = nullptr;
+    return;
+  }
+  cap = want;
+}
+
+void HostBuf::release() {
+  if (p) cudaFreeHost(p);
   p = nullptr;
   cap = 0;
 }
@@ -128,6 +152,8 @@ Plan::~Plan() {
     if (ev_vel[b]) cudaEventDestroy(ev_vel[b]);
   }
   each_buf([](DevBuf &b) { b.release(); });
+  arena.release();
+  pinned.release();
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
   for (cudaEvent_t e : stage_ev)
@@ -145,6 +171,7 @@ void Plan::release_workspace() {
   staged.clear();
   uploaded_sig.clear();
   each_buf([](DevBuf &b) { b.release(); });
+  arena.release();
   np_cap = nd_cap = nc_cap = 0;
 }
 
@@ -212,9 +239,33 @@ void check_parts(const cmh_particles *parts) {
     cmh::fail(CMH_ERR_CAPACITY, "more than 2^32 particles in one domain");
 }
 
-// Copies box b's part of the plan's last catalog to host arrays owned by
-// `cat` (a run's catalog lists the boxes one after another).
-void catalog_to_host(Plan &pl, cmh_catalog *cat, bool want_member, int b, cudaStream_t s) {
+// How much of the membership a caller wants: 0 none, 1 the whole, 2 the halo
+// indices only.
+int member_level(int32_t want_member) {
+  return want_member == 0 ? 0 : want_member == CMH_MEMBER_INDEX ? 2 : 1;
+}
+
+// The plan's last catalog (all boxes, one after another) in host memory: its
+// records and heads, copied together.
+struct HostCatalog {
+  std::vector<unsigned char> own;
+  const float *props = nullptr;
+  const uint32_t *head = nullptr;
+  HostCatalog(Plan &pl, cudaStream_t s) {
+    const size_t nh = (size_t)pl.out_nhalos, pb = sizeof(float) * nh * pl.hs, hb = 4 * nh;
+    if (nh == 0) return;
+    unsigned char *to = pl.host_room(pb + hb, own);
+    CMH_CUDA(cudaMemcpyAsync(to, pl.b_props.p, pb, cudaMemcpyDeviceToHost, s));
+    CMH_CUDA(cudaMemcpyAsync(to + pb, pl.b_head_out.p, hb, cudaMemcpyDeviceToHost, s));
+    CMH_CUDA(cudaStreamSynchronize(s));
+    props = reinterpret_cast<const float *>(to);
+    head = reinterpret_cast<const uint32_t *>(to + pb);
+  }
+};
+
+// Box b's part of the plan's last catalog in host arrays owned by `cat`.
+void catalog_to_host(Plan &pl, const HostCatalog &all, cmh_catalog *cat, int members, int b,
+                     cudaStream_t s) {
   const int nbox = (int)pl.boxes_host.size();
   const int64_t nh = pl.boxd_host[5 * nbox + b];
   const int64_t h0 = pl.boxd_host[6 * nbox + b];
@@ -230,33 +281,33 @@ void catalog_to_host(Plan &pl, cmh_catalog *cat, bool want_member, int b, cudaSt
   cat->member_proc = nullptr;
   cat->member_pos = nullptr;
   cat->impl = new cmh::CatalogStore{true};
-  if (want_member) {
-    const size_t nn = (size_t)std::max<int64_t>(n_in, 1);
-    cat->member = (int64_t *)malloc(sizeof(int64_t) * nn);
+  const size_t nn = (size_t)std::max<int64_t>(n_in, 1);
+  if (members) cat->member = (int64_t *)malloc(sizeof(int64_t) * nn);
+  if (members == 1) {
     cat->member_proc = (uint32_t *)malloc(sizeof(uint32_t) * nn);
     cat->member_pos = (float *)malloc(sizeof(float) * 3 * nn);
   }
-  if (!cat->props || !cat->head ||
-      (want_member && (!cat->member || !cat->member_proc || !cat->member_pos)))
+  if (!cat->props || !cat->head || (members && !cat->member) ||
+      (members == 1 && (!cat->member_proc || !cat->member_pos)))
     cmh::fail(CMH_ERR_OUT_OF_MEMORY, "host catalog allocation failed");
   if (nh > 0) {
-    CMH_CUDA(cudaMemcpyAsync(cat->props, pl.b_props.as<float>() + h0 * hs,
-                             sizeof(float) * nh * hs, cudaMemcpyDeviceToHost, s));
-    CMH_CUDA(cudaMemcpyAsync(cat->head, pl.b_head_out.as<uint32_t>() + h0,
-                             sizeof(uint32_t) * nh, cudaMemcpyDeviceToHost, s));
+    memcpy(cat->props, all.props + h0 * hs, sizeof(float) * nh * hs);
+    memcpy(cat->head, all.head + h0, sizeof(uint32_t) * nh);
   }
-  if (want_member && n_in > 0) {
+  if (members && n_in > 0) {
     CMH_CUDA(cudaMemcpyAsync(cat->member, pl.b_member.as<int64_t>() + i0,
                              sizeof(int64_t) * n_in, cudaMemcpyDeviceToHost, s));
-    CMH_CUDA(cudaMemcpyAsync(cat->member_proc, pl.b_member_proc.as<uint32_t>() + i0,
-                             sizeof(uint32_t) * n_in, cudaMemcpyDeviceToHost, s));
-    CMH_CUDA(cudaMemcpyAsync(cat->member_pos, pl.b_member_pos.as<float>() + 3 * i0,
-                             sizeof(float) * 3 * n_in, cudaMemcpyDeviceToHost, s));
+    if (members == 1) {
+      CMH_CUDA(cudaMemcpyAsync(cat->member_proc, pl.b_member_proc.as<uint32_t>() + i0,
+                               sizeof(uint32_t) * n_in, cudaMemcpyDeviceToHost, s));
+      CMH_CUDA(cudaMemcpyAsync(cat->member_pos, pl.b_member_pos.as<float>() + 3 * i0,
+                               sizeof(float) * 3 * n_in, cudaMemcpyDeviceToHost, s));
+    }
+    CMH_CUDA(cudaStreamSynchronize(s));
+    if (h0 > 0)
+      for (int64_t i = 0; i < n_in; i++)
+        if (cat->member[i] >= 0) cat->member[i] -= h0;
   }
-  CMH_CUDA(cudaStreamSynchronize(s));
-  if (want_member && h0 > 0)
-    for (int64_t i = 0; i < n_in; i++)
-      if (cat->member[i] >= 0) cat->member[i] -= h0;
   cat->stats = pl.stats;
   if (nbox > 1) {
     cat->stats.n_in = n_in;
@@ -267,15 +318,15 @@ void catalog_to_host(Plan &pl, cmh_catalog *cat, bool want_member, int b, cudaSt
   }
 }
 
-void catalog_on_device(Plan &pl, cmh_catalog *cat, bool want_member) {
+void catalog_on_device(Plan &pl, cmh_catalog *cat, int members) {
   cat->nhalos = pl.out_nhalos;
   cat->halosize = pl.hs;
   cat->location = CMH_DEVICE;
   cat->props = pl.b_props.as<float>();
   cat->head = pl.b_head_out.as<uint32_t>();
-  cat->member = want_member ? pl.b_member.as<int64_t>() : nullptr;
-  cat->member_proc = want_member ? pl.b_member_proc.as<uint32_t>() : nullptr;
-  cat->member_pos = want_member ? pl.b_member_pos.as<float>() : nullptr;
+  cat->member = members ? pl.b_member.as<int64_t>() : nullptr;
+  cat->member_proc = members == 1 ? pl.b_member_proc.as<uint32_t>() : nullptr;
+  cat->member_pos = members == 1 ? pl.b_member_pos.as<float>() : nullptr;
   cat->impl = nullptr;
   cat->stats = pl.stats;
 }
@@ -335,9 +386,10 @@ cmh_status cmh_plan_run(cmh_plan *plan, const cmh_particles *parts, cmh_catalog 
     Plan &p;
     ~Reset() { p.vel_wait = false; }
   } reset{pl};
-  pl.run(dp, want_member != 0, s);
-  if (out_location == CMH_DEVICE) catalog_on_device(pl, cat, want_member != 0);
-  else catalog_to_host(pl, cat, want_member != 0, 0, s);
+  const int members = member_level(want_member);
+  pl.run(dp, members, s);
+  if (out_location == CMH_DEVICE) catalog_on_device(pl, cat, members);
+  else catalog_to_host(pl, HostCatalog(pl, s), cat, members, 0, s);
   CMH_API_END
 }
 
@@ -447,28 +499,33 @@ void fof_once(const cmh_fof_params *params, const cmh_particles *parts,
   }
   const int dev = current_device();
   std::unique_ptr<Plan> pl(new Plan(*params, parts->pos_dtype, dev));
+  pl->use_graph = false;  // one run: nothing to replay
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   cmh_particles dp = *parts;
-  // device copies of host inputs, freed on every way out
+  // device copies of host inputs in one allocation, freed on every way out
   struct Copies {
-    cmh::DevBuf pos, vel, ids;
-    ~Copies() {
-      pos.release();
-      vel.release();
-      ids.release();
-    }
+    cmh::DevBuf all;
+    ~Copies() { all.release(); }
   } cp;
-  cmh::DevBuf &dpos = cp.pos, &dvel = cp.vel, &dids = cp.ids;
-  if (parts->location == CMH_HOST && parts->n > 0) {
+  const bool host = parts->location == CMH_HOST && parts->n > 0;
+  const uint64_t *ids = sampling && parts->n > 0 ? parts->id : nullptr;
+  if (host) {
+    auto up = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
     const size_t pb = (size_t)parts->n * 3 * (parts->pos_dtype == CMH_FLOAT64 ? 8 : 4);
     const size_t vb = (size_t)parts->n * 3 * (parts->vel_dtype == CMH_FLOAT64 ? 8 : 4);
-    dpos.ensure(pb);
-    dvel.ensure(vb);
-    CMH_CUDA(cudaMemcpyAsync(dpos.p, parts->pos, pb, cudaMemcpyHostToDevice, s));
-    CMH_CUDA(cudaMemcpyAsync(dvel.p, parts->vel, vb, cudaMemcpyHostToDevice, s));
-    dp.pos = dpos.p;
-    dp.vel = dvel.p;
+    const size_t ib = ids ? (size_t)parts->n * 8 : 0;
+    cp.all.ensure(up(pb) + up(vb) + ib);
+    unsigned char *to = cp.all.as<unsigned char>();
+    CMH_CUDA(cudaMemcpyAsync(to, parts->pos, pb, cudaMemcpyHostToDevice, s));
+    CMH_CUDA(cudaMemcpyAsync(to + up(pb), parts->vel, vb, cudaMemcpyHostToDevice, s));
+    dp.pos = to;
+    dp.vel = to + up(pb);
     dp.location = CMH_DEVICE;
+    if (ids) {
+      to += up(pb) + up(vb);
+      CMH_CUDA(cudaMemcpyAsync(to, ids, ib, cudaMemcpyHostToDevice, s));
+      ids = reinterpret_cast<const uint64_t *>(to);
+    }
   }
   if (sampling) {
     pl->sampling = true;
@@ -476,20 +533,11 @@ void fof_once(const cmh_fof_params *params, const cmh_particles *parts,
     pl->samp_out = sampling->samp_out;
     pl->samp_seed = (uint64_t)(int64_t)sampling->seed;
     for (int a = 0; a < 3; a++) pl->samp_closed |= (sampling->closed_hi[a] ? 1 : 0) << a;
-    pl->use_graph = false;  // one run: nothing to replay
-    if (parts->id && parts->n > 0) {
-      if (parts->location == CMH_HOST) {
-        dids.ensure((size_t)parts->n * 8);
-        CMH_CUDA(cudaMemcpyAsync(dids.p, parts->id, (size_t)parts->n * 8,
-                                 cudaMemcpyHostToDevice, s));
-        pl->samp_ids = dids.as<uint64_t>();
-      } else {
-        pl->samp_ids = parts->id;
-      }
-    }
+    pl->samp_ids = ids;
   }
-  pl->run(dp, want_member != 0, s);
-  catalog_to_host(*pl, cat, want_member != 0, 0, s);
+  const int members = member_level(want_member);
+  pl->run(dp, members, s);
+  catalog_to_host(*pl, HostCatalog(*pl, s), cat, members, 0, s);
   if (sampling) {
     const int64_t n = parts->n;
     std::vector<uint8_t> flag((size_t)std::max<int64_t>(n, 1), 0);
@@ -602,8 +650,9 @@ void run_batch_on(Plan &pl, const cmh_fof_params *params, const cmh_particles *p
     Plan &p;
     ~Reset() { p.vel_wait = false; }
   } reset{pl};
-  pl.run_batch(make_specs(pl, params, parts, nbox), false, s);
-  for (int b = 0; b < nbox; b++) catalog_to_host(pl, &cats[b], false, b, s);
+  pl.run_batch(make_specs(pl, params, parts, nbox), 0, s);
+  const HostCatalog all(pl, s);
+  for (int b = 0; b < nbox; b++) catalog_to_host(pl, all, &cats[b], 0, b, s);
 }
 }  // namespace
 

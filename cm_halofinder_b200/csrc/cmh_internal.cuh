@@ -62,11 +62,13 @@ inline unsigned grid_resident(const void *kernel, int threads, size_t smem, int6
   return (unsigned)(want < cap ? want : cap);
 }
 
-// Growable device buffer.
+// Growable device buffer, or a piece of another one (a view).
 struct DevBuf {
   void *p = nullptr;
   size_t cap = 0;
+  bool view = false;
   void ensure(size_t bytes);
+  void place(const DevBuf &in, size_t at, size_t bytes);
   void release();
   template <class T> T *as() const { return reinterpret_cast<T *>(p); }
 };

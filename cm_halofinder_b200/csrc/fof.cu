@@ -2216,6 +2216,7 @@ __global__ void __launch_bounds__(kT) k_member_copy(
     if (h == kNone) continue;
     const SPos<PT> p = spos[i];
     if (member[p.src] == (unsigned long long)h) {
+      if (!member_proc) continue;  // only the halo indices are wanted
       member_proc[p.src] = perm[i] - boxd[4 * nbox + run_box[run]];
       member_pos[3 * (uint64_t)p.src] = (float)p.x;
       member_pos[3 * (uint64_t)p.src + 1] = (float)p.y;
@@ -2456,7 +2457,7 @@ double image_estimate(const Geom &g, int64_t n) {
 }  // namespace
 
 template <class PT>
-void Plan::issue(bool want_member, cudaStream_t s, bool timed) {
+void Plan::issue(int want_member, cudaStream_t s, bool timed) {
   const int nbox = (int)boxes_host.size();
   const int64_t n = n_total, npc = np_cap, ncc = nc_cap;
   DevScal *sc = scal.as<DevScal>();
@@ -2503,8 +2504,10 @@ void Plan::issue(bool want_member, cudaStream_t s, bool timed) {
     if (cell_states_apart) f.add(sort_tmp, cell_state_bytes, 0u);
     if (want_member && n > 0) {
       f.add(b_member, (size_t)n * 8, 0xffffffffu);
-      f.add(b_member_proc, (size_t)n * 4, 0xffffffffu);
-      f.add(b_member_pos, (size_t)n * 12, 0u);
+      if (want_member == 1) {
+        f.add(b_member_proc, (size_t)n * 4, 0xffffffffu);
+        f.add(b_member_pos, (size_t)n * 12, 0u);
+      }
     }
     uint64_t most = 0;
     for (int q = 0; q < f.count; q++) most = std::max(most, f.n[q]);
@@ -2706,7 +2709,7 @@ void Plan::issue(bool want_member, cudaStream_t s, bool timed) {
   mark(7);
 }
 
-void Plan::prepare(const std::vector<BoxSpec> &specs, bool want_member) {
+void Plan::prepare(const std::vector<BoxSpec> &specs, int want_member) {
   if (!bf_stream) {
     CMH_CUDA(cudaStreamCreateWithFlags(&bf_stream, cudaStreamNonBlocking));
     CMH_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
@@ -2801,6 +2804,10 @@ void Plan::prepare(const std::vector<BoxSpec> &specs, bool want_member) {
   nc_cap = std::max<int64_t>(1, np_cap / div + 1);
 
   const int64_t nn = std::max<int64_t>(n_total, 1), npc = np_cap, ncc = nc_cap;
+  // the run's buffers, laid out in one allocation (one cudaMalloc and cudaFree
+  // where each buffer had its own: a one-shot run spent most of its time there)
+  std::vector<std::pair<DevBuf *, size_t>> pieces;
+  auto need = [&](DevBuf &b, size_t bytes) { pieces.emplace_back(&b, bytes); };
   // the small arrays that every run starts cleared, in one piece; the first
   // three are read back together
   auto up = [](size_t b) { return (b + 127) & ~(size_t)127; };
@@ -2809,44 +2816,44 @@ void Plan::prepare(const std::vector<BoxSpec> &specs, bool want_member) {
   at_bucket = at_boxd + up(sizeof(uint32_t) * 7 * nbox);
   at_counts = at_bucket + up((size_t)n_buckets * 4);
   small_bytes = at_counts + kRadixCounts * 4;
-  scal.ensure(small_bytes);
-  b_boxes.ensure(sizeof(BoxDev) * nbox);
-  b_keys.ensure(npc * 8);
-  b_keys_alt.ensure(npc * 8 + 8);  // (also run_of and run_start)
-  b_parent.ensure(npc * 4);
+  need(scal, small_bytes);
+  need(b_boxes, sizeof(BoxDev) * nbox);
+  need(b_keys, npc * 8);
+  need(b_keys_alt, npc * 8 + 8);  // (also run_of and run_start)
+  need(b_parent, npc * 4);
   run_tiles = (npc + kRunTile - 1) / kRunTile;
-  b_run_state.ensure((size_t)run_tiles * 8);
-  b_vals.ensure(npc * 4);
-  b_vals_alt.ensure(npc * 4);
+  need(b_run_state, (size_t)run_tiles * 8);
+  need(b_vals, npc * 4);
+  need(b_vals_alt, npc * 4);
   const bool dbl = pos_dtype == CMH_FLOAT64;
-  b_recs.ensure(npc * (dbl ? sizeof(PRec<double>) : sizeof(PRec<float>)));
-  b_spos.ensure(npc * (dbl ? sizeof(SPos<double>) : sizeof(SPos<float>)));
-  b_tiles.ensure((size_t)n_tiles * sizeof(uint2));
-  if (varlink) b_svl.ensure(npc * sizeof(VLRec64));
-  b_run_box.ensure(npc * 2);
-  b_top_range.ensure(n_top * 8);
-  b_top_slot.ensure(n_top * 4);
-  b_rows.ensure((size_t)nd_cap * rows_per_top(k3all) * sizeof(uint4));
-  b_dense_range.ensure((size_t)nd_cap * sizeof(uint2));
-  b_dense_big.ensure((size_t)nd_cap * sizeof(uint32_t));
-  b_count.ensure(npc * 4);
-  b_head.ensure(npc * 4);
-  b_cand_of_root.ensure(npc * 4);
-  if (sampling) b_samp.ensure((size_t)nn);
-  b_cand_root.ensure(ncc * 4);
-  b_sums.ensure(ncc * 18 * 8);
-  b_warn.ensure(ncc * 4);
-  b_own_head.ensure(ncc * 4);
-  b_own_cand.ensure(ncc * 4);
+  need(b_recs, npc * (dbl ? sizeof(PRec<double>) : sizeof(PRec<float>)));
+  need(b_spos, npc * (dbl ? sizeof(SPos<double>) : sizeof(SPos<float>)));
+  need(b_tiles, (size_t)n_tiles * sizeof(uint2));
+  if (varlink) need(b_svl, npc * sizeof(VLRec64));
+  need(b_run_box, npc * 2);
+  need(b_top_range, n_top * 8);
+  need(b_top_slot, n_top * 4);
+  need(b_rows, (size_t)nd_cap * rows_per_top(k3all) * sizeof(uint4));
+  need(b_dense_range, (size_t)nd_cap * sizeof(uint2));
+  need(b_dense_big, (size_t)nd_cap * sizeof(uint32_t));
+  need(b_count, npc * 4);
+  need(b_head, npc * 4);
+  need(b_cand_of_root, npc * 4);
+  if (sampling) need(b_samp, (size_t)nn);
+  need(b_cand_root, ncc * 4);
+  need(b_sums, ncc * 18 * 8);
+  need(b_warn, ncc * 4);
+  need(b_own_head, ncc * 4);
+  need(b_own_cand, ncc * 4);
   // marks of the heads (a bit each) and the counts of their groups
-  b_marks.ensure((size_t)((npc + kHeadGroup - 1) / kHeadGroup) * (kHeadGroup / 8 + 4));
-  b_props.ensure(ncc * hs * 4);
-  b_head_out.ensure(ncc * 4);
-  b_cat_of_cand.ensure(ncc * 4);
-  if (want_member) {
-    b_member.ensure(nn * 8);
-    b_member_proc.ensure(nn * 4);
-    b_member_pos.ensure(nn * 12);
+  need(b_marks, (size_t)((npc + kHeadGroup - 1) / kHeadGroup) * (kHeadGroup / 8 + 4));
+  need(b_props, ncc * hs * 4);
+  need(b_head_out, ncc * 4);
+  need(b_cat_of_cand, ncc * 4);
+  if (want_member) need(b_member, nn * 8);
+  if (want_member == 1) {
+    need(b_member_proc, nn * 4);
+    need(b_member_pos, nn * 12);
   }
   // shared memory of the dense-top kernel: one parent per fine cell of a top
   // cell (set here, outside any graph capture)
@@ -2864,11 +2871,30 @@ void Plan::prepare(const std::vector<BoxSpec> &specs, bool want_member) {
     for (const void *f : dense)
       CMH_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm));
   }
-  // the sort's scratch (issue() allocates nothing: it may be captured in a graph)
-  {
-    cell_states_apart = radix_states_apart(npc, key_bits, &cell_state_bytes);
-    sort_tmp.ensure(cell_state_bytes);
+  cell_states_apart = radix_states_apart(npc, key_bits, &cell_state_bytes);
+  need(sort_tmp, cell_state_bytes);
+  // (issue() allocates nothing: it may be captured in a graph)
+  auto room = [](size_t bytes) { return (bytes + 511) & ~(size_t)255; };
+  size_t total = 0;
+  for (const auto &q : pieces) total += room(q.second);
+  arena.ensure(total);
+  each_buf([](DevBuf &b) {
+    if (b.view) b.release();
+  });
+  total = 0;
+  for (const auto &q : pieces) {
+    q.first->place(arena, total, room(q.second));
+    total += room(q.second);
   }
+}
+
+// Host memory for `bytes` read back from the device: pinned from the plan's
+// second run on, else `unpinned`.
+unsigned char *Plan::host_room(size_t bytes, std::vector<unsigned char> &unpinned) {
+  if (runs > 0) pinned.ensure(bytes);
+  if (pinned.p && pinned.cap >= bytes) return static_cast<unsigned char *>(pinned.p);
+  unpinned.resize(bytes);
+  return unpinned.data();
 }
 
 void Plan::read_back(cudaStream_t s, bool timed) {
@@ -2878,13 +2904,15 @@ void Plan::read_back(cudaStream_t s, bool timed) {
     unsigned long long ngroups, nwarn;
   } hc;
   DevScal hs_;
-  small_host.resize(at_bucket);
-  CMH_CUDA(cudaMemcpyAsync(small_host.data(), scal.p, at_bucket, cudaMemcpyDeviceToHost, s));
+  std::vector<unsigned char> unpinned;
+  unsigned char *small = host_room(at_bucket, unpinned);
+  CMH_CUDA(cudaMemcpyAsync(small, scal.p, at_bucket, cudaMemcpyDeviceToHost, s));
   CMH_CUDA(cudaStreamSynchronize(s));
-  memcpy(&hs_, small_host.data(), sizeof hs_);
-  memcpy(&hc, small_host.data() + at_ctr, sizeof hc);
+  runs++;
+  memcpy(&hs_, small, sizeof hs_);
+  memcpy(&hc, small + at_ctr, sizeof hc);
   boxd_host.resize(7 * nbox);
-  memcpy(boxd_host.data(), small_host.data() + at_boxd, sizeof(uint32_t) * 7 * nbox);
+  memcpy(boxd_host.data(), small + at_boxd, sizeof(uint32_t) * 7 * nbox);
   last = hs_;
   // CMH_FAULT=overflow: the run is treated as having outgrown its buffers, so
   // it is repeated with room until the attempts run out (CMH_ERR_CAPACITY),
@@ -2929,7 +2957,7 @@ void Plan::read_back(cudaStream_t s, bool timed) {
   out_nhalos = hs_.nh;
 }
 
-void Plan::run_batch(const std::vector<BoxSpec> &specs, bool want_member, cudaStream_t s) {
+void Plan::run_batch(const std::vector<BoxSpec> &specs, int want_member, cudaStream_t s) {
   CMH_CUDA(cudaSetDevice(device));
   overwritten = false;
   for (int attempt = 0; attempt < 3; attempt++) {
@@ -3010,7 +3038,7 @@ void Plan::run_batch(const std::vector<BoxSpec> &specs, bool want_member, cudaSt
   fail(CMH_ERR_CAPACITY, "processed particles kept outgrowing the buffers");
 }
 
-void Plan::capture(bool want_member, cudaStream_t s, const std::vector<unsigned char> &sig) {
+void Plan::capture(int want_member, cudaStream_t s, const std::vector<unsigned char> &sig) {
   const int q = graph_next;
   graph_next = 1 - q;
   if (graph_exec[q]) {
@@ -3058,9 +3086,9 @@ cmh_tuning Plan::autotune(const std::vector<BoxSpec> &specs, int repeats, cudaSt
       release_workspace();
       float t = 0;
       try {
-        run_batch(specs, false, s);
+        run_batch(specs, 0, s);
         for (int r = 0; r < std::max(repeats, 1); r++) {
-          run_batch(specs, false, s);
+          run_batch(specs, 0, s);
           t += stats.ms_total;
         }
       } catch (const Error &e) {
@@ -3216,7 +3244,7 @@ std::vector<cmh_particles> Plan::take_inputs(const cmh_particles *parts, int nbo
   return dp;
 }
 
-void Plan::run(const cmh_particles &parts, bool want_member, cudaStream_t s) {
+void Plan::run(const cmh_particles &parts, int want_member, cudaStream_t s) {
   BoxSpec sp;
   sp.params = params;
   sp.ltab = ltab_host;

@@ -24,6 +24,14 @@ struct BoxSpec {
   int cell_factor = 0;  // 0: the params' value, or the autotuned one
 };
 
+// Pinned host memory.
+struct HostBuf {
+  void *p = nullptr;
+  size_t cap = 0;
+  void ensure(size_t bytes);
+  void release();
+};
+
 struct Plan : public cmh_plan {
   int device = 0;
   cmh_fof_params params{};
@@ -47,7 +55,11 @@ struct Plan : public cmh_plan {
   // byte offsets in `scal` of the counters, the per-box numbers, the buckets and
   // the sort's digit counts, and its bytes
   size_t at_ctr = 0, at_boxd = 0, at_bucket = 0, at_counts = 0, small_bytes = 0;
-  std::vector<unsigned char> small_host;
+  // what a run reads back passes through pinned memory from the plan's second run
+  // on (a single run would pay more for pinning than it saves)
+  HostBuf pinned;
+  int runs = 0;
+  unsigned char *host_room(size_t bytes, std::vector<unsigned char> &unpinned);
   bool cell_states_apart = false;  // each pass of the cell sort has its own tile states
   size_t cell_state_bytes = 0;
   int64_t run_tiles = 0;           // tiles of the gather
@@ -108,7 +120,8 @@ struct Plan : public cmh_plan {
   int samp_closed = 0;  // bit a: the domain includes its upper face on axis a
   const uint64_t *samp_ids = nullptr;
 
-  // workspace
+  // workspace: views of one allocation, laid out for each run's shape
+  DevBuf arena;
   DevBuf scal, sort_tmp, b_tiles, ltab_dev, b_boxes;
   DevBuf b_keys, b_keys_alt, b_vals, b_vals_alt, b_recs, b_spos, b_svl;
   DevBuf b_run_box, b_top_range, b_top_slot;
@@ -138,14 +151,15 @@ struct Plan : public cmh_plan {
   void set_params(const cmh_fof_params &p);
   Geom make_geometry(const cmh_fof_params &p, const std::vector<double> &ltab, int64_t n_in,
                      int cell_factor) const;
-  void prepare(const std::vector<BoxSpec> &specs, bool want_member);
+  // want_member: 0 no membership, 1 the whole, 2 the halo indices only
+  void prepare(const std::vector<BoxSpec> &specs, int want_member);
   template <class PT>
-  void issue(bool want_member, cudaStream_t s, bool timed);
+  void issue(int want_member, cudaStream_t s, bool timed);
   void read_back(cudaStream_t s, bool timed);
-  void capture(bool want_member, cudaStream_t s, const std::vector<unsigned char> &sig);
-  void run_batch(const std::vector<BoxSpec> &specs, bool want_member, cudaStream_t s);
+  void capture(int want_member, cudaStream_t s, const std::vector<unsigned char> &sig);
+  void run_batch(const std::vector<BoxSpec> &specs, int want_member, cudaStream_t s);
   cmh_tuning autotune(const std::vector<BoxSpec> &specs, int repeats, cudaStream_t s);
-  void run(const cmh_particles &parts, bool want_member, cudaStream_t s);
+  void run(const cmh_particles &parts, int want_member, cudaStream_t s);
   // host inputs of nbox boxes: start copying them into input buffer `buf`
   // (after the caller's queued work; every box's positions before any
   // velocities), returning the buffer; take the staged inputs that match

@@ -140,6 +140,10 @@ typedef struct cmh_catalog {
   void *impl;          /* library-owned storage                               */
 } cmh_catalog;
 
+/* Values of `want_member` below: 0 no membership, CMH_MEMBER_INDEX cat->member
+ * alone (member_proc and member_pos stay NULL), anything else all three. */
+#define CMH_MEMBER_INDEX 0x6d656d31
+
 typedef struct cmh_plan cmh_plan;
 
 /* ---- library ------------------------------------------------------------ */
