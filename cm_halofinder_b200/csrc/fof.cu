@@ -2366,10 +2366,22 @@ Geom Plan::make_geometry(const cmh_fof_params &p, const std::vector<double> &lta
   }
   int k = cell_factor > 0 ? cell_factor : p.cell_factor;
   if (k <= 0) {
-    // one top cell per particle on average, as the reference's lcell = L/Px,
-    // times the autotuned scale
-    const double sep = std::cbrt(vol / std::max<double>((double)n_in, 1.0));
-    k = (int)std::lround(sep / g.h * cell_scale);
+    // About one top cell per particle, as the reference's lcell = L/Px, or the
+    // tuned scale of it.  Untuned, somewhat smaller top cells for runs of up to
+    // 32M particles, where the largest dense top cells bound the befriending
+    // (scale 0.85 against 1: 64^3 box 0.361 and 0.384 ms, 1.5M particles 0.67 and
+    // 0.71, 64 boxes 10.5 and 10.9, 256^3 box 3.43 and 3.43, but the 512^3 box 32.9
+    // and 32.4); and none of more than 10^3 fine cells where that leaves at
+    // most four top cells per particle (50M lightcone 10.6 ms with 10, 11.5 with
+    // 14; 700,000-particle one 0.57 and 0.73), in runs whose top-cell tables are
+    // small beside the device's memory.
+    const double sep = std::cbrt(vol / std::max<double>((double)n_in, 1.0)) / g.h;
+    if (cell_scale > 0) {
+      k = (int)std::lround(sep * cell_scale);
+    } else {
+      k = (int)std::lround(sep * (n_in <= (int64_t)1 << 25 ? 0.85 : 1.0));
+      if (n_in < (int64_t)1 << 28) k = std::min(k, std::max(10, (int)std::ceil(0.63 * sep)));
+    }
   }
   if (g.W > kMaxCellFactor)
     fail(CMH_ERR_INVALID_ARGUMENT, "linking lengths span too wide a range (longest / shortest "

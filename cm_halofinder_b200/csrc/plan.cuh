@@ -40,7 +40,7 @@ struct Plan : public cmh_plan {
   bool fp32 = true;
   bool use_graph = true;    // replay the captured run when its shape repeats
   uint32_t dense_min = 16;  // top cells with more occupied fine cells get a map
-  double cell_scale = 1.0;  // autotuned scale of the default cell-size factor
+  double cell_scale = 0.0;  // tuned scale of the cell-size factor (0: by rule)
   // bounds of the device loops that retry or wait (cmh_plan_set_limits)
   uint32_t union_cap = kUnionCap;  // retries of one union after a lost race
   uint32_t spin_cap = kSpinCap;    // polls of one sort tile state
