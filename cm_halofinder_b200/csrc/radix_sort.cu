@@ -87,11 +87,15 @@ constexpr int kSThreads = 512;
 constexpr int kSWarps = kSThreads / 32;
 constexpr int kSIPT = kTile / kSThreads;  // 8
 
-template <class K, int BINS>
+// A tile in shared memory: its pairs in digit order, with the digits where the
+// written keys no longer hold them, and 16-bit counters (a tile has 4096 keys;
+// 32-bit ones cost the 9-bit passes a CTA per SM).
+template <class KO, int BINS, bool NARROW>
 struct ScatterSmem {
-  K keys[kTile];
+  KO keys[kTile];
   uint32_t vals[kTile];
-  uint32_t wcnt[kSWarps][BINS];
+  uint8_t digit[NARROW ? kTile : 4];
+  uint16_t wcnt[kSWarps][BINS];
   uint32_t dstart[BINS];
   uint32_t gofs[BINS];
   uint32_t thist[BINS];
@@ -116,12 +120,15 @@ __device__ __forceinline__ uint64_t load_state(const uint64_t *p) {
   return *reinterpret_cast<const volatile uint64_t *>(p);
 }
 
-// Keys are read as K and written as KO = K >> out_shift (out_shift 0 unless
-// the pass narrows 64-bit keys to 32 bits); digits have log2(BINS) bits.
-// With 32-bit keys and 8-bit digits a CTA's shared memory is small enough for
-// 4 CTAs per SM.
-template <class K, class KO, int BINS>
-__global__ void __launch_bounds__(kSThreads, (sizeof(K) == 4 && BINS == BINS) ? 4 : 3) k_rs_scatter(
+// Keys are read as K and written as KO: K >> out_shift in a pass that narrows
+// 64-bit keys to 32 bits (NARROW), K itself otherwise, and not at all in the last
+// pass; digits have log2(BINS) bits.  Bound by instruction issue (ranking and
+// staging).  256^3 box, 17.7M keys: 0.26 + 0.22 + 0.21 + 0.17 ms with 32-bit
+// counters, whole keys staged in the narrowing pass and keys written in the last,
+// 0.22 + 0.20 + 0.20 + 0.16 ms so; counts published after the ranking, which then
+// needs no second histogram: 0.22 + 0.21 + 0.21 + 0.16.
+template <class K, class KO, int BINS, bool NARROW, bool LAST>
+__global__ void __launch_bounds__(kSThreads, NARROW || sizeof(KO) == 8 ? 3 : 4) k_rs_scatter(
     KeySource<K> keys_in, const uint32_t *__restrict__ vals_in,
     KO *__restrict__ keys_out, uint32_t *__restrict__ vals_out, int64_t n_cap,
     const uint32_t *__restrict__ n_dev, int shift, int out_shift,
@@ -130,31 +137,36 @@ __global__ void __launch_bounds__(kSThreads, (sizeof(K) == 4 && BINS == BINS) ? 
     unsigned int *__restrict__ giveups, SortWaits waits) {
   const int64_t n = n_dev ? (int64_t)*n_dev : n_cap;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  ScatterSmem<K, BINS> &sm = *reinterpret_cast<ScatterSmem<K, BINS> *>(smem_raw);
+  using Smem = ScatterSmem<KO, BINS, NARROW>;
+  Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) sm.tile = atomicAdd(tile_ctr, 1u);
-  for (int i = threadIdx.x; i < kSWarps * BINS; i += kSThreads) (&sm.wcnt[0][0])[i] = 0;
+  for (int i = threadIdx.x; i < kSWarps * BINS / 2; i += kSThreads)
+    reinterpret_cast<uint32_t *>(&sm.wcnt[0][0])[i] = 0;
   if (threadIdx.x < BINS) sm.thist[threadIdx.x] = 0;
   __syncthreads();
   const uint32_t tile = sm.tile;
   const int64_t base = (int64_t)tile * kTile;
   if (base >= n) return;  // the whole CTA leaves together
   const uint32_t lt_mask = (1u << lane) - 1u;
-  K k[kSIPT];
-  uint32_t v[kSIPT], rank[kSIPT];
+  const int rem = n - base < kTile ? (int)(n - base) : kTile;
+  const int mine = warp * 32 * kSIPT + lane;  // the thread's keys: mine + 32 j
+  KO k[kSIPT];
+  uint32_t v[kSIPT], dr[kSIPT];  // digit, later digit | rank << 16
 #pragma unroll
   for (int j = 0; j < kSIPT; j++) {
-    const int64_t i = base + (int64_t)warp * 32 * kSIPT + j * 32 + lane;
-    const bool valid = i < n;
-    k[j] = valid ? keys_in[i] : K(0);
+    const int64_t i = base + mine + 32 * j;
+    const bool valid = mine + 32 * j < rem;
+    const K key = valid ? keys_in[i] : K(0);
+    k[j] = NARROW ? (KO)(key >> out_shift) : (KO)key;
+    dr[j] = valid ? digit_of<BINS>(key, shift) : (uint32_t)BINS;
     v[j] = valid ? (vals_in ? vals_in[i] : (uint32_t)i) : 0u;
   }
   // the tile's digit counts first, published before the ranking so that
   // the higher tiles' look-back finds them early
 #pragma unroll
   for (int j = 0; j < kSIPT; j++)
-    if (base + (int64_t)warp * 32 * kSIPT + j * 32 + lane < n)
-      atomicAdd(&sm.thist[digit_of<BINS>(k[j], shift)], 1u);
+    if (dr[j] < BINS) atomicAdd(&sm.thist[dr[j]], 1u);
   __syncthreads();
   // (a tile named by waits.stall_tile publishes nothing: a test hook whose
   // successor's capped wait then runs out)
@@ -163,17 +175,16 @@ __global__ void __launch_bounds__(kSThreads, (sizeof(K) == 4 && BINS == BINS) ? 
                (unsigned long long)((tile == 0 ? kInclusive : kAggregate) | sm.thist[threadIdx.x]));
 #pragma unroll
   for (int j = 0; j < kSIPT; j++) {
-    const int64_t i = base + (int64_t)warp * 32 * kSIPT + j * 32 + lane;
-    const bool valid = i < n;
-    const uint32_t d = valid ? digit_of<BINS>(k[j], shift) : (uint32_t)BINS;
+    const uint32_t d = dr[j];
+    const bool valid = d < BINS;
     const uint32_t peers = peers_of<BINS == 512 ? 10 : 9>(d);
     const uint32_t lt = peers & lt_mask;
     uint32_t c = 0;
     if (valid) c = sm.wcnt[warp][d];
     __syncwarp();
-    if (valid && lt == 0) sm.wcnt[warp][d] = c + __popc(peers);
+    if (valid && lt == 0) sm.wcnt[warp][d] = (uint16_t)(c + __popc(peers));
     __syncwarp();
-    rank[j] = c + __popc(lt);
+    dr[j] = d | (c + __popc(lt)) << 16;
   }
   __syncthreads();
   {
@@ -183,8 +194,8 @@ __global__ void __launch_bounds__(kSThreads, (sizeof(K) == 4 && BINS == BINS) ? 
     if (d < BINS) {
 #pragma unroll
       for (int w = 0; w < kSWarps; w++) {
-        uint32_t t = sm.wcnt[w][d];
-        sm.wcnt[w][d] = acc;
+        const uint32_t t = sm.wcnt[w][d];
+        sm.wcnt[w][d] = (uint16_t)acc;
         acc += t;
       }
     }
@@ -198,9 +209,10 @@ __global__ void __launch_bounds__(kSThreads, (sizeof(K) == 4 && BINS == BINS) ? 
     }
     __syncthreads();
     if (d < BINS) {
-      sm.dstart[d] = inc - acc + sm.warp_sums[warp];
+      const uint32_t first = inc - acc + sm.warp_sums[warp];
+      sm.dstart[d] = first;
       // add up the lower tiles' counts, then publish the running total
-      uint64_t *mine = state + (uint64_t)tile * BINS + d;
+      uint64_t *own = state + (uint64_t)tile * BINS + d;
       uint32_t excl = 0;
       if (tile != 0) {
         for (int64_t j = (int64_t)tile - 1; j >= 0; j--) {
@@ -216,37 +228,57 @@ __global__ void __launch_bounds__(kSThreads, (sizeof(K) == 4 && BINS == BINS) ? 
           if ((w >> 32) == 2) break;
         }
         if (tile != waits.stall_tile)
-          atomicExch(reinterpret_cast<unsigned long long *>(mine),
+          atomicExch(reinterpret_cast<unsigned long long *>(own),
                      (unsigned long long)(kInclusive | (uint64_t)(excl + acc)));
       }
-      sm.gofs[d] = goff[d] + excl;
+      sm.gofs[d] = goff[d] + excl - first;  // (modulo 2^32: first is added back below)
     }
   }
   __syncthreads();
-  const int64_t rem = n - base;
 #pragma unroll
   for (int j = 0; j < kSIPT; j++) {
-    const int64_t i = base + (int64_t)warp * 32 * kSIPT + j * 32 + lane;
-    if (i < n) {
-      const uint32_t d = digit_of<BINS>(k[j], shift);
-      const uint32_t lp = sm.dstart[d] + sm.wcnt[warp][d] + rank[j];
+    const uint32_t d = dr[j] & 0xffffu;
+    if (d < BINS) {
+      const uint32_t lp = sm.dstart[d] + sm.wcnt[warp][d] + (dr[j] >> 16);
       sm.keys[lp] = k[j];
       sm.vals[lp] = v[j];
+      if constexpr (NARROW) sm.digit[lp] = (uint8_t)d;
     }
   }
   __syncthreads();
-  const int tile_n = rem < kTile ? (int)rem : kTile;
-  for (int q = threadIdx.x; q < tile_n; q += kSThreads) {
-    const K key = sm.keys[q];
-    const uint32_t d = digit_of<BINS>(key, shift);
-    const uint32_t g = sm.gofs[d] + (uint32_t)q - sm.dstart[d];
-    keys_out[g] = (KO)(key >> out_shift);
+  for (int q = threadIdx.x; q < rem; q += kSThreads) {
+    const KO key = sm.keys[q];
+    const uint32_t d = NARROW ? sm.digit[q] : digit_of<BINS>(key, shift);
+    const uint32_t g = sm.gofs[d] + (uint32_t)q;
+    if constexpr (!LAST) keys_out[g] = key;
     vals_out[g] = sm.vals[q];
   }
 }
 
+// A pass: its kernel and dynamic shared memory.
+template <class K, class KO, int BINS, bool NARROW, bool LAST>
+void scatter_pass(const void *keys, uint32_t stride, const uint32_t *vals, void *keys_out,
+                  uint32_t *vals_out, int64_t n, const uint32_t *n_dev, int shift, int out_shift,
+                  const uint32_t *goff, uint64_t *state, uint32_t *tile_ctr,
+                  unsigned int *giveups, SortWaits waits, cudaStream_t s) {
+  constexpr size_t smem = sizeof(ScatterSmem<KO, BINS, NARROW>);
+  const int64_t ntiles = (n + kTile - 1) / kTile;
+  k_rs_scatter<K, KO, BINS, NARROW, LAST><<<(unsigned)ntiles, kSThreads, smem, s>>>(
+      KeySource<K>{static_cast<const K *>(keys), stride}, vals, static_cast<KO *>(keys_out),
+      vals_out, n, n_dev, shift, out_shift, goff, state, tile_ctr, giveups, waits);
+  CMH_LAUNCHED();
+}
+
 // Dynamic shared memory of every scatter instantiation, set once per device
 // (never inside a graph capture).
+template <class K, class KO, int BINS, bool NARROW> void set_smem() {
+  const int bytes = (int)sizeof(ScatterSmem<KO, BINS, NARROW>);
+  CMH_CUDA(cudaFuncSetAttribute(k_rs_scatter<K, KO, BINS, NARROW, false>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  CMH_CUDA(cudaFuncSetAttribute(k_rs_scatter<K, KO, BINS, NARROW, true>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+}
+
 void set_scatter_smem(cudaStream_t s) {
   static bool done[64] = {};
   int dev = 0;
@@ -254,18 +286,10 @@ void set_scatter_smem(cudaStream_t s) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   CMH_CUDA(cudaStreamIsCapturing(s, &cs));
   if (dev >= 64 || done[dev] || cs != cudaStreamCaptureStatusNone) return;
-  CMH_CUDA(cudaFuncSetAttribute(k_rs_scatter<uint64_t, uint64_t, kBins>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(ScatterSmem<uint64_t, kBins>)));
-  CMH_CUDA(cudaFuncSetAttribute(k_rs_scatter<uint64_t, uint32_t, kBins>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(ScatterSmem<uint64_t, kBins>)));
-  CMH_CUDA(cudaFuncSetAttribute(k_rs_scatter<uint32_t, uint32_t, kBins>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(ScatterSmem<uint32_t, kBins>)));
-  CMH_CUDA(cudaFuncSetAttribute(k_rs_scatter<uint32_t, uint32_t, kMaxBins>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(ScatterSmem<uint32_t, kMaxBins>)));
+  set_smem<uint64_t, uint64_t, kBins, false>();
+  set_smem<uint64_t, uint32_t, kBins, true>();
+  set_smem<uint32_t, uint32_t, kBins, false>();
+  set_smem<uint32_t, uint32_t, kMaxBins, false>();
   done[dev] = true;
 }
 
@@ -343,32 +367,25 @@ void radix_order_records(const void *records, uint32_t stride, uint32_t key_at, 
     uint32_t *dst_v = out_v[p % 2];
     // the stall hook applies to the first pass only
     const SortWaits wp{waits.spin_cap, p == 0 ? waits.stall_tile : 0xffffffffu};
-    const KeySource<uint64_t> s8{static_cast<const uint64_t *>(src_k), src_stride};
-    const KeySource<uint32_t> s4{static_cast<const uint32_t *>(src_k), src_stride};
-    if (p < m - 1) {
-      k_rs_scatter<uint64_t, uint64_t, kBins>
-          <<<(unsigned)ntiles, kSThreads, sizeof(ScatterSmem<uint64_t, kBins>), s>>>(
-              s8, src_v, static_cast<uint64_t *>(dst_k), dst_v, n, n_dev, pd.shift[p], 0, go,
-              state, tile_ctr + p, giveups, wp);
-      src_stride = sizeof(uint64_t);
-    } else if (p < m) {
-      k_rs_scatter<uint64_t, uint32_t, kBins>
-          <<<(unsigned)ntiles, kSThreads, sizeof(ScatterSmem<uint64_t, kBins>), s>>>(
-              s8, src_v, static_cast<uint32_t *>(dst_k), dst_v, n, n_dev, pd.shift[p], 8 * m, go,
-              state, tile_ctr + p, giveups, wp);
-      src_stride = sizeof(uint32_t);
-    } else if (bins == kMaxBins) {
-      k_rs_scatter<uint32_t, uint32_t, kMaxBins>
-          <<<(unsigned)ntiles, kSThreads, sizeof(ScatterSmem<uint32_t, kMaxBins>), s>>>(
-              s4, src_v, static_cast<uint32_t *>(dst_k), dst_v, n, n_dev, pd.shift[p] - 8 * m, 0,
-              go, state, tile_ctr + p, giveups, wp);
-    } else {
-      k_rs_scatter<uint32_t, uint32_t, kBins>
-          <<<(unsigned)ntiles, kSThreads, sizeof(ScatterSmem<uint32_t, kBins>), s>>>(
-              s4, src_v, static_cast<uint32_t *>(dst_k), dst_v, n, n_dev, pd.shift[p] - 8 * m, 0,
-              go, state, tile_ctr + p, giveups, wp);
-    }
-    CMH_LAUNCHED();
+    const bool last = p == pd.passes - 1;
+    auto run = [&](auto pass, auto last_pass) {
+      (last ? last_pass : pass)(src_k, src_stride, src_v, dst_k, dst_v, n, n_dev,
+                                p < m ? pd.shift[p] : pd.shift[p] - 8 * m, 8 * m, go, state,
+                                tile_ctr + p, giveups, wp, s);
+    };
+    if (p < m - 1)
+      run(scatter_pass<uint64_t, uint64_t, kBins, false, false>,
+          scatter_pass<uint64_t, uint64_t, kBins, false, true>);
+    else if (p < m)
+      run(scatter_pass<uint64_t, uint32_t, kBins, true, false>,
+          scatter_pass<uint64_t, uint32_t, kBins, true, true>);
+    else if (bins == kMaxBins)
+      run(scatter_pass<uint32_t, uint32_t, kMaxBins, false, false>,
+          scatter_pass<uint32_t, uint32_t, kMaxBins, false, true>);
+    else
+      run(scatter_pass<uint32_t, uint32_t, kBins, false, false>,
+          scatter_pass<uint32_t, uint32_t, kBins, false, true>);
+    src_stride = p < m - 1 ? sizeof(uint64_t) : sizeof(uint32_t);
     if (tmp.apart) state += (size_t)ntiles * bins;
     src_k = dst_k;
     src_v = dst_v;
