@@ -1473,11 +1473,13 @@ template <class PT, bool FP32, bool VL>
 __global__ void __launch_bounds__(kT, 4) k_befriend_sparse(
     const PairArgs<PT, FP32> A, DevScal *sc, const uint2 *__restrict__ top_range,
     const uint32_t *__restrict__ top_slot, uint32_t *parent, uint32_t *__restrict__ q_cell,
-    uint32_t *__restrict__ q_top, uint32_t q_cap) {
+    uint32_t *__restrict__ q_top, uint32_t q_cap, uint32_t dense_min) {
   if (sc->failed) return;  // a sort of this run gave up: its order is not valid
   const uint32_t R = sc->R;
   const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5, below = (1u << lane) - 1u;
-  __shared__ uint2 s_item[kT / 32][kListSlots];  // {fine cell, neighbour}
+  // {fine cell, forward neighbour (below 14) or 15 + distance in key order of a
+  // fine cell in its own top cell}
+  __shared__ uint2 s_item[kT / 32][kListSlots];
   __shared__ uint2 s_cand[kT / 32][kListSlots];  // {fine cell, candidate}
   __shared__ uint2 s_pairs[kT / 32][kPairSlots];
   uint2 *items = s_item[wid], *cands = s_cand[wid], *pairs = s_pairs[wid];
@@ -1497,19 +1499,57 @@ __global__ void __launch_bounds__(kT, 4) k_befriend_sparse(
     const bool last = base >= R;
     const uint32_t end = last ? base + 1 : min(base + step, R);
     for (uint32_t a0 = base; a0 < end || last; a0 += 32) {
-      uint32_t tops = 0;
-      if (!last && a0 + lane < end) {
-        const Geom &g = A.boxes[A.run_box[a0 + lane]].g;
-        const uint64_t pg = A.run_g[a0 + lane];
-        const int c[3] = {(int)(pg & kM21), (int)((pg >> 21) & kM21), (int)(pg >> 42)};
-        const int t[3] = {div_k(c[0], g), div_k(c[1], g), div_k(c[2], g)};
-        const int f[3] = {c[0] - t[0] * g.k, c[1] - t[1] * g.k, c[2] - t[2] * g.k};
-        tops = reached_tops(g, g.W, t, f);
+      uint32_t tops = 0, own = 0;  // own: bit d, fine cell a + 1 + d of a's top cell
+      {
+        const bool act = !last && a0 + lane < end;
+        uint64_t pg = 0, t_own = ~0ull;
+        int W = 0;
+        if (act) {
+          const BoxDev &bx = A.boxes[A.run_box[a0 + lane]];
+          const Geom &g = bx.g;
+          pg = A.run_g[a0 + lane];
+          const int c[3] = {(int)(pg & kM21), (int)((pg >> 21) & kM21), (int)(pg >> 42)};
+          const int t[3] = {div_k(c[0], g), div_k(c[1], g), div_k(c[2], g)};
+          const int f[3] = {c[0] - t[0] * g.k, c[1] - t[1] * g.k, c[2] - t[2] * g.k};
+          W = g.W;
+          tops = reached_tops(g, W, t, f);
+          t_own = bx.top_base + ((uint64_t)t[2] * g.T[1] + t[1]) * g.T[0] + t[0];
+        }
+        // The rest of a's top cell lies in the following lanes, unless it goes on
+        // past the warp's last cell (then it is an item like the others).
+        // A top cell that starts here and has at most dense_min fine cells is
+        // sparse; of the others the slot tells.
+        const uint64_t t_prev = __shfl_up_sync(0xffffffffu, t_own, 1);
+        const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0 || t_own != t_prev);
+        const uint32_t acts = __ballot_sync(0xffffffffu, act);
+        const uint32_t after = heads & ~((2u << lane) - 1u);  // (none past the last lane)
+        const bool whole = act && after && (acts >> (__ffs(after) - 1) & 1u);
+        uint32_t n = 0;
+        if (whole) {
+          tops &= ~1u;
+          n = (uint32_t)__ffs(after) - 2u - lane;
+          if (n) {
+            const uint32_t first = 31u - (uint32_t)__clz((int)(heads & ((2u << lane) - 1u)));
+            if ((first == 0 || lane - first + n + 1 > dense_min) && top_slot[t_own] != kNone) n = 0;
+          }
+        }
+        const uint32_t most = __reduce_max_sync(0xffffffffu, n);
+        for (uint32_t d = 1; d <= most; d++) {
+          const uint64_t qg = __shfl_down_sync(0xffffffffu, pg, d);
+          if (d <= n &&
+              max(abs((int)(qg & kM21) - (int)(pg & kM21)),
+                  max(abs((int)((qg >> 21) & kM21) - (int)((pg >> 21) & kM21)),
+                      abs((int)(qg >> 42) - (int)(pg >> 42)))) <= W)
+            own |= 1u << (d - 1);
+        }
       }
       do {
         {
-          const uint32_t m = __ballot_sync(0xffffffffu, tops != 0);
-          if (tops) {
+          const uint32_t m = __ballot_sync(0xffffffffu, (tops | own) != 0);
+          if (own) {
+            items[nitem + __popc(m & below)] = make_uint2(a0 + lane, 15u + (uint32_t)__ffs(own));
+            own &= own - 1u;
+          } else if (tops) {
             items[nitem + __popc(m & below)] = make_uint2(a0 + lane, (uint32_t)__ffs(tops) - 1u);
             tops &= tops - 1u;
           }
@@ -1533,15 +1573,20 @@ __global__ void __launch_bounds__(kT, 4) k_befriend_sparse(
           gy = (int)((pg >> 21) & kM21);
           gz = (int)(pg >> 42);
           W = g.W;
-          const uint64_t tb = bx.top_base +
-                              ((uint64_t)(div_k(gz, g) + kFwd[nb][2]) * g.T[1] +
-                               (uint64_t)(div_k(gy, g) + kFwd[nb][1])) * g.T[0] +
-                              (uint64_t)(div_k(gx, g) + kFwd[nb][0]);
-          const uint2 tr = top_range[tb];
-          slot = top_slot[tb];
-          r0 = nb == 0 ? a + 1 : tr.x;
-          cnt = tr.y > r0 ? tr.y - r0 : 0u;
-          if (nb == 0 && slot != kNone) cnt = 0;  // k_befriend_dense's
+          if (nb < 14) {
+            const uint64_t tb = bx.top_base +
+                                ((uint64_t)(div_k(gz, g) + kFwd[nb][2]) * g.T[1] +
+                                 (uint64_t)(div_k(gy, g) + kFwd[nb][1])) * g.T[0] +
+                                (uint64_t)(div_k(gx, g) + kFwd[nb][0]);
+            const uint2 tr = top_range[tb];
+            slot = top_slot[tb];
+            r0 = nb == 0 ? a + 1 : tr.x;
+            cnt = tr.y > r0 ? tr.y - r0 : 0u;
+            if (nb == 0 && slot != kNone) cnt = 0;  // k_befriend_dense's
+          } else {
+            r0 = a + nb - 15u;  // a fine cell of a's own top cell, in reach
+            cnt = 1;
+          }
         }
         const bool dense = cnt != 0 && slot != kNone;
         const uint32_t qm = __ballot_sync(0xffffffffu, dense);
@@ -1602,7 +1647,7 @@ __global__ void __launch_bounds__(kT, 4) k_befriend_sparse(
             } while (flush && ncand);
           } while (__any_sync(0xffffffffu, todo != 0));
         }
-      } while (__any_sync(0xffffffffu, tops != 0));
+      } while (__any_sync(0xffffffffu, (tops | own) != 0));
       if (last) break;
     }
     if (last) break;
@@ -2618,7 +2663,7 @@ void Plan::issue(int want_member, cudaStream_t s, bool timed) {
     CMH_CUDA(cudaEventRecord(ev_join, bf_stream));
     k_befriend_sparse<PT, FP, VL><<<rg(k_befriend_sparse<PT, FP, VL>, npc), kT, 0, s>>>(
         pa, sc, b_top_range.as<uint2>(), b_top_slot.as<uint32_t>(), parent,
-        q_cell, q_top, q_cap);
+        q_cell, q_top, q_cap, dense_min);
     CMH_LAUNCHED();
     CMH_CUDA(cudaStreamWaitEvent(s, ev_join, 0));
     k_befriend_cross<PT, FP, VL, 0><<<rg(k_befriend_cross<PT, FP, VL, 0>, npc * 8), kT, 0, s>>>(
