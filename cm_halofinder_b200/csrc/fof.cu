@@ -786,10 +786,6 @@ __global__ void __launch_bounds__(kT) k_varlink_recs(const SPos<PT> *__restrict_
   }
 }
 
-// Dense top cells with more fine cells than this are joined by a whole CTA,
-// the others by one warp each.
-constexpr uint32_t kBigTop = 64;
-
 // Warp-aggregated slot from a counter for the lanes with `pick` set: one
 // atomic per warp, the lanes in lane order after the returned base.
 __device__ __forceinline__ uint32_t warp_slot(bool pick, uint32_t *counter) {
@@ -813,7 +809,8 @@ __global__ void __launch_bounds__(kT) k_dense_pick(const uint64_t *__restrict__ 
                                                    const BoxDev *__restrict__ boxes,
                                                    DevScal *sc,
                                                    const uint2 *__restrict__ top_range,
-                                                   uint32_t dense_min, uint32_t nd_cap,
+                                                   uint32_t dense_min, uint32_t big_min,
+                                                   uint32_t nd_cap,
                                                    uint32_t *__restrict__ top_slot,
                                                    uint2 *__restrict__ dense_range,
                                                    uint32_t *__restrict__ big) {
@@ -835,7 +832,7 @@ __global__ void __launch_bounds__(kT) k_dense_pick(const uint64_t *__restrict__ 
     if (slot < nd_cap) {
       top_slot[t] = slot;
       dense_range[slot] = tr;
-      if (tr.y - tr.x > kBigTop) big[atomicAdd(&sc->nbig, 1u)] = slot;
+      if (tr.y - tr.x > big_min) big[atomicAdd(&sc->nbig, 1u)] = slot;
     } else {
       atomicOr(&sc->overflow, 2u);
     }
@@ -1032,10 +1029,11 @@ struct LocalUF {
 constexpr uint32_t kPairSlots = 64;
 // Steps that one lane spends on a cell pair by itself; the whole warp takes
 // those that need more, 32 particle pairs a step.  Most pairs that link do so
-// within a few steps (of the 256^3 box's 2 million listed pairs a few hundred
-// need the warp), and giving the warp every pair of more than 32 particle
-// pairs made the dense kernel 1.6 times as long.
-constexpr int kSoloSteps = 48;
+// within a few steps: 8, 16, 24 and 48 steps give a befriending of 1.09, 1.10,
+// 1.11 and 1.13 ms for the 256^3 box and 0.154, 0.144, 0.149 and 0.158 ms for the
+// 64^3 one; giving the warp every pair of more than 32 particle pairs made the
+// dense kernel 1.6 times as long.
+constexpr int kSoloSteps = 16;
 
 // What the pair tests read, the same for all warps of a kernel.
 template <class PT, bool FP32>
@@ -1380,7 +1378,7 @@ __device__ __forceinline__ void dense_top(const PairArgs<PT, FP32> &A, uint32_t 
   sync();
 }
 
-// The dense top cells.  The big ones (more than kBigTop fine cells, listed
+// The dense top cells.  The big ones (more than big_min fine cells, listed
 // in `big`) go first, one per CTA, so that the largest, which bound the
 // kernel's length, start early and have many threads; then each warp takes
 // the small ones one at a time, with its own slice of `lstride` words of
@@ -1390,7 +1388,7 @@ template <class PT, bool FP32, bool VL>
 __global__ void __launch_bounds__(128) k_befriend_dense(
     const PairArgs<PT, FP32> A, uint64_t k3all, const uint2 *__restrict__ dense_range,
     const uint32_t *__restrict__ big, DevScal *sc, uint32_t nd_cap, uint4 *__restrict__ grows,
-    uint32_t kk, uint32_t rows_stride, uint32_t *parent, uint32_t lstride) {
+    uint32_t kk, uint32_t rows_stride, uint32_t *parent, uint32_t lstride, uint32_t big_min) {
   if (sc->failed) return;  // a sort of this run gave up: its order is not valid
   extern __shared__ uint32_t smem[];
   __shared__ uint32_t s_slot;
@@ -1420,7 +1418,7 @@ __global__ void __launch_bounds__(128) k_befriend_dense(
       slot = __shfl_sync(0xffffffffu, slot, 0);
       if (slot >= nd) break;
       const uint2 fr = dense_range[slot];
-      if (fr.y - fr.x > kBigTop) continue;
+      if (fr.y - fr.x > big_min) continue;
     }
     dense_top<PT, FP32, VL>(A, slot, cta ? smem : own, cta, pairs, k3all, dense_range, grows, kk,
                             rows_stride, parent, st);
@@ -2465,6 +2463,15 @@ uint64_t dense_words(uint64_t k3all) {
   return k3all + 3 * k * k + 2;
 }
 
+// Fine cells above which a dense top cell is joined by a whole CTA, not a warp.
+// A CTA shortens one top cell's chain of steps, which bounds a small run, but
+// waits at its barriers, which costs a large one.  Befriending with 32, 64, 128
+// and 300: 64^3 box 0.137, 0.150, 0.187, 0.215 ms; 1.5M particles 0.231, 0.223,
+// 0.262, 0.332; 256^3 box 1.16, 1.11, 1.09, 1.14; 512^3 box 14.3, 13.1, 12.5, 12.1.
+uint32_t big_top_min(int64_t np) {
+  return (uint32_t)std::max(32.0, 48.0 * std::pow((double)np / 1e6, 0.35));
+}
+
 // Warps per CTA of the dense-top kernel: up to 4, each with the words of one
 // top cell, within 200 KiB per CTA.
 int dense_warps_per_cta(uint64_t k3all) {
@@ -2631,8 +2638,9 @@ void Plan::issue(int want_member, cudaStream_t s, bool timed) {
                                                   b_svl.as<VLRec64>());
     CMH_LAUNCHED();
   }
+  const uint32_t big_min = big_top_min(npc);
   k_dense_pick<<<rg(k_dense_pick, npc), kT, 0, s>>>(
-      run_g, b_run_box.as<uint16_t>(), boxes, sc, b_top_range.as<uint2>(), dense_min,
+      run_g, b_run_box.as<uint16_t>(), boxes, sc, b_top_range.as<uint2>(), dense_min, big_min,
       (uint32_t)nd_cap, b_top_slot.as<uint32_t>(), b_dense_range.as<uint2>(),
       b_dense_big.as<uint32_t>());
   CMH_LAUNCHED();
@@ -2658,7 +2666,8 @@ void Plan::issue(int want_member, cudaStream_t s, bool timed) {
                               b_spos.as<SPos<PT>>(), svl, c};
     k_befriend_dense<PT, FP, VL><<<gd, 32 * dwpc, dsm, bf_stream>>>(
         pa, k3all, b_dense_range.as<uint2>(), b_dense_big.as<uint32_t>(), sc, (uint32_t)nd_cap,
-        b_rows.as<uint4>(), kk, rows_stride, parent, (uint32_t)dense_words(k3all));
+        b_rows.as<uint4>(), kk, rows_stride, parent, (uint32_t)dense_words(k3all),
+        big_min);
     CMH_LAUNCHED();
     CMH_CUDA(cudaEventRecord(ev_join, bf_stream));
     k_befriend_sparse<PT, FP, VL><<<rg(k_befriend_sparse<PT, FP, VL>, npc), kT, 0, s>>>(
