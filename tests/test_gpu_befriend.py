@@ -6,7 +6,7 @@ the smallest to the largest), with few and with many queued cells."""
 import numpy as np
 import pytest
 
-from cm_halofinder_b200 import FofConfig, fof, synth
+from cm_halofinder_b200 import FofConfig, Plan, fof, synth
 from oracle import cpu
 from tests.helpers import assert_same_catalog
 
@@ -66,3 +66,29 @@ def test_reach_of_a_variable_length(ratio):
     tab = np.linspace(w.linklength / ratio, w.linklength, 65)
     w.varlink = {"origin": (0.0,) * 3, "rmax": float(w.hi[0]), "table": tab}
     assert_same_catalog(fof(w.pos, w.vel, FofConfig.from_workload(w), members=True), cpu.run(w))
+
+
+@pytest.mark.parametrize("cell_factor,dense_min", [(4, 4), (8, 16), (3, 1)])
+def test_queue_beyond_its_room(cell_factor, dense_min):
+    """Near the percolation density with nearly every top cell dense and (but
+    for the second case) every neighbour in reach: more (fine cell, dense top
+    cell) pairs than the queue holds; those beyond are read cell by cell."""
+    import torch
+    rng = np.random.default_rng(71)
+    n, l = 40000, 1.0
+    L = (n / 0.6) ** (1 / 3)
+    pos = (rng.random((n, 3)) * L).astype(np.float32)
+    w = synth.Workload(name="uniform", pos=pos, vel=np.zeros_like(pos),
+                       ids=np.arange(n, dtype=np.uint64), lo=(0.0,) * 3, hi=(L,) * 3,
+                       linklength=l, boundary=2.0, nphalomin=5, periodic=False,
+                       cells=int(L / 2))
+    ref = cpu.run(w)
+    plan = Plan(FofConfig.from_workload(w, cell_factor=cell_factor))
+    plan.set_tuning({"cell_scale": 1.0, "dense_min": dense_min})
+    dpos, dvel = torch.from_numpy(w.pos).cuda(), torch.from_numpy(w.vel).cuda()
+    for _ in range(2):
+        cat = plan.run(dpos, dvel, members=True)
+        assert_same_catalog(cat, ref)
+    if cell_factor != 8:
+        assert cat.stats["n_queued"] > cat.stats["n_proc"]
+    plan.close()
