@@ -651,13 +651,15 @@ __device__ __forceinline__ uint32_t runs_before(const uint64_t *state, uint32_t 
 // runs moved 40 bytes more per particle: 0.60 ms on the 256^3 box, this 0.37;
 // 512^3 box 5.9 and 2.9 ms.
 //
-// A warp has 128 consecutive elements, 32 at a time; lane l compares with lane
+// A warp has 32 PER consecutive elements, 32 at a time; lane l compares with lane
 // l - 1's cell, lane 0 with the last of the 32 before (before the first 32 it
 // recomputes its predecessor's).
-constexpr int kRunPer = 4;
-constexpr int kRunTile = kT * kRunPer;
+// PER is 8 in large runs, where a tile's barriers and its wait for the lower
+// tiles weigh more than the tiles' number (512^3 box 3.33 ms with 4, 3.09 with 8,
+// 3.51 with 16), and 4 in small ones (10,007 particles: 16 and 18 us).
+constexpr int kRunPerSmall = 4, kRunPerLarge = 8;
 
-template <class PT>
+template <class PT, int kRunPer>
 __global__ void __launch_bounds__(kT) k_gather_runs(
     const uint32_t *__restrict__ order, const PRec<PT> *__restrict__ recs,
     const BoxDev *__restrict__ boxes, int nbox, SPos<PT> *__restrict__ spos,
@@ -665,6 +667,7 @@ __global__ void __launch_bounds__(kT) k_gather_runs(
     uint64_t *__restrict__ run_g, uint16_t *__restrict__ run_box, uint32_t *__restrict__ parent,
     uint32_t *__restrict__ top_range, uint64_t *state, DevScal *sc, uint32_t polls) {
   if (sc->failed) return;  // a sort of this run gave up: its order is not valid
+  constexpr int kRunTile = kT * kRunPer;
   __shared__ uint64_t s_base[kMaxBoxes];
   __shared__ uint32_t s_tile, s_warp[kT / 32], s_before;
   if (threadIdx.x == 0) s_tile = atomicAdd(&sc->next_tile, 1u);
@@ -2626,11 +2629,15 @@ void Plan::issue(int want_member, cudaStream_t s, bool timed) {
   mark(1);
   // ---- runs, top-cell ranges, dense top cells ----
   CMH_CUDA(cudaStreamWaitEvent(s, ev_cleared, 0));  // the later stages' tables
-  k_gather_runs<PT><<<(unsigned)run_tiles, kT, 0, s>>>(
-      order, b_recs.as<PRec<PT>>(), boxes, nbox, b_spos.as<SPos<PT>>(), perm, run_of, run_start,
-      run_g, b_run_box.as<uint16_t>(), parent, b_top_range.as<uint32_t>(),
-      b_run_state.as<uint64_t>(), sc, spin_cap);
-  CMH_LAUNCHED();
+  auto gather = [&](auto per) {
+    k_gather_runs<PT, decltype(per)::value><<<(unsigned)run_tiles, kT, 0, s>>>(
+        order, b_recs.as<PRec<PT>>(), boxes, nbox, b_spos.as<SPos<PT>>(), perm, run_of, run_start,
+        run_g, b_run_box.as<uint16_t>(), parent, b_top_range.as<uint32_t>(),
+        b_run_state.as<uint64_t>(), sc, spin_cap);
+    CMH_LAUNCHED();
+  };
+  if (run_per == kRunPerLarge) gather(std::integral_constant<int, kRunPerLarge>{});
+  else gather(std::integral_constant<int, kRunPerSmall>{});
   if (varlink) {
     if (fp32)
       k_varlink_recs<PT, true><<<rg(k_varlink_recs<PT, true>, npc), kT, 0, s>>>(b_spos.as<SPos<PT>>(), run_of,
@@ -2891,7 +2898,8 @@ void Plan::prepare(const std::vector<BoxSpec> &specs, int want_member) {
   need(b_keys, npc * 8);
   need(b_keys_alt, npc * 8 + 8);  // (also run_of and run_start)
   need(b_parent, npc * 4);
-  run_tiles = (npc + kRunTile - 1) / kRunTile;
+  run_per = npc >= (int64_t)kSMs * 4 * kT * kRunPerLarge ? kRunPerLarge : kRunPerSmall;
+  run_tiles = (npc + kT * run_per - 1) / (kT * run_per);
   need(b_run_state, (size_t)run_tiles * 8);
   need(b_vals, npc * 4);
   need(b_vals_alt, npc * 4);

@@ -63,6 +63,7 @@ struct Plan : public cmh_plan {
   bool cell_states_apart = false;  // each pass of the cell sort has its own tile states
   size_t cell_state_bytes = 0;
   int64_t run_tiles = 0;           // tiles of the gather
+  int run_per = 4;                 // its elements per thread
   uint64_t n_top = 0, k3all = 1;
   int key_bits = 0, hs = 7, props = 0;
   bool varlink = false;             // some box has a variable linking length
