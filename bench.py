@@ -131,15 +131,16 @@ def describe(args, w, dtype, n):
 
 # DRAM bytes per processed particle of the befriending launches (ncu
 # dram__bytes_read.sum + dram__bytes_write.sum of the stage's six launches,
-# 256^3 box at scale 1/2: 431.9 MB for 8,971,801 processed particles)
-BEFRIEND_DRAM_PER_PROC = 431.88e6 / 8971801
+# 256^3 box at scale 1/2: 398.5 MB for 8,971,801 processed particles)
+BEFRIEND_DRAM_PER_PROC = 398.53e6 / 8971801
 
 # the launches behind each stage's CUDA-event interval
 KERNELS = {
-    "befriend": "befriending stage: k_befriend_dense + k_befriend_simple + 2 x k_befriend "
-                "(near, far) + 2 x k_compress",
-    "sort": "radix sort: k_rs_upfront + one k_rs_scatter per digit pass (4 for 34-bit keys)",
-    "ingest": "k_ingest_count + 2 scans + k_ingest_emit",
+    "befriend": "befriending stage: k_befriend_dense + k_befriend_sparse + 2 x "
+                "k_befriend_cross (near, far) + 2 x k_compress",
+    "sort": "radix sort: k_rs_offsets + one k_rs_scatter per digit pass (4 for 34-bit keys)",
+    "ingest": "k_ingest_count + k_ingest_scan + k_ingest_emit",
+    "cells": "k_gather_runs + k_dense_pick",
 }
 
 
@@ -149,18 +150,20 @@ def stage_bytes(st, pos_bytes):
     n, npr, R = st["n_in"], st["n_proc"], st["n_cells"]
     bits = st["key_bits"]
     # passes reading 64-bit keys (the last of them writes 32-bit key words),
-    # then 32-bit passes, 9-bit digits where that saves a pass
-    wide = min((bits + 7) // 8, max(1, -(-(bits - 32) // 8)))
+    # then 32-bit passes, 9-bit digits where that saves a pass; the first reads
+    # the keys from the records, the last writes none
+    wide = max(1, min((bits + 7) // 8, -(-(bits - 32) // 8)))
     rest = max(0, bits - 8 * wide)
     passes = wide + min((rest + 7) // 8, (rest + 8) // 9)
-    rec = 16 if pos_bytes == 4 else 32
+    rec = 32 if pos_bytes == 4 else 48   # emitted record: position, source, key, index
+    spos = 16 if pos_bytes == 4 else 32  # position in cell order
     return {
-        "ingest": 2 * 3 * pos_bytes * n + npr * (8 + 4 + rec),
-        "sort": npr * (8 + (wide - 1) * 24 + 20 + (passes - wide) * 16),
-        "cells": npr * (4 + rec + rec + 8 + 4) + R * 12,
-        "befriend": npr * rec + R * (8 + 4 + 4),
+        "ingest": 2 * 3 * pos_bytes * n + npr * rec,
+        "sort": npr * (8 + (wide - 1) * 24 + 8 + (passes - wide) * 16 - 4),
+        "cells": npr * (4 + rec + spos + 4 + 4) + R * (4 + 8 + 2 + 4),
+        "befriend": npr * spos + R * (8 + 4 + 4),
         "groups": npr * (4 + 4 + 4) + R * 12,
-        "sums": npr * (4 + 4 + rec + 12),
+        "sums": npr * (4 + 4 + spos + 12),
     }
 
 
