@@ -130,14 +130,14 @@ def describe(args, w, dtype, n):
 
 
 # DRAM bytes per processed particle of the befriending launches (ncu
-# dram__bytes_read.sum + dram__bytes_write.sum of the stage's six launches,
-# 256^3 box at scale 1/2: 398.5 MB for 8,971,801 processed particles)
-BEFRIEND_DRAM_PER_PROC = 398.53e6 / 8971801
+# dram__bytes_read.sum + dram__bytes_write.sum of the stage's five launches,
+# 256^3 box at scale 1/2: 381.7 MB for 8,971,801 processed particles)
+BEFRIEND_DRAM_PER_PROC = 381.73e6 / 8971801
 
 # the launches behind each stage's CUDA-event interval
 KERNELS = {
     "befriend": "befriending stage: k_befriend_dense + k_befriend_sparse + 2 x "
-                "k_befriend_cross (near, far) + 2 x k_compress",
+                "k_befriend_cross (near, far) + k_compress",
     "sort": "radix sort: k_rs_offsets + one k_rs_scatter per digit pass (4 for 34-bit keys)",
     "ingest": "k_ingest_count + k_ingest_scan + k_ingest_emit",
     "cells": "k_gather_runs + k_dense_pick",
@@ -162,8 +162,8 @@ def stage_bytes(st, pos_bytes):
         "sort": npr * (8 + (wide - 1) * 24 + 8 + (passes - wide) * 16 - 4),
         "cells": npr * (4 + rec + spos + 4 + 4) + R * (4 + 8 + 2 + 4),
         "befriend": npr * spos + R * (8 + 4 + 4),
-        "groups": npr * (4 + 4 + 4) + R * 12,
-        "sums": npr * (4 + 4 + spos + 12),
+        "groups": R * (4 + 4 + 4 + 4) + R * 12,
+        "sums": npr * (4 + 4 + spos + 4 + 12),
     }
 
 
@@ -322,7 +322,7 @@ def run_ours(args):
         # DRAM bytes of the befriending launches per processed particle, from
         # an ncu capture of the 256^3 box at scale 1/2
         traffic = int(BEFRIEND_DRAM_PER_PROC * st["n_proc"])
-        traffic_src = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the stage's six "
+        traffic_src = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the stage's five "
                        "launches on the 256^3 box at scale 1/2, scaled by processed particles")
     roofline = {"bound": "hbm", "kernel": KERNELS.get(dominant, dominant),
                 "achieved": round(ach, 1),

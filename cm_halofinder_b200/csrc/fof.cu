@@ -1846,7 +1846,7 @@ __global__ void __launch_bounds__(kT) k_compress(uint32_t *parent,
 // Lanes of a warp holding the same key in adjacent lanes form a segment; the
 // segment's first lane receives the segment's sum of v (and min of m).
 template <int NV>
-__device__ __forceinline__ bool warp_segments(uint32_t key, double (&v)[NV]) {
+__device__ __forceinline__ bool warp_segments(uint32_t key, double (&v)[NV], uint32_t &m) {
   const int lane = threadIdx.x & 31;
   const uint32_t prev = __shfl_up_sync(0xffffffffu, key, 1);
   const bool head = lane == 0 || prev != key;
@@ -1861,12 +1861,13 @@ __device__ __forceinline__ bool warp_segments(uint32_t key, double (&v)[NV]) {
       const double t = __shfl_down_sync(0xffffffffu, v[c], d);
       if (take) v[c] += t;
     }
+    const uint32_t om = __shfl_down_sync(0xffffffffu, m, d);
+    if (take) m = min(m, om);
   }
   return head;
 }
 
-__device__ __forceinline__ bool warp_segments_count_min(uint32_t key, uint32_t &cnt,
-                                                        uint32_t &mn) {
+__device__ __forceinline__ bool warp_segments_count(uint32_t key, uint32_t &cnt) {
   const int lane = threadIdx.x & 31;
   const uint32_t prev = __shfl_up_sync(0xffffffffu, key, 1);
   const bool head = lane == 0 || prev != key;
@@ -1876,35 +1877,35 @@ __device__ __forceinline__ bool warp_segments_count_min(uint32_t key, uint32_t &
   for (int d = 1; d < 32; d <<= 1) {
     const uint32_t oseg = __shfl_down_sync(0xffffffffu, seg, d);
     const uint32_t oc = __shfl_down_sync(0xffffffffu, cnt, d);
-    const uint32_t om = __shfl_down_sync(0xffffffffu, mn, d);
-    if ((lane + d < 32) && oseg == seg) {
-      cnt += oc;
-      mn = min(mn, om);
-    }
+    if ((lane + d < 32) && oseg == seg) cnt += oc;
   }
   return head;
 }
 
-// Group size and head (lowest processing index) per root cell.
-__global__ void __launch_bounds__(kT) k_group_count(const uint32_t *__restrict__ run_of,
-                                                    const uint32_t *__restrict__ parent,
-                                                    const uint32_t *__restrict__ perm,
-                                                    const DevScal *__restrict__ sc,
-                                                    uint32_t *__restrict__ count,
-                                                    uint32_t *__restrict__ head) {
+// After the last union: each cell's root as its parent, and the roots' group
+// sizes, a cell's run of particles at a time: half the elements of a count by
+// particle and none of its look-ups.  The groups' heads are found for the
+// candidates alone, by k_group_sums, not with an atomic per group here.  Bound
+// by the parents' reads and the counts' atomics.  Befriending, groups and sums
+// with a compression, then counts and heads by particle, and so: 256^3 box
+// 1.52 and 1.46 ms, 512^3 box 16.06 and 15.73, 50M lightcone 4.52 and 4.41.
+__global__ void __launch_bounds__(kT) k_compress_count(uint32_t *parent,
+                                                       const uint32_t *__restrict__ run_start,
+                                                       const DevScal *__restrict__ sc,
+                                                       uint32_t *__restrict__ count) {
   if (sc->failed) return;  // a sort of this run gave up: its order is not valid
-  const int64_t np = sc->np;
-  const int64_t n_iter = (np + 31) / 32 * 32;
-  for (int64_t i = gtid(); i < n_iter; i += gstride()) {
-    const bool valid = i < np;
-    const uint32_t root = valid ? parent[run_of[i]] : kNone;
-    uint32_t c = valid ? 1u : 0u;
-    uint32_t m = valid ? perm[i] : kNone;
-    const bool h = warp_segments_count_min(root, c, m);
-    if (valid && h) {
-      atomicAdd(count + root, c);
-      atomicMin(head + root, m);
+  const int64_t R = sc->R;
+  const int64_t n_iter = (R + 31) / 32 * 32;
+  for (int64_t r = gtid(); r < n_iter; r += gstride()) {
+    const bool valid = r < R;
+    uint32_t root = kNone, c = 0;
+    if (valid) {
+      root = uf_find(parent, (uint32_t)r);
+      parent[r] = root;
+      c = run_start[r + 1] - run_start[r];
     }
+    const bool h = warp_segments_count(root, c);
+    if (valid && h) atomicAdd(count + root, c);
   }
 }
 
@@ -1990,19 +1991,20 @@ __global__ void __launch_bounds__(kT) k_cand_pick(const uint32_t *__restrict__ p
 
 // Property sums per candidate halo, in double as Output_Halos does
 // (FOF.c:806-832): 6 first moments, then 6 position and 6 velocity second
-// moments when INERTIA / DISPERSION are asked for.
+// moments when INERTIA / DISPERSION are asked for; and its head, the lowest
+// processing index of its particles.
 template <class PT, int NS>
 __global__ void __launch_bounds__(kT) k_group_sums(
     const uint32_t *__restrict__ run_of, const uint32_t *__restrict__ parent,
     const uint32_t *__restrict__ cand_of_root, const uint16_t *__restrict__ run_box,
     const BoxDev *__restrict__ boxes, const SPos<PT> *__restrict__ spos,
-    const DevScal *__restrict__ sc, int props, double *__restrict__ sums,
-    uint32_t *__restrict__ warn) {
+    const uint32_t *__restrict__ perm, const DevScal *__restrict__ sc, int props,
+    double *__restrict__ sums, uint32_t *__restrict__ head, uint32_t *__restrict__ warn) {
   if (sc->failed) return;  // a sort of this run gave up: its order is not valid
   const int64_t np = sc->np;
   const int64_t n_iter = (np + 31) / 32 * 32;
   for (int64_t i = gtid(); i < n_iter; i += gstride()) {
-    uint32_t ci = kNone;
+    uint32_t ci = kNone, m = kNone;
     double v[NS];
 #pragma unroll
     for (int c = 0; c < NS; c++) v[c] = 0.0;
@@ -2013,6 +2015,7 @@ __global__ void __launch_bounds__(kT) k_group_sums(
         const BoxDev &bx = boxes[run_box[run]];
         const Geom &g = bx.g;
         const SPos<PT> p = spos[i];
+        m = perm[i];
         const double x = (double)p.x, y = (double)p.y, z = (double)p.z;
         const uint64_t li = 3 * ((uint64_t)p.src - bx.in_base);
         double vx, vy, vz;
@@ -2050,8 +2053,9 @@ __global__ void __launch_bounds__(kT) k_group_sums(
     // 64 boxes 0.87 -> 0.76; two or four particles per step, their gathers in flight
     // together, were 10 and 20 % slower: fewer warps)
     if (!__any_sync(0xffffffffu, ci != kNone)) continue;
-    const bool h = warp_segments<NS>(ci, v);
+    const bool h = warp_segments<NS>(ci, v, m);
     if (h && ci != kNone) {
+      atomicMin(head + ci, m);
       double *s = sums + (uint64_t)ci * NS;
 #pragma unroll
       for (int c = 0; c < NS; c++) atomicAdd(s + c, v[c]);
@@ -2101,7 +2105,7 @@ __global__ void __launch_bounds__(kT) k_own_pick(const double *__restrict__ sums
         const double com = __ddiv_rn(sums[(uint64_t)c * NS + a], n);
         ok &= (com >= g.lo[a]) && (com < g.hi[a]);
       }
-      hd = head[root];
+      hd = head[c];
       ok &= hd < np_cap;
     }
     const uint32_t o = warp_slot(ok, &sc->nh);
@@ -2569,7 +2573,7 @@ void Plan::issue(int want_member, cudaStream_t s, bool timed) {
     f.add(b_warn, (size_t)ncc * 4, 0u);
     f.add(b_cat_of_cand, (size_t)ncc * 4, 0xffffffffu);
     f.add(b_count, npc * 4, 0u);
-    f.add(b_head, npc * 4, 0xffffffffu);
+    f.add(b_head, (size_t)ncc * 4, 0xffffffffu);
     f.add(b_marks, (size_t)((npc + kHeadGroup - 1) / kHeadGroup) * (kHeadGroup / 8), 0u);
     f.add(b_run_state, (size_t)run_tiles * 8, 0u);
     if (cell_states_apart) f.add(sort_tmp, cell_state_bytes, 0u);
@@ -2699,13 +2703,11 @@ void Plan::issue(int want_member, cudaStream_t s, bool timed) {
   else if (fp32) befriend(std::true_type{}, std::false_type{});
   else if (varlink) befriend(std::false_type{}, std::true_type{});
   else befriend(std::false_type{}, std::false_type{});
-  k_compress<<<rg(k_compress, npc), kT, 0, s>>>(parent, sc);
-  CMH_LAUNCHED();
   mark(3);
 
   // ---- groups, candidates ----
-  k_group_count<<<rg(k_group_count, npc), kT, 0, s>>>(run_of, parent, perm, sc, b_count.as<uint32_t>(),
-                                  b_head.as<uint32_t>());
+  k_compress_count<<<rg(k_compress_count, npc), kT, 0, s>>>(parent, run_start, sc,
+                                                            b_count.as<uint32_t>());
   CMH_LAUNCHED();
   if (sampling && n > 0) {
     CMH_CUDA(cudaMemsetAsync(b_samp.p, 0, (size_t)n, s));
@@ -2732,8 +2734,9 @@ void Plan::issue(int want_member, cudaStream_t s, bool timed) {
   k_group_sums<PT, NSV><<<rg(k_group_sums<PT, NSV>, npc), kT, 0, s>>>(run_of, parent,  \
                                           b_cand_of_root.as<uint32_t>(),                      \
                                           b_run_box.as<uint16_t>(), boxes,                    \
-                                          b_spos.as<SPos<PT>>(), sc, props,                   \
-                                          b_sums.as<double>(), b_warn.as<uint32_t>())
+                                          b_spos.as<SPos<PT>>(), perm, sc, props,             \
+                                          b_sums.as<double>(), b_head.as<uint32_t>(),         \
+                                          b_warn.as<uint32_t>())
   if (NS == 6) CMH_SUMS(6);
   else if (NS == 12) CMH_SUMS(12);
   else CMH_SUMS(18);
@@ -2915,7 +2918,7 @@ void Plan::prepare(const std::vector<BoxSpec> &specs, int want_member) {
   need(b_dense_range, (size_t)nd_cap * sizeof(uint2));
   need(b_dense_big, (size_t)nd_cap * sizeof(uint32_t));
   need(b_count, npc * 4);
-  need(b_head, npc * 4);
+  need(b_head, ncc * 4);
   need(b_cand_of_root, npc * 4);
   if (sampling) need(b_samp, (size_t)nn);
   need(b_cand_root, ncc * 4);

@@ -58,3 +58,22 @@ def test_large_membership_outlives_its_catalog():
     gc.collect()
     np.testing.assert_array_equal(member, ref["member"])
     np.testing.assert_array_equal(tail, ref["member"][-1000:])
+
+
+@pytest.mark.parametrize("cells", [1, 31, 32, 33, 65])
+def test_sizes_and_heads_by_cells(cells):
+    """Group sizes are counted a fine cell at a time and heads found for the
+    candidates alone: a chain of cells of one to three particles each and lone
+    particles, every group a candidate (1 member), in shuffled input order."""
+    rng = np.random.default_rng(cells)
+    chain = np.repeat(np.arange(cells), 1 + np.arange(cells) % 3)
+    pts = np.full((len(chain), 3), 5.0)
+    pts[:, 0] = 2.0 + 0.045 * chain
+    lone = np.stack([1.0 + 0.2 * np.arange(cells // 2), *np.full((2, cells // 2), 8.0)], 1)
+    pos = rng.permutation(np.concatenate([pts, lone])).astype(np.float32)
+    w = synth.Workload(name="chain", pos=pos, vel=rng.normal(0, 300, pos.shape).astype(np.float32),
+                       ids=np.arange(len(pos), dtype=np.uint64), lo=(0.0,) * 3, hi=(10.0,) * 3,
+                       linklength=0.05, boundary=1.0, nphalomin=1, periodic=False, cells=100)
+    cat = fof(w.pos, w.vel, FofConfig.from_workload(w), members=True)
+    assert cat.nhalos == 1 + cells // 2
+    assert_same_catalog(cat, cpu.run(w))
