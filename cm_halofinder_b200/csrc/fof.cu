@@ -2294,23 +2294,24 @@ int bits_for(uint64_t v) {
 // ---------------------------------------------------------------------------
 
 namespace {
-// Values of the position type in order as integers, and back.
-int64_t ordinal(float x) {
-  int32_t i;
+// Values of the position type in order as unsigned integers, and back.  (The
+// ordinals of two doubles may be more than 2^63 apart.)
+uint64_t ordinal(float x) {
+  uint32_t i;
   memcpy(&i, &x, 4);
-  return i >= 0 ? (int64_t)i : -(int64_t)(i & 0x7fffffff);
+  return i >> 31 ? ~i : i | 0x80000000u;
 }
-int64_t ordinal(double x) {
-  int64_t i;
+uint64_t ordinal(double x) {
+  uint64_t i;
   memcpy(&i, &x, 8);
-  return i >= 0 ? i : -(i & 0x7fffffffffffffffll);
+  return i >> 63 ? ~i : i | 0x8000000000000000ull;
 }
-void from_ordinal(int64_t o, float *x) {
-  const int32_t i = o >= 0 ? (int32_t)o : (int32_t)((uint32_t)(-o) | 0x80000000u);
+void from_ordinal(uint64_t o, float *x) {
+  const uint32_t i = o >> 31 ? (uint32_t)o & 0x7fffffffu : ~(uint32_t)o;
   memcpy(x, &i, 4);
 }
-void from_ordinal(int64_t o, double *x) {
-  const uint64_t i = o >= 0 ? (uint64_t)o : (uint64_t)(-o) | 0x8000000000000000ull;
+void from_ordinal(uint64_t o, double *x) {
+  const uint64_t i = o >> 63 ? o & 0x7fffffffffffffffull : ~o;
   memcpy(x, &i, 8);
 }
 
@@ -2323,9 +2324,9 @@ template <class PT, class F> PT edge_value(double guess, double slack, int dir, 
   if (!ok(in)) in = dir * std::numeric_limits<PT>::max();
   if (!ok(in)) return dir * inf;
   if (ok(out)) out = -dir * inf;  // (no coordinate: ok() is not asked about it)
-  int64_t a = ordinal(in), b = ordinal(out);
+  uint64_t a = ordinal(in), b = ordinal(out);
   while ((a > b ? a - b : b - a) > 1) {
-    const int64_t m = b + (a - b) / 2;
+    const uint64_t m = a > b ? b + (a - b) / 2 : a + (b - a) / 2;
     PT x;
     from_ordinal(m, &x);
     if (ok(x)) a = m;
