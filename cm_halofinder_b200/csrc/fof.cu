@@ -1884,7 +1884,11 @@ __device__ __forceinline__ bool warp_segments_count(uint32_t key, uint32_t &cnt)
 
 // After the last union: each cell's root as its parent, and the roots' group
 // sizes, a cell's run of particles at a time: half the elements of a count by
-// particle and none of its look-ups.  The groups' heads are found for the
+// particle and none of its look-ups.  The walk to the root only reads, so that a
+// cell's parent is written by its own thread alone: the kernels that follow take
+// it as the root without a find, and a halving find's late store of an ancestor
+// over the root would take the cell out of its group's sums and membership.
+// The groups' heads are found for the
 // candidates alone, by k_group_sums, not with an atomic per group here.  Bound
 // by the parents' reads and the counts' atomics.  Befriending, groups and sums
 // with a compression, then counts and heads by particle, and so: 256^3 box
@@ -1900,7 +1904,7 @@ __global__ void __launch_bounds__(kT) k_compress_count(uint32_t *parent,
     const bool valid = r < R;
     uint32_t root = kNone, c = 0;
     if (valid) {
-      root = uf_find(parent, (uint32_t)r);
+      root = uf_root(parent, (uint32_t)r);
       parent[r] = root;
       c = run_start[r + 1] - run_start[r];
     }

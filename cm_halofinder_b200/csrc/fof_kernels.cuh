@@ -260,6 +260,15 @@ __device__ __forceinline__ uint32_t uf_find(uint32_t *parent, uint32_t x) {
   }
 }
 
+// find() without the halving: it only reads.
+__device__ __forceinline__ uint32_t uf_root(const uint32_t *parent, uint32_t x) {
+  while (true) {
+    const uint32_t p = __ldcg(parent + x);
+    if (p == x) return x;
+    x = p;
+  }
+}
+
 // find() that also counts its parent loads
 __device__ __forceinline__ uint32_t uf_find_n(uint32_t *parent, uint32_t x, uint32_t &steps) {
   while (true) {
