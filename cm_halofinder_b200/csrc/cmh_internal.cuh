@@ -37,7 +37,7 @@ extern thread_local long long g_launches;
 // comma-separated words of the CMH_FAULT environment variable (alloc: device
 // allocations fail; io: opening a file fails; overflow: every run overflows
 // its capacity; lookback: one tile of the cell sort publishes nothing, so a
-// capped device wait runs out).  Read on every call, in host code only.
+// capped device wait runs out; gather: the same of the run count).  Read on every call, in host code only.
 bool fault_active(const char *kind);
 
 // Grid size for a grid-stride kernel: a multiple of the SM count, capped by
@@ -74,11 +74,11 @@ struct DevBuf {
 };
 
 // ---- radix_sort.cu -----------------------------------------------------------
-// Bounds of the sorts' look-back waits: a tile polls a lower tile's state at
-// most spin_cap times, then gives up (the sort's giveups counter is raised;
-// its output is then not an ordering).  stall_tile (a test hook) names a tile
-// of the first pass that publishes nothing, so that its successor's wait
-// runs out.
+// Bounds of the look-back waits (the sort's and the run count's): a tile polls
+// a lower tile's state at most spin_cap times, then gives up (the run's giveups
+// counter is raised; a sort's output is then not an ordering).  stall_tile (a
+// test hook) names a tile (of a sort's first pass) that publishes nothing, so
+// that its successor's wait runs out.
 constexpr uint32_t kSpinCap = 1u << 22;
 struct SortWaits {
   uint32_t spin_cap = kSpinCap;

@@ -611,7 +611,7 @@ constexpr uint64_t kTileAll = 2ull << 32;   // the runs up to and with this tile
 // Runs before `tile`: one warp adds up the lower tiles' published states, 32 at
 // a time, back to the first inclusive one.  Every lower tile publishes its own
 // count before it waits, so every wait ends; a wait is capped all the same
-// (`polls` reads) and then raises *failed.
+// (`polls` reads) and then raises *failed and gives kNone.
 __device__ __forceinline__ uint32_t runs_before(const uint64_t *state, uint32_t tile,
                                                 uint32_t polls, unsigned int *failed) {
   const uint32_t lane = threadIdx.x & 31;
@@ -628,7 +628,7 @@ __device__ __forceinline__ uint32_t runs_before(const uint64_t *state, uint32_t 
     if (none & need) {
       if (left-- == 0) {
         if (lane == 0) atomicAdd(failed, 1u);
-        return sum;
+        return kNone;
       }
       continue;
     }
@@ -647,9 +647,11 @@ __device__ __forceinline__ uint32_t runs_before(const uint64_t *state, uint32_t 
 // occupied top cell (top_range starts zeroed; where the top cell changes
 // between two particles, the new one's first run is the old one's end).  A tile
 // counts its run starts, publishes the count and learns the lower tiles' by
-// look-back.  A gather, a three-kernel scan of start flags and a kernel for the
-// runs moved 40 bytes more per particle: 0.60 ms on the 256^3 box, this 0.37;
-// 512^3 box 5.9 and 2.9 ms.
+// look-back; one that gives up writes no runs.  The failed flag may be raised
+// while this kernel runs, so one thread reads it for its whole CTA, before it
+// takes a tile (the tiles taken are all worked on).  A gather, a three-kernel
+// scan of start flags and a kernel for the runs moved 40 bytes more per particle:
+// 0.60 ms on the 256^3 box, this 0.37; 512^3 box 5.9 and 2.9 ms.
 //
 // A warp has 32 PER consecutive elements, 32 at a time; lane l compares with lane
 // l - 1's cell, lane 0 with the last of the 32 before (before the first 32 it
@@ -665,16 +667,16 @@ __global__ void __launch_bounds__(kT) k_gather_runs(
     const BoxDev *__restrict__ boxes, int nbox, SPos<PT> *__restrict__ spos,
     uint32_t *__restrict__ perm, uint32_t *__restrict__ run_of, uint32_t *__restrict__ run_start,
     uint64_t *__restrict__ run_g, uint16_t *__restrict__ run_box, uint32_t *__restrict__ parent,
-    uint32_t *__restrict__ top_range, uint64_t *state, DevScal *sc, uint32_t polls) {
-  if (sc->failed) return;  // a sort of this run gave up: its order is not valid
+    uint32_t *__restrict__ top_range, uint64_t *state, DevScal *sc, SortWaits waits) {
   constexpr int kRunTile = kT * kRunPer;
   __shared__ uint64_t s_base[kMaxBoxes];
   __shared__ uint32_t s_tile, s_warp[kT / 32], s_before;
-  if (threadIdx.x == 0) s_tile = atomicAdd(&sc->next_tile, 1u);
+  if (threadIdx.x == 0)  // (after a sort that gave up the order is not valid)
+    s_tile = __ldcg(&sc->failed) ? kNone : atomicAdd(&sc->next_tile, 1u);
   load_bases(boxes, nbox, s_base, false);
   const uint32_t tile = s_tile;
   const int64_t np = sc->np;
-  if ((int64_t)tile * kRunTile >= np) return;  // the whole CTA leaves together
+  if (tile == kNone || (int64_t)tile * kRunTile >= np) return;  // the whole CTA leaves together
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t i0 = (int64_t)tile * kRunTile + w * (32 * kRunPer) + lane;
   uint32_t from[kRunPer], before = 0;
@@ -728,14 +730,17 @@ __global__ void __launch_bounds__(kT) k_gather_runs(
   }
   if (w == 0) {
     unsigned long long *own = reinterpret_cast<unsigned long long *>(state + tile);
-    if (lane == 0 && tile != 0) atomicExch(own, (unsigned long long)(kTileOwn | in_tile));
-    const uint32_t b = runs_before(state, tile, polls, &sc->failed);
-    if (lane == 0) {
-      atomicExch(own, (unsigned long long)(kTileAll | (b + in_tile)));
-      s_before = b;
-    }
+    // (a tile named by waits.stall_tile publishes nothing: a test hook whose
+    // successor's capped wait then runs out)
+    const bool publish = lane == 0 && tile != waits.stall_tile;
+    if (publish && tile != 0) atomicExch(own, (unsigned long long)(kTileOwn | in_tile));
+    const uint32_t b = runs_before(state, tile, waits.spin_cap, &sc->failed);
+    // (after a give-up any count in range will do: the next tiles' waits end)
+    if (publish) atomicExch(own, (unsigned long long)(kTileAll | ((b == kNone ? 0u : b) + in_tile)));
+    if (lane == 0) s_before = b;
   }
   __syncthreads();
+  if (s_before == kNone) return;
   uint32_t done = s_before + wbefore;  // runs that start before these 32
 #pragma unroll
   for (int j = 0; j < kRunPer; j++) {
@@ -2642,7 +2647,7 @@ void Plan::issue(int want_member, cudaStream_t s, bool timed) {
     k_gather_runs<PT, decltype(per)::value><<<(unsigned)run_tiles, kT, 0, s>>>(
         order, b_recs.as<PRec<PT>>(), boxes, nbox, b_spos.as<SPos<PT>>(), perm, run_of, run_start,
         run_g, b_run_box.as<uint16_t>(), parent, b_top_range.as<uint32_t>(),
-        b_run_state.as<uint64_t>(), sc, spin_cap);
+        b_run_state.as<uint64_t>(), sc, SortWaits{spin_cap, stall_gather ? 1u : 0xffffffffu});
     CMH_LAUNCHED();
   };
   if (run_per == kRunPerLarge) gather(std::integral_constant<int, kRunPerLarge>{});
@@ -3007,7 +3012,9 @@ void Plan::read_back(cudaStream_t s, bool timed) {
   if (hc.c.uf_giveups)
     fail(CMH_ERR_DEVICE_TIMEOUT, "union-find retry loop reached its iteration cap");
   if (hs_.failed)
-    fail(CMH_ERR_DEVICE_TIMEOUT, "radix sort look-back wait reached its cap");
+    fail(CMH_ERR_DEVICE_TIMEOUT, hs_.next_tile == 0  // (the gather takes no tile then)
+                                     ? "radix sort look-back wait reached its cap"
+                                     : "run count look-back wait reached its cap");
   stats = cmh_stats{};
   stats.n_in = n_total;
   stats.n_out = n_total - hs_.kept_total;
@@ -3056,11 +3063,13 @@ void Plan::run_batch(const std::vector<BoxSpec> &specs, int want_member, cudaStr
     memcpy(&samp_bits[1], &samp_out, 8);
     samp_bits[2] = (int64_t)samp_seed ^ ((int64_t)samp_closed << 40);
     stall_sort = fault_active("lookback");
+    stall_gather = fault_active("gather");
     const int64_t caps[12] = {np_cap, nd_cap, nc_cap, (int64_t)want_member, (int64_t)fp32,
                               (int64_t)dense_min, (int64_t)vel_wait,
                               sampling ? samp_bits[0] : -1, samp_bits[1],
                               samp_bits[2] ^ (int64_t)(uintptr_t)samp_ids,
-                              (int64_t)spin_cap, (int64_t)stall_sort};
+                              (int64_t)spin_cap,
+                              (int64_t)stall_sort | (int64_t)stall_gather << 1};
     sig.insert(sig.end(), (const unsigned char *)caps, (const unsigned char *)caps + sizeof caps);
     // and the workspace addresses the recorded launches use
     each_buf([&](DevBuf &b) {

@@ -43,8 +43,9 @@ struct Plan : public cmh_plan {
   double cell_scale = 0.0;  // tuned scale of the cell-size factor (0: by rule)
   // bounds of the device loops that retry or wait (cmh_plan_set_limits)
   uint32_t union_cap = kUnionCap;  // retries of one union after a lost race
-  uint32_t spin_cap = kSpinCap;    // polls of one sort tile state
+  uint32_t spin_cap = kSpinCap;    // polls of one tile state (sort, run count)
   bool stall_sort = false;         // CMH_FAULT=lookback for this run
+  bool stall_gather = false;       // CMH_FAULT=gather for this run
 
   // shape of the current run
   std::vector<BoxDev> boxes_host;

@@ -162,7 +162,8 @@ size_t cmh_last_error(char *buf, size_t len);
  *              (CMH_ERR_CAPACITY), as a rank's receive-buffer overflow stops
  *              the reference (read_data.c:551-556)
  *   lookback : one tile of the cell sort publishes nothing, so that the next
- *              tile's wait runs into its bound (CMH_ERR_DEVICE_TIMEOUT)   */
+ *              tile's wait runs into its bound (CMH_ERR_DEVICE_TIMEOUT)
+ *   gather   : the same of the run count after the sort                    */
 
 /* ---- one-shot run: replaces void FOF(void) (src_v2/FOF.c:23, vars.h:121) - */
 
