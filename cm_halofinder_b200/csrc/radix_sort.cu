@@ -82,7 +82,9 @@ __global__ void __launch_bounds__(kMaxBins) k_rs_offsets(const uint32_t *__restr
 // inclusive states end the walk) and writes each digit's run contiguously to
 // goff[digit] + (keys of the digit in lower tiles).  A tile publishes its own
 // counts before it waits on anything, so every wait ends; a wait is still
-// capped, and a capped one sets *giveups.
+// capped, and a capped one sets *giveups.  The output then has holes of stale
+// keys that the digit counts do not know, which a later pass would place past the
+// arrays' ends: a CTA that finds *giveups set when it starts moves nothing.
 constexpr int kSThreads = 512;
 constexpr int kSWarps = kSThreads / 32;
 constexpr int kSIPT = kTile / kSThreads;  // 8
@@ -100,7 +102,7 @@ struct ScatterSmem {
   uint32_t gofs[BINS];
   uint32_t thist[BINS];
   uint32_t warp_sums[kSWarps];
-  uint32_t tile;
+  uint32_t tile, stop;
 };
 
 // Lanes of the warp with the same NB-bit value d (a digit, or BINS for an
@@ -141,6 +143,7 @@ __global__ void __launch_bounds__(kSThreads, NARROW || sizeof(KO) == 8 ? 3 : 4) 
   Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) sm.tile = atomicAdd(tile_ctr, 1u);
+  if (threadIdx.x == 32) sm.stop = __ldcg(giveups);  // (beside the other's wait)
   for (int i = threadIdx.x; i < kSWarps * BINS / 2; i += kSThreads)
     reinterpret_cast<uint32_t *>(&sm.wcnt[0][0])[i] = 0;
   if (threadIdx.x < BINS) sm.thist[threadIdx.x] = 0;
@@ -148,6 +151,13 @@ __global__ void __launch_bounds__(kSThreads, NARROW || sizeof(KO) == 8 ? 3 : 4) 
   const uint32_t tile = sm.tile;
   const int64_t base = (int64_t)tile * kTile;
   if (base >= n) return;  // the whole CTA leaves together
+  if (sm.stop) {          // so too here, with an end to the higher tiles' waits
+    if (threadIdx.x < BINS)
+      atomicExch(reinterpret_cast<unsigned long long *>(state + (uint64_t)tile * BINS +
+                                                        threadIdx.x),
+                 (unsigned long long)kInclusive);
+    return;
+  }
   const uint32_t lt_mask = (1u << lane) - 1u;
   const int rem = n - base < kTile ? (int)(n - base) : kTile;
   const int mine = warp * 32 * kSIPT + lane;  // the thread's keys: mine + 32 j

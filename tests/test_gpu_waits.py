@@ -15,7 +15,8 @@ TIMEOUT = 7
 
 
 @pytest.mark.parametrize("n", [60_000, 1_400_000])   # tiles of 1024 and of 2048 elements
-@pytest.mark.parametrize("kind,who", [("gather", "run count")])
+@pytest.mark.parametrize("kind,who", [("gather", "run count"), ("lookback", "radix sort"),
+                                      ("lookback,gather", "radix sort")])
 def test_wait_runs_out_then_recovery(n, kind, who, monkeypatch):
     import torch
     w = synth.config2(seed=611, scale=n / 256 ** 3)
@@ -34,6 +35,14 @@ def test_wait_runs_out_then_recovery(n, kind, who, monkeypatch):
                 assert e.value.status == TIMEOUT and f"{who} look-back" in str(e.value)
             monkeypatch.delenv("CMH_FAULT")
             plan.set_limits()
+        # no poll at all: whichever wait comes first, if any
+        plan.set_limits(lookback_polls=0)
+        for _ in range(3):
+            try:
+                assert_same_catalog(plan.run(pos, vel, members=True), ref)
+            except cmh.CmhError as e:
+                assert e.status == TIMEOUT and "look-back" in str(e)
+        plan.set_limits()
         for _ in range(2):
             assert_same_catalog(plan.run(pos, vel, members=True), ref)
     finally:
