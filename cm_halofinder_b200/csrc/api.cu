@@ -72,11 +72,11 @@ int resident_ctas(const void *kernel, int threads, size_t smem) {
 
 void DevBuf::ensure(size_t bytes) {
   if (bytes <= cap && p) return;
-  if (fault_active("alloc"))
-    fail(CMH_ERR_OUT_OF_MEMORY, "device allocation failed (injected: CMH_FAULT=alloc)");
   if (p) CMH_CUDA(cudaFree(p));
   p = nullptr;
   cap = 0;
+  if (fault_active("alloc"))  // (as cudaMalloc would: the old buffer is gone)
+    fail(CMH_ERR_OUT_OF_MEMORY, "device allocation failed (injected: CMH_FAULT=alloc)");
   size_t want = bytes + bytes / 64 + 256;  // headroom against small regrowth
   const cudaError_t e = cudaMalloc(&p, want);
   if (e == cudaErrorMemoryAllocation) {

@@ -2865,6 +2865,7 @@ void Plan::prepare(const std::vector<BoxSpec> &specs, int want_member) {
       ltab_all.insert(ltab_all.end(), specs[b].ltab.begin(), specs[b].ltab.end());
     }
   if (varlink) {
+    if (ltab_all.size() * sizeof(double) > ltab_dev.cap) uploaded_sig.clear();
     ltab_dev.ensure(ltab_all.size() * sizeof(double));
     size_t off = 0;
     for (int b = 0; b < nbox; b++)
@@ -2968,6 +2969,9 @@ void Plan::prepare(const std::vector<BoxSpec> &specs, int want_member) {
   auto room = [](size_t bytes) { return (bytes + 511) & ~(size_t)255; };
   size_t total = 0;
   for (const auto &q : pieces) total += room(q.second);
+  // new memory, which may come to lie at the old address (as after a run that did
+  // not fit), holds no box table
+  if (total > arena.cap) uploaded_sig.clear();
   arena.ensure(total);
   each_buf([](DevBuf &b) {
     if (b.view) b.release();
