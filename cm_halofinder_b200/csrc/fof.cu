@@ -1597,8 +1597,8 @@ __global__ void __launch_bounds__(kT, 4) k_befriend_sparse(
         const bool dense = cnt != 0 && slot != kNone;
         const uint32_t qm = __ballot_sync(0xffffffffu, dense);
         if (qm) {
-          uint32_t at = 0;
-          if (lane == 0) at = atomicAdd(&sc->qcount, (uint32_t)__popc(qm));
+          unsigned long long at = 0;  // (may pass 2^32: no early place is taken twice)
+          if (lane == 0) at = atomicAdd(&sc->qcount, (unsigned long long)__popc(qm));
           at = __shfl_sync(0xffffffffu, at, 0) + __popc(qm & below);
           if (dense && at < q_cap) {  // (past the queue's end the cells are read one by one)
             q_cell[at] = a;
@@ -1703,7 +1703,7 @@ __global__ void __launch_bounds__(kT, 3) k_befriend_cross(
   uint2 *pairs = s_pairs[threadIdx.x >> 5];
   uint4 *rows = s_row[threadIdx.x >> 5];
   const GlobalUF uf{parent};
-  const uint32_t NQ = min(sc->qcount, q_cap);
+  const uint32_t NQ = (uint32_t)min(sc->qcount, (unsigned long long)q_cap);
   if (NQ == 0) return;
   uint32_t *next = PHASE == 0 ? &sc->next0 : &sc->next1;
   const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u;
@@ -3041,7 +3041,7 @@ void Plan::read_back(cudaStream_t s, bool timed) {
   stats.n_scan_iters = (int64_t)hc.c.scan_iters;
   stats.n_window_iters = (int64_t)hc.c.window_iters;
   stats.n_dense_tops = hs_.nd;
-  stats.n_queued = hs_.qcount;
+  stats.n_queued = (int64_t)hs_.qcount;
   stats.n_big_tops = hs_.nbig;
   if (timed) {
     float ms = 0;

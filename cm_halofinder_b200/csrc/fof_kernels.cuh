@@ -94,10 +94,11 @@ struct BoxDev {
 // Device-side sizes of one run: nothing is read back by the host until the
 // run has been issued, so the whole run can be captured in a CUDA graph.
 struct DevScal {
+  unsigned long long qcount;       // queued items found: up to 13 per fine cell
   uint32_t kept_total, img_total;  // totals of the keep / image scans
   uint32_t np_raw, np;             // processed particles (np clamped to the capacity)
   uint32_t R, nd, nc, nh;          // fine cells, dense top cells, candidates, halos
-  uint32_t qcount, next_dense, next0, next1;
+  uint32_t next_dense, next0, next1;
   uint32_t overflow;               // bit 0: processed particles above capacity
   uint32_t nbig, next_big;          // dense top cells handled by a whole CTA
   uint32_t next_simple;             // fine cells taken by the sparse path
