@@ -908,12 +908,30 @@ __device__ __forceinline__ double box_dist2(const Geom &g, double x, double y, d
   return ex * ex + ey * ey + ez * ez;
 }
 
-// Per-thread tallies of the befriending kernels, flushed once per warp.
-// (one thread's share of a run stays far below 2^32)
+// Per-thread tallies of the befriending kernels, flushed once per warp.  They are
+// 32 bits wide (registers): spill() moves them to the counters before they
+// wrap, between the kernels' items, none of which adds 2^31, and between the
+// steps of a search of two crowded cells, which can take any number.
 struct BfStats {
   uint32_t tests = 0, rechecks = 0, cand = 0, skips = 0, unions = 0, steps = 0;
   uint32_t scan = 0, window = 0;
 
+  // (by any lane for itself)
+  __device__ __forceinline__ void spill(Counters *ctr) {
+    if (!((tests | rechecks | cand | skips | unions | steps | scan | window) >> 31)) return;
+    auto move = [](unsigned long long *to, uint32_t &v) {
+      if (v) atomicAdd(to, (unsigned long long)v);
+      v = 0;
+    };
+    move(&ctr->pair_tests, tests);
+    move(&ctr->rechecks, rechecks);
+    move(&ctr->cand_pairs, cand);
+    move(&ctr->root_skips, skips);
+    move(&ctr->unions, unions);
+    move(&ctr->find_steps, steps);
+    move(&ctr->scan_iters, scan);
+    move(&ctr->window_iters, window);
+  }
   __device__ void add(unsigned long long *to, uint32_t v) {
     unsigned long long w = v;
 #pragma unroll
@@ -1110,6 +1128,7 @@ __device__ __forceinline__ bool warp_cells_linked(const PairArgs<PT, FP32> &A, c
         }
         if (__any_sync(0xffffffffu, hit)) return true;
       }
+      st.spill(A.ctr);
       // joined by another warp meanwhile: the answer no longer matters
       if ((step & 7) == 0 && __any_sync(0xffffffffu, uf.find(a, st) == uf.find(b, st)))
         return false;
@@ -1430,6 +1449,7 @@ __global__ void __launch_bounds__(128) k_befriend_dense(
     }
     dense_top<PT, FP32, VL>(A, slot, cta ? smem : own, cta, pairs, k3all, dense_range, grows, kk,
                             rows_stride, parent, st);
+    st.spill(A.ctr);
   }
   st.flush(A.ctr);
 }
@@ -1498,6 +1518,7 @@ __global__ void __launch_bounds__(kT, 4) k_befriend_sparse(
   const uint32_t warps = gridDim.x * (kT / 32);
   const uint32_t step = R >= warps * 256 ? 128u : 32u;
   while (true) {
+    st.spill(A.ctr);
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(&sc->next_simple, step);
     base = __shfl_sync(0xffffffffu, base, 0);
@@ -1718,6 +1739,7 @@ __global__ void __launch_bounds__(kT, 3) k_befriend_cross(
   uint32_t npair = 0, nrow = 0;
   BfStats st;
   while (true) {
+    st.spill(A.ctr);
     uint32_t q0 = 0;
     if (lane == 0) q0 = atomicAdd(next, 32u >> lg);
     q0 = __shfl_sync(0xffffffffu, q0, 0);
