@@ -1615,6 +1615,7 @@ __global__ void __launch_bounds__(kT, 4) k_befriend_sparse(
             cnt = 1;
           }
         }
+        __syncwarp();  // (read before other lanes list items there again)
         const bool dense = cnt != 0 && slot != kNone;
         const uint32_t qm = __ballot_sync(0xffffffffu, dense);
         if (qm) {
@@ -1669,6 +1670,7 @@ __global__ void __launch_bounds__(kT, 4) k_befriend_sparse(
                 apart = rb != ra;
                 if (!apart) st.skips++;
               }
+              __syncwarp();  // (read before other lanes list candidates there again)
               push_pairs<PT, FP32, VL>(A, uf, pairs, npair, apart, c.x, c.y, flush && ncand == 0,
                                        st);
             } while (flush && ncand);
