@@ -2913,9 +2913,10 @@ void Plan::prepare(const std::vector<BoxSpec> &specs, int want_member) {
   // per 650 processed particles, the 256^3 ones one per 1100)
   nd_cap = std::max<int64_t>(nd_cap, std::max(np_cap / 1024 + 1024, np_cap / 256));
   nd_cap = std::min<int64_t>(nd_cap, std::max<int64_t>(1024, rows_cap_for(np_cap, k3all)));
-  double mincut = 1e300;
-  for (const BoxDev &bd : boxes_host) mincut = std::min(mincut, bd.g.nphalomin);
-  const int64_t div = (int64_t)std::max(1.0, std::floor(mincut));
+  double mincut = 1e18;
+  for (const BoxDev &bd : boxes_host)  // (below 1, and NaN: every group is a candidate)
+    mincut = std::min(mincut, bd.g.nphalomin >= 1.0 ? bd.g.nphalomin : 1.0);
+  const int64_t div = (int64_t)std::floor(mincut);
   nc_cap = std::max<int64_t>(1, np_cap / div + 1);
 
   const int64_t nn = std::max<int64_t>(n_total, 1), npc = np_cap, ncc = nc_cap;
