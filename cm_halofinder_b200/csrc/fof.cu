@@ -96,6 +96,7 @@ struct Fills {
   int count = 0;
   void add(const DevBuf &b, size_t bytes, uint32_t w) {
     if (bytes == 0) return;
+    if (count == kMax) fail(CMH_ERR_CAPACITY, "too many tables to fill");  // (14 at most)
     p[count] = b.as<uint4>();
     n[count] = (bytes + 15) / 16;
     word[count++] = w;
