@@ -3009,8 +3009,8 @@ void Plan::prepare(const std::vector<BoxSpec> &specs, int want_member) {
   }
 }
 
-// Host memory for `bytes` read back from the device: pinned from the plan's
-// second run on, else `unpinned`.
+// Host memory for `bytes` read back from the device: pinned once the plan's first
+// run has ended, else `unpinned`.
 unsigned char *Plan::host_room(size_t bytes, std::vector<unsigned char> &unpinned) {
   if (runs > 0) pinned.ensure(bytes);
   if (pinned.p && pinned.cap >= bytes) return static_cast<unsigned char *>(pinned.p);

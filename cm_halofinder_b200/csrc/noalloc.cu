@@ -230,8 +230,10 @@ __device__ __forceinline__ FineCell na_fine(const FineGrid &g, const PT *pos, ui
   return f;
 }
 
-// Multiplicative hash of a cell's coordinates (odd constants; the high bits
-// of the product are the best mixed).
+// Multiplicative hash of a cell's coordinates (the high bits of the product are
+// the best mixed).  The odd constants are published ones: 2^64 over the golden
+// ratio (Fibonacci hashing, Knuth, The Art of Computer Programming 3, 6.4) and two
+// of the 64-bit primes of xxHash (Collet).
 __device__ __forceinline__ uint32_t na_hash(const FineCell &f) {
   uint64_t x = (uint64_t)f.c[0] * 0x9E3779B97F4A7C15ull;
   x = (x ^ (x >> 32)) + (uint64_t)f.c[1] * 0xC2B2AE3D27D4EB4Full;

@@ -56,8 +56,8 @@ struct Plan : public cmh_plan {
   // byte offsets in `scal` of the counters, the per-box numbers, the buckets and
   // the sort's digit counts, and its bytes
   size_t at_ctr = 0, at_boxd = 0, at_bucket = 0, at_counts = 0, small_bytes = 0;
-  // what a run reads back passes through pinned memory from the plan's second run
-  // on (a single run would pay more for pinning than it saves)
+  // what a run reads back passes through pinned memory once the plan's first run
+  // has ended (its counters come back unpinned, its catalog pinned)
   HostBuf pinned;
   int runs = 0;
   unsigned char *host_room(size_t bytes, std::vector<unsigned char> &unpinned);

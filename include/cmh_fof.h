@@ -238,7 +238,9 @@ cmh_status cmh_plan_set_graph(cmh_plan *plan, int32_t enable);
  * cmh_plan_run_batch) over a grid of cell-size scales (fine cells per
  * top-cell edge relative to one particle per top cell) and dense-top
  * thresholds, `repeats` timed runs each, and keeps the fastest setting in
- * the plan for its later runs.  Boxes whose params set cell_factor keep it. */
+ * the plan for its later runs.  Boxes whose params set cell_factor keep it.
+ * A plan that was never tuned sizes its cells by a rule of the library's own,
+ * which is not among the settings timed and cannot be set again. */
 typedef struct cmh_tuning {
   double cell_scale;   /* chosen scale of the cell-size factor            */
   int32_t dense_min;   /* occupied fine cells above which a top cell is dense */
