@@ -41,6 +41,9 @@
 #include <cstdio>
 #include <cstring>
 #include <limits>
+#include <map>
+#include <mutex>
+#include <utility>
 #include <vector>
 
 #include "cmh_internal.cuh"
@@ -2537,6 +2540,39 @@ int64_t rows_cap_for(int64_t np_cap, uint64_t k3all) {
   return (int64_t)(((uint64_t)np_cap * 4 + (1ull << 30)) / (rows_per_top(k3all) * sizeof(uint4)));
 }
 
+// The dense-top kernel's limit of dynamic shared memory belongs to the kernel and
+// device, not to a launch: while runs of several plans overlap (from several
+// threads) it is the most that one of them takes.  (The largest possible at all
+// times makes the driver give the SMs less L1: 256^3 box 3.24 -> 3.30 ms, 50M
+// lightcone 10.1 -> 10.3.)  `bytes`: what the plan's run takes; 0 when it has ended.
+void dense_room(const Plan *plan, int device, int bytes) {
+  struct Needs {
+    std::mutex mu;
+    std::map<std::pair<int, const Plan *>, int> of;
+  };
+  static Needs *needs = new Needs;  // (never freed: a run may outlive static objects)
+  std::lock_guard<std::mutex> lock(needs->mu);
+  if (bytes == 0) {
+    needs->of.erase({device, plan});
+    return;
+  }
+  needs->of[{device, plan}] = bytes;
+  int most = 0;
+  for (const auto &q : needs->of)
+    if (q.first.first == device) most = std::max(most, q.second);
+  const void *dense[] = {
+      (const void *)k_befriend_dense<float, true, false>,
+      (const void *)k_befriend_dense<float, false, false>,
+      (const void *)k_befriend_dense<double, true, false>,
+      (const void *)k_befriend_dense<double, false, false>,
+      (const void *)k_befriend_dense<float, true, true>,
+      (const void *)k_befriend_dense<float, false, true>,
+      (const void *)k_befriend_dense<double, true, true>,
+      (const void *)k_befriend_dense<double, false, true>};
+  for (const void *f : dense)
+    CMH_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+}
+
 bool capturing(cudaStream_t s) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   CMH_CUDA(cudaStreamIsCapturing(s, &cs));
@@ -2974,21 +3010,9 @@ void Plan::prepare(const std::vector<BoxSpec> &specs, int want_member) {
     need(b_member_pos, nn * 12);
   }
   // shared memory of the dense-top kernel: one parent per fine cell of a top
-  // cell (set here, outside any graph capture)
-  {
-    const int dsm = (int)(dense_warps_per_cta(k3all) * dense_words(k3all) * sizeof(uint32_t));
-    const void *dense[] = {
-        (const void *)k_befriend_dense<float, true, false>,
-        (const void *)k_befriend_dense<float, false, false>,
-        (const void *)k_befriend_dense<double, true, false>,
-        (const void *)k_befriend_dense<double, false, false>,
-        (const void *)k_befriend_dense<float, true, true>,
-        (const void *)k_befriend_dense<float, false, true>,
-        (const void *)k_befriend_dense<double, true, true>,
-        (const void *)k_befriend_dense<double, false, true>};
-    for (const void *f : dense)
-      CMH_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm));
-  }
+  // cell (set here, outside any graph capture, until the run ends)
+  dense_room(this, device,
+             (int)(dense_warps_per_cta(k3all) * dense_words(k3all) * sizeof(uint32_t)));
   cell_states_apart = radix_states_apart(npc, key_bits, &cell_state_bytes);
   need(sort_tmp, cell_state_bytes);
   // (issue() allocates nothing: it may be captured in a graph)
@@ -3083,6 +3107,10 @@ void Plan::read_back(cudaStream_t s, bool timed) {
 void Plan::run_batch(const std::vector<BoxSpec> &specs, int want_member, cudaStream_t s) {
   CMH_CUDA(cudaSetDevice(device));
   overwritten = false;
+  struct Room {
+    const Plan *plan;
+    ~Room() { dense_room(plan, plan->device, 0); }
+  } room{this};
   for (int attempt = 0; attempt < 3; attempt++) {
     prepare(specs, want_member);
     // the graph stays valid while the inputs, sizes and capacities do
