@@ -131,8 +131,8 @@ def describe(args, w, dtype, n):
 
 # DRAM bytes per processed particle of the befriending launches (ncu
 # dram__bytes_read.sum + dram__bytes_write.sum of the stage's five launches,
-# 256^3 box at scale 1/2: 381.7 MB for 8,971,801 processed particles)
-BEFRIEND_DRAM_PER_PROC = 381.73e6 / 8971801
+# 256^3 box at scale 1/2: 381.4 MB for 8,971,801 processed particles)
+BEFRIEND_DRAM_PER_PROC = 381.41e6 / 8971801
 
 # the launches behind each stage's CUDA-event interval
 KERNELS = {

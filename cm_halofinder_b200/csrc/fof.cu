@@ -2463,7 +2463,8 @@ Geom Plan::make_geometry(const cmh_fof_params &p, const std::vector<double> &lta
     // 32M particles, where the largest dense top cells bound the befriending
     // (scale 0.85 against 1: 64^3 box 0.361 and 0.384 ms, 1.5M particles 0.67 and
     // 0.71, 64 boxes 10.5 and 10.9, 256^3 box 3.43 and 3.43, but the 512^3 box 32.9
-    // and 32.4); and none of more than 10^3 fine cells where that leaves at
+    // and 32.4; the line lies between the last two, with no size measured between);
+    // and none of more than 10^3 fine cells where that leaves at
     // most four top cells per particle (50M lightcone 10.6 ms with 10, 11.5 with
     // 14; 700,000-particle one 0.57 and 0.73), in runs whose top-cell tables are
     // small beside the device's memory.
@@ -2517,6 +2518,7 @@ uint64_t dense_words(uint64_t k3all) {
 // waits at its barriers, which costs a large one.  Befriending with 32, 64, 128
 // and 300: 64^3 box 0.137, 0.150, 0.187, 0.215 ms; 1.5M particles 0.231, 0.223,
 // 0.262, 0.332; 256^3 box 1.16, 1.11, 1.09, 1.14; 512^3 box 14.3, 13.1, 12.5, 12.1.
+// The power law passes near the best of these four.
 uint32_t big_top_min(int64_t np) {
   return (uint32_t)std::max(32.0, 48.0 * std::pow((double)np / 1e6, 0.35));
 }
